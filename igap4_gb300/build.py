@@ -20,7 +20,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libigapgpu.so")
 
-CU_SOURCES = ["context.cu", "assemble.cu", "krylov.cu", "noalloc.cu", "tc_tangent.cu", "graph.cu", "predictor.cu",
+CU_SOURCES = ["context.cu", "assemble.cu", "krylov.cu", "krylov_cycle.cu", "noalloc.cu", "tc_tangent.cu", "graph.cu", "predictor.cu",
               "batch.cu", "tc_gram.cu", "tc_ozaki.cu", "density.cu", "cubic.cu", "res_df.cu"]
 C_SOURCES: list[str] = []
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -182,8 +182,8 @@ static __global__ void __launch_bounds__(AS_THREADS) asm_setup_kernel(const int6
 // z = restricted additive Schwarz applied to v: a warp per subdomain (grid
 // stride), lane c < 3 (cell points) computes the cell's DOF c in FP64 from
 // the FP32 rows.
-__device__ __forceinline__ void asm_apply(double *__restrict__ z, const double *__restrict__ v,
-                                          const float *__restrict__ Z, const CellGeom &g, int64_t ncell)
+__device__ __forceinline__ void asm_apply(double *z, const double *v, const float *__restrict__ Z, const CellGeom &g,
+                                          int64_t ncell)
 {
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);

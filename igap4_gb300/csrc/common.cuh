@@ -102,6 +102,7 @@ struct DevLaw {
 };
 
 struct GraphWork;
+struct CycleWork;
 struct Batch;
 
 // One work item of a batched launch: element (ex, ey, ez) of instance inst,
@@ -196,6 +197,7 @@ struct Context {
   cudaStream_t stream = nullptr;
   // CUDA graphs (graph.cu)
   GraphWork *gmres_graph = nullptr;
+  CycleWork *cycle = nullptr;  // GMRES cycle kernel (krylov_cycle.cu)
   cudaGraphExec_t asm_graph[12] = {};  // key: residual + 2 tangent + 4 precision mode
   int64_t asm_graph_nodes[12] = {};
   bool capturing = false;
@@ -311,6 +313,16 @@ bool spmv_df(const Context *c);
 int ksp_gmres(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int *its,
               double *rnorm);
 int dev_norm2(Context *c, const double *x, double *out);
+// out = |b - w| (w is overwritten)
+int dev_diff_norm2(Context *c, const double *b, double *w, double *out);
+// preconditioner data of the context matrix for the cycle kernel
+int setup_pc(Context *c, int pc, const double **pcd);
+// krylov_cycle.cu: GMRES restart cycles as one cooperative kernel each
+bool cycle_applies(const Context *c, int m);
+int ksp_cycles(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int m, int pc, const double *pcd,
+               double *V, double *Z, double *w, bool cap, int *its, double *rnorm);
+int launch_diag_reciprocal(Context *c, double *inv);
+void cycle_release(Context *c);
 struct CellGeom;
 CellGeom cell_geom(const Context *c);
 int ensure_cblock(Context *c, int64_t ncell);

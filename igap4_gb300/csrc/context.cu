@@ -178,6 +178,7 @@ static int free_ctx(Context *c)
 {
   if (!c) return IGAPGPU_OK;
   graph_release(c);
+  cycle_release(c);
   batch_release(c);
   void *bufs[] = {c->d_wq, c->d_xq, c->d_w, c->d_X, c->d_Uhist, c->d_RR, c->d_vals,
                   c->d_rowptr, c->d_cols, c->d_Dconst, c->d_Fneu, c->d_dir_rows, c->d_dir_g,

@@ -1,6 +1,7 @@
 // CUDA-graph execution of the Newton-Krylov step.
 //
-// * GMRES(m) with modified Gram-Schmidt and right Jacobi preconditioning,
+// * GMRES(m) for restarts that the cycle kernel (krylov_cycle.cu) does not
+//   take, with modified Gram-Schmidt and right Jacobi preconditioning,
 //   device-resident: the Hessenberg column, the Givens rotations and the
 //   convergence test run in single-thread kernels, so one restart cycle
 //   (residual, m Arnoldi steps, least-squares update of x) is one graph with
@@ -402,6 +403,12 @@ int ksp_gmres_graph(Context *c, const double *b, double *x, const igapgpu_solver
   if ((pc == 3 || pc == 4) && c->batch) {
     set_error("block preconditioners (pc = 3, 4) need a single lattice; a batch takes pc 0, 1 or 2");
     return IGAPGPU_ERR_ARG;
+  }
+  if (cycle_applies(c, m)) {
+    const double *pcd;
+    int r = setup_pc(c, pc, &pcd);
+    if (r) return r;
+    return ksp_cycles(c, b, x, o, m, pc, pcd, c->d_V, c->d_Z, c->d_work, false, its_out, rnorm_out);
   }
   if (!c->gmres_graph || c->gmres_graph->m != m || c->gmres_graph->pc != pc || c->gmres_graph->orth != orth ||
       c->gmres_graph->df != spmv_df(c)) {

@@ -106,7 +106,6 @@ __global__ void scale_div_kernel(double *y, const double *x, const double *pden,
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = x[i] * inv;
 }
-// z = v / diag (Jacobi; zero diagonal -> 1, as PCJACOBI)
 __global__ void cblock_kernel(double *z, const double *v, const double *inv, CellGeom g, int64_t ncell)
 {
   cblock_apply(z, v, inv, g, ncell);
@@ -117,12 +116,11 @@ __global__ void bdiag_kernel(double *z, const double *v, const double *inv, int6
   bdiag_apply(z, v, inv, ncp);
 }
 
-__global__ void jacobi_kernel(double *z, const double *v, const double *diag, int64_t n)
+// z = v * (reciprocal diagonal) (Jacobi)
+__global__ void jacobi_kernel(double *z, const double *v, const double *rdiag, int64_t n)
 {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double d = diag[i];
-    z[i] = v[i] / (d != 0.0 ? d : 1.0);
-  }
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    z[i] = v[i] * rdiag[i];
 }
 // r = b - r
 __global__ void sub_from_kernel(double *r, const double *b, int64_t n)
@@ -225,6 +223,13 @@ int dev_norm2(Context *c, const double *x, double *out)
   return IGAPGPU_OK;
 }
 
+int dev_diff_norm2(Context *c, const double *b, double *w, double *out)
+{
+  sub_from_kernel<<<vec_blocks(c->ndof), 256, 0, c->stream>>>(w, b, c->ndof);
+  count_launch();
+  return dev_norm2(c, w, out);
+}
+
 // Lattice cells of the cell-block Jacobi preconditioner (2 x 2 x 2 control points).
 CellGeom cell_geom(const Context *c)
 {
@@ -276,7 +281,46 @@ int asm_setup(Context *c, float *Z)
   return IGAPGPU_OK;
 }
 
-// Right-preconditioned GMRES(m) with MGS, x in/out (device), b device.
+// Set-up of the preconditioner from the context matrix; *pcd: the data the
+// cycle kernel applies (pc = 1: reciprocal diagonal).
+int setup_pc(Context *c, int pc, const double **pcd)
+{
+  const int64_t n = c->ndof;
+  const CellGeom cg = cell_geom(c);
+  const int64_t ncell = cell_count(cg);
+  int r;
+  *pcd = nullptr;
+  if (pc == 1) {
+    if ((r = launch_diag_reciprocal(c, c->d_diag))) return r;
+    *pcd = c->d_diag;
+  } else if (pc == 2) {  // point-block Jacobi: inverted 3 x 3 blocks, 9 per control point
+    bdiag_invert_kernel<<<(unsigned)((n / 3 + 255) / 256), 256, 0, c->stream>>>(c->d_rowptr, c->d_cols, c->d_vals,
+                                                                               c->d_bdiag, n / 3);
+    count_launch();
+    *pcd = c->d_bdiag;
+  } else if (pc == 3) {  // cell-block Jacobi: inverted blocks of the 2 x 2 x 2 control-point cells
+    if ((r = ensure_cblock(c, ncell))) return r;
+    cblock_invert_kernel<<<(unsigned)((ncell + CB_WARPS - 1) / CB_WARPS), 32 * CB_WARPS, 0, c->stream>>>(
+        c->d_rowptr, c->d_vals, c->d_cinv, cg, ncell);
+    count_launch();
+    *pcd = c->d_cinv;
+  } else if (pc == 4) {  // restricted additive Schwarz
+    if (!c->d_asmz && cudaMalloc(&c->d_asmz, sizeof(float) * (size_t)ncell * AS_NC * AS_N) != cudaSuccess) {
+      cudaGetLastError();
+      c->d_asmz = nullptr;
+      set_error("additive Schwarz: allocation of %lld subdomains failed", (long long)ncell);
+      return IGAPGPU_ERR_NOMEM;
+    }
+    if ((r = asm_setup(c, c->d_asmz))) return r;
+    *pcd = reinterpret_cast<const double *>(c->d_asmz);
+  }
+  IGAP_CHECK_LAUNCH();
+  return IGAPGPU_OK;
+}
+
+// Right-preconditioned GMRES(m) with MGS, x in/out (device), b device.  The
+// cycle kernel (krylov_cycle.cu) takes it unless the restart is too long for
+// its shared memory; then one launch per vector operation.
 int ksp_gmres(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int *its_out,
               double *rnorm_out)
 {
@@ -292,29 +336,10 @@ int ksp_gmres(Context *c, const double *b, double *x, const igapgpu_solver_opts 
     set_error("block preconditioners (pc = 3, 4) use the quadratic stencil; degree 3 takes pc 0, 1 or 2");
     return IGAPGPU_ERR_ARG;
   }
-  if (o->pc == 1) {
-    get_diag_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->d_rowptr, c->d_cols, c->d_vals, c->d_diag, n);
-    count_launch();
-  } else if (o->pc == 2) {  // point-block Jacobi: inverted 3 x 3 blocks, 9 per control point
-    bdiag_invert_kernel<<<(unsigned)((n / 3 + 255) / 256), 256, 0, c->stream>>>(c->d_rowptr, c->d_cols, c->d_vals,
-                                                                               c->d_bdiag, n / 3);
-    count_launch();
-    IGAP_CHECK_LAUNCH();
-  } else if (o->pc == 3) {  // cell-block Jacobi: inverted blocks of the 2 x 2 x 2 control-point cells
-    if ((r = ensure_cblock(c, ncell))) return r;
-    cblock_invert_kernel<<<(unsigned)((ncell + CB_WARPS - 1) / CB_WARPS), 32 * CB_WARPS, 0, c->stream>>>(
-        c->d_rowptr, c->d_vals, c->d_cinv, cg, ncell);
-    count_launch();
-    IGAP_CHECK_LAUNCH();
-  } else if (o->pc == 4) {  // restricted additive Schwarz
-    if (!c->d_asmz && cudaMalloc(&c->d_asmz, sizeof(float) * (size_t)ncell * AS_NC * AS_N) != cudaSuccess) {
-      cudaGetLastError();
-      c->d_asmz = nullptr;
-      set_error("additive Schwarz: allocation of %lld subdomains failed", (long long)ncell);
-      return IGAPGPU_ERR_NOMEM;
-    }
-    if ((r = asm_setup(c, c->d_asmz))) return r;
-  }
+  const int pc = o->pc >= 1 && o->pc <= 4 ? o->pc : 0;
+  const double *pcd;
+  if ((r = setup_pc(c, pc, &pcd))) return r;
+  if (cycle_applies(c, m)) return ksp_cycles(c, b, x, o, m, pc, pcd, V, Z, w, true, its_out, rnorm_out);
   std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m);
   double rnorm0 = -1.0, rnorm = 0.0;
   int its = 0;

@@ -1,0 +1,732 @@
+// One GMRES restart cycle as one cooperative kernel: residual, the Arnoldi
+// steps (preconditioner, multiply, orthogonalisation, Givens rotation,
+// convergence test) and the update of x, the stages separated by grid
+// barriers instead of kernel launches (role of KSPSolve with
+// KSPGMRESModifiedGramSchmidtOrthogonalization, src/interface.c:228-241).
+//
+// A lattice of a few thousand control points keeps the GPU busy for a few
+// microseconds per stage, so launches bound the cycle: modified Gram-Schmidt
+// as a dot product and an update per basis vector took three launches a
+// vector, 15,150 in a cycle of 100 steps (85 ms launched one by one at
+// 32x8x8, 29 ms as a graph of the 16x4x4 system).  Here
+//  * modified Gram-Schmidt runs in its inverse compact WY form (Swirydowicz,
+//    Langou, Ananthan, Yang, Thomas, Numer. Linear Algebra Appl. 28 (2021)):
+//    the sequential projections (I - v_j v_j^T) ... (I - v_0 v_0^T) w equal
+//    w - V h with (I + L) h = V^T w, L the strictly lower triangle of V^T V,
+//    so one pass over V gives every dot product with w and, beside it, the
+//    new row of L (dot products with v_j); T = (I + L)^-1 grows by one row per
+//    step and is kept in every block's shared memory, and h = T V^T w;
+//  * opts.orth = 1 (classical Gram-Schmidt twice) runs the same two passes
+//    twice with T = I;
+//  * the Givens chain of a column runs on one warp while the other warps
+//    multiply for the next step; the cycle stops one multiply later than the
+//    test, with the same iterate;
+//  * the FP64 pipe (2 FMA per clock and SM) bounds the stages, so cross-lane
+//    sums are merged: a warp of the multiply owns the three rows of a control
+//    point (one gather of x for three products), a warp of the projection
+//    four basis vectors, and the partial sums of several rows or vectors are
+//    folded together (9 instead of 40 additions for 8 sums).
+//
+// Measured: 100 iterations at 32x8x8 (10,200 rows, Jacobi) 86.2 -> 4.5 ms; the
+// static solve of the 16x4x4 beam 79.3 -> 13.9 ms; the transient step at
+// 32x8x8 (cell blocks, CGS2) 18.3 -> 13.8 ms.
+//
+// One block of 1024 threads per SM (cooperative launch: all blocks resident).
+// Data that other blocks wrote are read with plain or L2 loads after the
+// barrier (release/acquire at GPU scope), never through the read-only path.
+// Every barrier wait is bounded; a block that gives up sets the error word
+// and returns, the others see the word and return.
+#include <cuda_runtime.h>
+#include <math.h>
+#include <string.h>
+
+#include "common.cuh"
+#include "spmv.cuh"
+#include "asm_pc.cuh"
+
+namespace igap {
+
+namespace {
+constexpr int CY_THREADS = 1024, CY_WARPS = CY_THREADS / 32;
+constexpr int CY_VB = 4;             // basis vectors per item of the projection
+constexpr int CY_RMAX = 1024;        // row chunks per group of vectors
+constexpr int CY_MAX_RESTART = 200;  // T (m (m - 1) / 2 doubles) in shared memory
+constexpr uint32_t CY_WAIT_LIMIT = 1u << 24;
+
+struct CycleState {
+  int its;        // Arnoldi steps of this cycle
+  int stop;       // the cycle ended before its last step (converged or broke down)
+  double beta;    // |r| at the start of the cycle
+  double rnorm;   // residual estimate
+  double rnorm0;  // |r| of the first cycle (negative before it)
+  double tol;
+};
+
+struct CycleArgs {
+  const int64_t *rowptr;
+  const int32_t *cols;
+  const double *vals;
+  const double *b;
+  double *x, *w, *V, *Z;
+  const double *pcd;   // Jacobi: reciprocal diagonal; block preconditioners: their blocks
+  double *H;           // [m][m + 1] columns
+  double *cs, *sn, *g, *y;
+  double *part;        // projection partial sums [2][vectors][CY_RMAX]
+  double *npart;       // norm partial sums [2][blocks]
+  CycleState *st;
+  unsigned *bar;       // arrivals at the grid barrier
+  int *err;
+  CellGeom cg;
+  int64_t n;
+  int m, steps, pc, orth;
+  double rtol, abstol, dtol;
+};
+
+struct CycleSmem {
+  double red[CY_THREADS];
+  double r[CY_MAX_RESTART + 1], l[CY_MAX_RESTART + 1], h[CY_MAX_RESTART + 1];
+  double bc;           // a broadcast sum
+  int ok;
+  // packed rows of T (row i: entries c < i at i (i - 1) / 2) follow
+};
+
+// All blocks arrive and wait.  Release/acquire at GPU scope by thread 0, the
+// block barriers around it order the other threads.
+__device__ __forceinline__ bool grid_sync(const CycleArgs &a, CycleSmem &S, unsigned &target)
+{
+  __syncthreads();
+  target += gridDim.x;
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+    int ok = 0;
+    for (uint32_t it = 0; it < CY_WAIT_LIMIT; it++) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+      if ((int)(v - target) >= 0) {
+        ok = 1;
+        break;
+      }
+      if ((it & 1023u) == 1023u && *(volatile int *)a.err) break;
+    }
+    if (!ok) atomicExch(a.err, 4);
+    S.ok = ok;
+  }
+  __syncthreads();
+  return S.ok != 0;
+}
+
+// Sum of s over the block in a fixed order: the threads' values through
+// shared memory, then one warp (37 instead of 165 FP64 warp additions).
+// Valid in thread 0.
+__device__ __forceinline__ double block_sum(CycleSmem &S, double s)
+{
+  S.red[threadIdx.x] = s;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int k = 0; k < CY_WARPS; k++) t += S.red[threadIdx.x + 32 * k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  }
+  return t;
+}
+
+// Square root of the sum of the blocks' partial sums, by every block in the
+// same order.
+__device__ __forceinline__ double total_norm(const CycleArgs &a, CycleSmem &S, int slot)
+{
+  if (threadIdx.x < 32) {
+    double t = 0.0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += 32) t += __ldcg(a.npart + slot * gridDim.x + k);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (threadIdx.x == 0) S.bc = sqrt(t);
+  }
+  __syncthreads();
+  return S.bc;
+}
+
+// Three sums over the lanes of a group of G lanes (16 or 32): the first two
+// steps exchange, so that the quarters of the group carry different sums (6
+// instead of 15 additions at G = 32).  Returns this lane's sum; `which` tells
+// which of the three it is (3: none).
+template <int G>
+__device__ __forceinline__ double fold3(double s0, double s1, double s2, int sub, int &which)
+{
+  constexpr int A = G / 2, B = G / 4;
+  const bool up = sub & A;
+  // upper half keeps s2 (and an empty slot), lower half s0 and s1
+  double k0 = up ? s2 : s0, k1 = up ? 0.0 : s1;
+  const double g0 = up ? s0 : s2, g1 = up ? s1 : 0.0;
+  k0 += __shfl_xor_sync(0xffffffffu, g0, A);
+  k1 += __shfl_xor_sync(0xffffffffu, g1, A);
+  const bool up2 = sub & B;
+  double v = up2 ? k1 : k0;
+  v += __shfl_xor_sync(0xffffffffu, up2 ? k0 : k1, B);
+#pragma unroll
+  for (int o = G / 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  which = up ? (up2 ? 3 : 2) : (up2 ? 1 : 0);
+  return v;
+}
+
+// w = A x (or b - A x with RES) over this grid's groups of G lanes, one
+// control point (three rows sharing their columns) per group; returns this
+// thread's part of |w|^2 with RES.
+template <int G, bool RES>
+__device__ __forceinline__ double multiply(const CycleArgs &a, const double *x, double *w)
+{
+  const int64_t ncp = a.n / 3;
+  const int sub = threadIdx.x % G;
+  const int64_t ng = (int64_t)gridDim.x * (CY_THREADS / G);
+  double nn = 0.0;
+  // consecutive groups of one block take control points a grid apart: every
+  // SM gets the same share when there are fewer points than groups
+  for (int64_t c0 = blockIdx.x + (int64_t)gridDim.x * (threadIdx.x / 32 * (32 / G)); c0 < ncp; c0 += ng) {
+    const int64_t cp = c0 + (int64_t)gridDim.x * ((threadIdx.x % 32) / G);
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+    if (cp < ncp) {
+      const int64_t r0 = __ldg(a.rowptr + 3 * cp), r1 = __ldg(a.rowptr + 3 * cp + 1);
+      const int len = (int)(r1 - r0);
+      const double *v0 = a.vals + r0, *v1 = v0 + len, *v2 = v1 + len;
+      const int32_t *col = a.cols + r0;
+#pragma unroll 4
+      for (int k = sub; k < len; k += G) {
+        const double xv = x[__ldg(col + k)];
+        s0 = fma(__ldg(v0 + k), xv, s0);
+        s1 = fma(__ldg(v1 + k), xv, s1);
+        s2 = fma(__ldg(v2 + k), xv, s2);
+      }
+    }
+    int which;
+    double v = fold3<G>(s0, s1, s2, sub, which);
+    if (cp < ncp && which < 3 && (sub & (G / 4 - 1)) == 0) {
+      const int64_t row = 3 * cp + which;
+      if (RES) {
+        v = a.b[row] - v;
+        nn = fma(v, v, nn);
+      }
+      w[row] = v;
+    }
+  }
+  return nn;
+}
+
+template <bool RES>
+__device__ __forceinline__ double multiply_any(const CycleArgs &a, const double *x, double *w)
+{
+  // 32 lanes a control point while there are fewer points than groups of 16
+  return a.n / 3 < (int64_t)gridDim.x * CY_WARPS * 2 ? multiply<32, RES>(a, x, w) : multiply<16, RES>(a, x, w);
+}
+
+// Partial dot products of the basis vectors 0..j with w (and, with LROW, with
+// v_j): item (group of CY_VB vectors, row chunk) per warp.
+template <bool LROW>
+__device__ __forceinline__ void project_partial(const CycleArgs &a, int j, int R)
+{
+  const int lane = threadIdx.x & 31;
+  const int ngroup = (j + CY_VB) / CY_VB;
+  const int64_t chunk = (a.n + R - 1) / R;
+  const double *vj = a.V + (size_t)j * a.n;
+  for (int it = blockIdx.x + gridDim.x * (threadIdx.x >> 5); it < ngroup * R; it += gridDim.x * CY_WARPS) {
+    const int i0 = (it / R) * CY_VB, r = it % R;
+    const int64_t lo = r * chunk, hi = lo + chunk < a.n ? lo + chunk : a.n;
+    const double *v[CY_VB];
+#pragma unroll
+    for (int q = 0; q < CY_VB; q++) v[q] = a.V + (size_t)min(i0 + q, j) * a.n;
+    double s[2 * CY_VB];
+#pragma unroll
+    for (int q = 0; q < 2 * CY_VB; q++) s[q] = 0.0;
+#pragma unroll 2
+    for (int64_t k = lo + lane; k < hi; k += 32) {
+      const double wk = __ldcg(a.w + k);
+      const double vk = LROW ? __ldcg(vj + k) : 0.0;
+#pragma unroll
+      for (int q = 0; q < CY_VB; q++) {
+        const double u = __ldcg(v[q] + k);
+        s[q] = fma(u, wk, s[q]);
+        if (LROW) s[CY_VB + q] = fma(u, vk, s[CY_VB + q]);
+      }
+    }
+    // fold the sums over the lanes: each exchange halves the number of sums a
+    // lane carries
+    int id = 0;
+    constexpr int NS = LROW ? 8 : 4;
+#pragma unroll
+    for (int o = 16, cnt = NS; o > 0; o >>= 1) {
+      if (cnt > 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int q = 0; q < cnt / 2; q++) {
+          const double keep = up ? s[q + cnt / 2] : s[q], give = up ? s[q] : s[q + cnt / 2];
+          s[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+        if (up) id += cnt / 2;
+        cnt /= 2;
+      } else {
+        s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+      }
+    }
+    const int q = id % CY_VB, kind = id / CY_VB;
+    if ((lane & (32 / NS - 1)) == 0 && i0 + q <= j)
+      a.part[((size_t)kind * (a.m + 1) + i0 + q) * CY_RMAX + r] = s[0];
+  }
+}
+
+// Sums the partial dot products into S.r (with w) and S.l (with v_j).
+template <bool LROW>
+__device__ __forceinline__ void project_total(const CycleArgs &a, CycleSmem &S, int j, int R)
+{
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x >> 5; i <= j; i += CY_WARPS) {
+    const double *p = a.part + (size_t)i * CY_RMAX, *pl = p + (size_t)(a.m + 1) * CY_RMAX;
+    double s = 0.0, t = 0.0;
+    for (int r = lane; r < R; r += 32) {
+      s += __ldcg(p + r);
+      if (LROW) t += __ldcg(pl + r);
+    }
+    if (LROW) {  // the halves of the warp carry one sum each
+      const bool up = lane & 16;
+      s = (up ? t : s) + __shfl_xor_sync(0xffffffffu, up ? s : t, 16);
+    } else {
+      s += __shfl_xor_sync(0xffffffffu, s, 16);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) S.r[i] = s;
+    if (LROW && lane == 16) S.l[i] = s;
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ double *t_row(CycleSmem &S, int i)
+{
+  return reinterpret_cast<double *>(&S + 1) + (size_t)i * (i - 1) / 2;
+}
+
+// Row j of T = (I + L)^-1 and h = T r, redundantly in every block.
+__device__ __forceinline__ void solve_t(CycleSmem &S, int j)
+{
+  const int width = (j + 32) & ~31;             // threads per slice of the sums
+  const int ns = CY_THREADS / width;            // slices
+  const int c = threadIdx.x % width, sl = threadIdx.x / width;
+  // t_j[c] = -(l_c + sum_{c < k < j} l_k T[k][c])
+  double s = 0.0;
+  if (sl < ns && c < j)
+    for (int k = c + 1 + sl; k < j; k += ns) s = fma(S.l[k], t_row(S, k)[c], s);
+  if (sl < ns) S.red[sl * width + c] = s;
+  __syncthreads();
+  if (threadIdx.x < j) {
+    double t = S.l[threadIdx.x];
+    for (int q = 0; q < ns; q++) t += S.red[q * width + threadIdx.x];
+    t_row(S, j)[threadIdx.x] = -t;
+  }
+  __syncthreads();
+  // h_i = r_i + sum_{c < i} T[i][c] r_c
+  s = 0.0;
+  if (sl < ns && c <= j)
+    for (int k = sl; k < c; k += ns) s = fma(t_row(S, c)[k], S.r[k], s);
+  if (sl < ns) S.red[sl * width + c] = s;
+  __syncthreads();
+  if (threadIdx.x <= j) {
+    double t = S.r[threadIdx.x];
+    for (int q = 0; q < ns; q++) t += S.red[q * width + threadIdx.x];
+    S.h[threadIdx.x] = t;
+  }
+  __syncthreads();
+}
+
+// w -= V h on this block's rows (h = hs); returns this thread's part of |w|^2.
+// With fewer rows than threads the basis vectors are split over ns threads a
+// row and their sums joined through shared memory.
+__device__ __forceinline__ double update_w(const CycleArgs &a, CycleSmem &S, const double *hs, int j)
+{
+  const int64_t per = (a.n + gridDim.x - 1) / gridDim.x;
+  const int64_t lo = (int64_t)blockIdx.x * per, hi = lo + per < a.n ? lo + per : a.n;
+  double nn = 0.0;
+  int width = 32;
+  while (width < per && width < CY_THREADS) width *= 2;
+  const int ns = CY_THREADS / width < 8 ? CY_THREADS / width : 8;
+  if (ns == 1) {
+    for (int64_t r = lo + threadIdx.x; r < hi; r += CY_THREADS) {
+      double s = __ldcg(a.w + r);
+#pragma unroll 8
+      for (int i = 0; i <= j; i++) s = fma(-hs[i], __ldcg(a.V + (size_t)i * a.n + r), s);
+      a.w[r] = s;
+      nn = fma(s, s, nn);
+    }
+    return nn;
+  }
+  const int c = threadIdx.x % width, sl = threadIdx.x / width;
+  const int64_t r = lo + c;
+  if (sl < ns) {
+    double s = 0.0;
+    if (r < hi) {
+#pragma unroll 4
+      for (int i = sl; i <= j; i += ns) s = fma(hs[i], __ldcg(a.V + (size_t)i * a.n + r), s);
+    }
+    S.red[sl * width + c] = s;
+  }
+  __syncthreads();
+  if (sl == 0 && r < hi) {
+    double s = __ldcg(a.w + r);
+    for (int q = 0; q < ns; q++) s -= S.red[q * width + c];
+    a.w[r] = s;
+    nn = s * s;
+  }
+  __syncthreads();
+  return nn;
+}
+
+// v = w / den on this block's rows and, without or with scalar Jacobi
+// preconditioning, z = M^-1 v.
+__device__ __forceinline__ void normalise(const CycleArgs &a, double den, double *v, double *z)
+{
+  const int64_t per = (a.n + gridDim.x - 1) / gridDim.x;
+  const int64_t lo = (int64_t)blockIdx.x * per, hi = lo + per < a.n ? lo + per : a.n;
+  const double inv = 1.0 / den;
+  for (int64_t r = lo + threadIdx.x; r < hi; r += CY_THREADS) {
+    const double t = __ldcg(a.w + r) * inv;
+    v[r] = t;
+    if (a.pc == 0) z[r] = t;
+    else if (a.pc == 1) z[r] = t * __ldg(a.pcd + r);
+  }
+}
+
+__device__ __forceinline__ void block_precondition(const CycleArgs &a, const double *v, double *z)
+{
+  if (a.pc == 2) bdiag_apply(z, v, a.pcd, a.n / 3);
+  else if (a.pc == 3) cblock_apply(z, v, a.pcd, a.cg, cell_count(a.cg));
+  else asm_apply(z, v, reinterpret_cast<const float *>(a.pcd), a.cg, cell_count(a.cg));
+}
+
+// Givens update of Hessenberg column j by one warp (lane 0 runs the chain on
+// values staged in shared memory) and the convergence test.
+__device__ void givens(const CycleArgs &a, double *sh, int j)
+{
+  const int lane = threadIdx.x & 31;
+  double *h = a.H + (size_t)j * (a.m + 1);
+  double *hh = sh, *cc = sh + CY_MAX_RESTART + 2, *ss = cc + CY_MAX_RESTART + 2;
+  for (int i = lane; i <= j + 1; i += 32) hh[i] = __ldcg(h + i);
+  for (int i = lane; i < j; i += 32) {
+    cc[i] = __ldcg(a.cs + i);
+    ss[i] = __ldcg(a.sn + i);
+  }
+  __syncwarp();
+  if (lane == 0) {
+    double hi = hh[0];
+    for (int i = 0; i < j; i++) {
+      const double hn = hh[i + 1];
+      hh[i] = fma(ss[i], hn, cc[i] * hi);
+      hi = fma(-ss[i], hi, cc[i] * hn);
+    }
+    const double hl = hh[j + 1];
+    double den = hypot(hi, hl);
+    const bool breakdown = !(den > 0.0) || !isfinite(den);
+    if (breakdown) den = 1e-300;
+    const double c = hi / den, s = hl / den;
+    a.cs[j] = c;
+    a.sn[j] = s;
+    hh[j] = den;
+    hh[j + 1] = 0.0;
+    const double gj = __ldcg(a.g + j), gn = -s * gj;
+    a.g[j] = c * gj;
+    a.g[j + 1] = gn;
+    a.st->rnorm = fabs(gn);
+    a.st->its = j + 1;
+    if (fabs(gn) <= a.st->tol || breakdown || !isfinite(gn)) a.st->stop = 1;
+  }
+  __syncwarp();
+  for (int i = lane; i <= j + 1; i += 32) h[i] = hh[i];
+}
+
+// y = H(0:k, 0:k)^-1 g by one block, column by column.
+__device__ void backsolve(const CycleArgs &a, CycleSmem &S, int k)
+{
+  for (int i = threadIdx.x; i < k; i += CY_THREADS) S.h[i] = __ldcg(a.g + i);
+  for (int i = k - 1; i >= 0; i--) {
+    const double *col = a.H + (size_t)i * (a.m + 1);
+    const double hc = threadIdx.x <= i ? __ldcg(col + threadIdx.x) : 0.0;
+    __syncthreads();
+    if (threadIdx.x == i) S.bc = S.h[i] = S.h[i] / hc;
+    __syncthreads();
+    if (threadIdx.x < i) S.h[threadIdx.x] = fma(-hc, S.bc, S.h[threadIdx.x]);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < k; i += CY_THREADS) a.y[i] = S.h[i];
+}
+
+__global__ void __launch_bounds__(CY_THREADS, 1) gmres_cycle_kernel(CycleArgs a)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  CycleSmem &S = *reinterpret_cast<CycleSmem *>(smem_raw);
+  __shared__ double gsh[3 * (CY_MAX_RESTART + 2)];
+  __shared__ int s_stop;
+  unsigned target = 0;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const bool last_block = blockIdx.x == gridDim.x - 1;
+  CycleState *st = a.st;
+  // r = b - A x, beta = |r|
+  {
+    const double nn = block_sum(S, multiply_any<true>(a, a.x, a.w));
+    if (tid == 0) a.npart[blockIdx.x] = nn;
+  }
+  if (!grid_sync(a, S, target)) return;
+  const double beta = total_norm(a, S, 0);
+  const double rnorm0 = st->rnorm0 < 0.0 ? beta : st->rnorm0;
+  const double tol = st->rnorm0 < 0.0 ? fmax(a.rtol * beta, a.abstol) : st->tol;
+  const bool go = beta > tol && isfinite(beta) && !(beta > a.dtol * rnorm0) && a.steps > 0;
+  if (!grid_sync(a, S, target)) return;  // every block has read rnorm0 and tol
+  if (last_block && tid == 0) {
+    st->rnorm0 = rnorm0;
+    st->tol = tol;
+    st->beta = st->rnorm = beta;
+    st->its = 0;
+    st->stop = go ? 0 : 1;
+    a.g[0] = beta;
+  }
+  if (!go) return;
+  normalise(a, beta, a.V, a.Z);
+  if (!grid_sync(a, S, target)) return;
+  int k = 0;
+  for (int j = 0; j < a.steps; j++) {
+    double *vj = a.V + (size_t)j * a.n, *zj = a.Z + (size_t)j * a.n;
+    if (a.pc >= 2) {
+      block_precondition(a, vj, zj);
+      if (!grid_sync(a, S, target)) return;
+    }
+    // the previous column's rotation beside the multiply
+    if (j > 0 && last_block && warp == CY_WARPS - 1) givens(a, gsh, j - 1);
+    multiply_any<false>(a, zj, a.w);
+    if (!grid_sync(a, S, target)) return;
+    if (j > 0) {
+      if (tid == 0) s_stop = *(volatile int *)&st->stop;
+      __syncthreads();
+      if (s_stop) {
+        k = j;
+        break;
+      }
+    }
+    // orthogonalise
+    const int ngroup = (j + CY_VB) / CY_VB;
+    int R = (int)(gridDim.x * CY_WARPS) / ngroup;
+    const int64_t rmax = (a.n + 127) / 128;
+    R = R < CY_RMAX ? R : CY_RMAX;
+    R = R < rmax ? R : (int)rmax;
+    R = R > 0 ? R : 1;
+    double nn;
+    if (a.orth == 1) {
+      project_partial<false>(a, j, R);
+      if (!grid_sync(a, S, target)) return;
+      project_total<false>(a, S, j, R);
+      update_w(a, S, S.r, j);
+      if (tid <= j) S.h[tid] = S.r[tid];
+      if (!grid_sync(a, S, target)) return;
+      project_partial<false>(a, j, R);
+      if (!grid_sync(a, S, target)) return;
+      project_total<false>(a, S, j, R);
+      nn = update_w(a, S, S.r, j);
+      if (tid <= j) S.h[tid] += S.r[tid];
+    } else {
+      project_partial<true>(a, j, R);
+      if (!grid_sync(a, S, target)) return;
+      project_total<true>(a, S, j, R);
+      solve_t(S, j);
+      nn = update_w(a, S, S.h, j);
+    }
+    nn = block_sum(S, nn);
+    if (tid == 0) a.npart[gridDim.x * (1 + (j & 1)) + blockIdx.x] = nn;
+    if (!grid_sync(a, S, target)) return;
+    const double hn = total_norm(a, S, 1 + (j & 1));
+    if (last_block) {
+      if (tid <= j) a.H[(size_t)j * (a.m + 1) + tid] = S.h[tid];
+      if (tid == 0) a.H[(size_t)j * (a.m + 1) + j + 1] = hn;
+    }
+    if (j + 1 < a.steps) {
+      normalise(a, hn, vj + a.n, zj + a.n);
+    } else {
+      __syncthreads();
+      if (last_block && warp == CY_WARPS - 1) givens(a, gsh, j);
+      k = j + 1;
+    }
+    if (!grid_sync(a, S, target)) return;
+  }
+  // x += Z y
+  if (last_block) backsolve(a, S, k);
+  if (!grid_sync(a, S, target)) return;
+  for (int i = tid; i < k; i += CY_THREADS) S.h[i] = __ldcg(a.y + i);
+  __syncthreads();
+  for (int64_t r = (int64_t)blockIdx.x + (int64_t)gridDim.x * tid; r < a.n; r += (int64_t)gridDim.x * CY_THREADS) {
+    double s = a.x[r];
+    for (int i = 0; i < k; i++) s = fma(S.h[i], __ldcg(a.Z + (size_t)i * a.n + r), s);
+    a.x[r] = s;
+  }
+}
+
+__global__ void diag_reciprocal_kernel(const int64_t *rowptr, const int32_t *cols, const double *vals, double *inv,
+                                       int64_t n)
+{
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  int64_t lo = rowptr[r], hi = rowptr[r + 1];
+  const int64_t end = hi;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (cols[mid] < r) lo = mid + 1;
+    else hi = mid;
+  }
+  const double d = (lo < end && cols[lo] == r) ? vals[lo] : 0.0;
+  inv[r] = d != 0.0 ? 1.0 / d : 1.0;  // a zero diagonal counts as 1, as PCJACOBI
+}
+}  // namespace
+
+struct CycleWork {
+  int m = 0, grid = 0;
+  double *buf = nullptr;      // H, cs, sn, g, y, partial sums
+  unsigned *ctl = nullptr;    // barrier counter, error word (128 B apart), state
+  CycleState *h_st = nullptr; // pinned: state and error word
+};
+
+void cycle_release(Context *c)
+{
+  CycleWork *cw = c->cycle;
+  if (!cw) return;
+  if (cw->buf) cudaFree(cw->buf);
+  if (cw->ctl) cudaFree(cw->ctl);
+  if (cw->h_st) cudaFreeHost(cw->h_st);
+  delete cw;
+  c->cycle = nullptr;
+}
+
+constexpr size_t CY_CTL_BYTES = 256 + sizeof(CycleState);
+
+static int ensure_cycle(Context *c, int m)
+{
+  if (c->cycle && c->cycle->m >= m) return IGAPGPU_OK;
+  cycle_release(c);
+  CycleWork *cw = new CycleWork();
+  c->cycle = cw;
+  int dev = 0, nsm = 0;
+  IGAP_CUDA(cudaGetDevice(&dev));
+  IGAP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const size_t cnt = (size_t)(m + 1) * m + 4 * (size_t)(m + 1) + 2 * (size_t)(m + 1) * CY_RMAX + 3 * (size_t)nsm;
+  if (cudaMalloc(&cw->buf, sizeof(double) * cnt) != cudaSuccess || cudaMalloc(&cw->ctl, CY_CTL_BYTES) != cudaSuccess ||
+      cudaMallocHost(&cw->h_st, CY_CTL_BYTES) != cudaSuccess) {
+    cudaGetLastError();
+    cycle_release(c);
+    set_error("GMRES cycle workspace (restart %d) does not fit", m);
+    return IGAPGPU_ERR_NOMEM;
+  }
+  cw->m = m;
+  cw->grid = nsm;
+  return IGAPGPU_OK;
+}
+
+static size_t cycle_smem(int m) { return sizeof(CycleSmem) + sizeof(double) * ((size_t)m * (m - 1) / 2 + 1); }
+
+// Whether the cycle kernel takes this solve (19 times faster than the separate
+// launches at 32x8x8, so up to the longest restart that fits): T fits in shared memory, the
+// multiply in FP64 arithmetic (IGAPGPU_SPMV_DF keeps the separate kernels).
+bool cycle_applies(const Context *c, int m) { return m <= CY_MAX_RESTART && !spmv_df(c); }
+
+// GMRES cycles on the context matrix; b, x device vectors, pcd the
+// preconditioner's data, V and Z the basis buffers.  `cap`: stop at ksp_max_it
+// inside a cycle and return the true residual norm (else whole cycles and the
+// recurrence's estimate).
+int ksp_cycles(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int m, int pc, const double *pcd,
+               double *V, double *Z, double *w, bool cap, int *its_out, double *rnorm_out)
+{
+  int r = ensure_cycle(c, m);
+  if (r) return r;
+  CycleWork *cw = c->cycle;
+  CycleArgs a;
+  memset(&a, 0, sizeof a);
+  a.rowptr = c->d_rowptr;
+  a.cols = c->d_cols;
+  a.vals = c->d_vals;
+  a.b = b;
+  a.x = x;
+  a.w = w;
+  a.V = V;
+  a.Z = Z;
+  a.pcd = pcd;
+  a.H = cw->buf;
+  a.cs = a.H + (size_t)(cw->m + 1) * cw->m;
+  a.sn = a.cs + cw->m + 1;
+  a.g = a.sn + cw->m + 1;
+  a.y = a.g + cw->m + 1;
+  a.part = a.y + cw->m + 1;
+  a.npart = a.part + 2 * (size_t)(cw->m + 1) * CY_RMAX;
+  a.bar = cw->ctl;
+  a.err = reinterpret_cast<int *>(cw->ctl + 32);
+  a.st = reinterpret_cast<CycleState *>(cw->ctl + 64);
+  a.cg = cell_geom(c);
+  a.n = c->ndof;
+  a.m = m;
+  a.pc = pc;
+  a.orth = !cap && o->orth == 1 ? 1 : 0;
+  a.rtol = o->ksp_rtol;
+  a.abstol = o->ksp_abstol;
+  a.dtol = o->ksp_dtol;
+  const size_t smem = cycle_smem(m);
+  IGAP_CUDA(cudaFuncSetAttribute(gmres_cycle_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cycle_smem(CY_MAX_RESTART)));
+  CycleState h0;
+  memset(&h0, 0, sizeof h0);
+  h0.rnorm0 = -1.0;
+  IGAP_CUDA(cudaMemcpyAsync(a.st, &h0, sizeof h0, cudaMemcpyHostToDevice, c->stream));
+  int its = 0;
+  double rnorm = 0.0;
+  for (;;) {
+    a.steps = m;
+    if (cap && o->ksp_max_it - its < m) a.steps = o->ksp_max_it - its > 0 ? o->ksp_max_it - its : 0;
+    IGAP_CUDA(cudaMemsetAsync(cw->ctl, 0, 256, c->stream));
+    void *params[] = {&a};
+    IGAP_CUDA(cudaLaunchCooperativeKernel((const void *)gmres_cycle_kernel, dim3(cw->grid), dim3(CY_THREADS), params,
+                                          smem, c->stream));
+    count_launch();
+    IGAP_CUDA(cudaMemcpyAsync(cw->h_st, cw->ctl, CY_CTL_BYTES, cudaMemcpyDeviceToHost, c->stream));
+    IGAP_CUDA(cudaStreamSynchronize(c->stream));
+    const unsigned *ctl = reinterpret_cast<const unsigned *>(cw->h_st);
+    if (ctl[32]) {
+      set_error("GMRES: a bounded grid barrier wait expired (code %u)", ctl[32]);
+      return IGAPGPU_ERR_TIMEOUT;
+    }
+    CycleState st;
+    memcpy(&st, ctl + 64, sizeof st);
+    its += st.its;
+    rnorm = st.rnorm;
+    if (!isfinite(rnorm) || !isfinite(st.beta)) {
+      set_error("GMRES: non-finite residual norm");
+      return IGAPGPU_ERR_NUMERIC;
+    }
+    const bool met = rnorm <= st.tol, out_of_its = its >= o->ksp_max_it;
+    // the step limit and the tolerance are looked at before the divergence
+    // test when the limit is exact, after it in whole cycles
+    if (cap && st.its == 0 && (met || out_of_its)) break;
+    if (st.rnorm0 > 0 && st.beta > o->ksp_dtol * st.rnorm0) {
+      set_error("GMRES diverged (dtol)");
+      return IGAPGPU_ERR_NUMERIC;
+    }
+    if (met || out_of_its || st.its == 0) {
+      if (cap) {  // true residual of the final iterate
+        if ((r = spmv(c, c->d_vals, x, w))) return r;
+        if ((r = dev_diff_norm2(c, b, w, &rnorm))) return r;
+      }
+      break;
+    }
+  }
+  if (its_out) *its_out = its;
+  if (rnorm_out) *rnorm_out = rnorm;
+  return IGAPGPU_OK;
+}
+
+int launch_diag_reciprocal(Context *c, double *inv)
+{
+  diag_reciprocal_kernel<<<(unsigned)((c->ndof + 255) / 256), 256, 0, c->stream>>>(c->d_rowptr, c->d_cols, c->d_vals, inv,
+                                                                                   c->ndof);
+  count_launch();
+  IGAP_CHECK_LAUNCH();
+  return IGAPGPU_OK;
+}
+
+}  // namespace igap

@@ -256,9 +256,9 @@ static __global__ void __launch_bounds__(32 * CB_WARPS) cblock_invert_kernel(con
 }
 
 // z = B^-1 v with the inverted cell blocks: a warp per cell, lane a < bs
-// computes the cell's DOF a (grid-stride over cells).
-__device__ __forceinline__ void cblock_apply(double *__restrict__ z, const double *__restrict__ v,
-                                             const double *__restrict__ inv, const CellGeom &g, int64_t ncell)
+// computes the cell's DOF a (grid-stride over cells).  v may have been
+// written earlier in the same kernel (no read-only loads of v here and below).
+__device__ __forceinline__ void cblock_apply(double *z, const double *v, const double *__restrict__ inv, const CellGeom &g, int64_t ncell)
 {
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -276,8 +276,7 @@ __device__ __forceinline__ void cblock_apply(double *__restrict__ z, const doubl
 }
 
 // z = B^-1 v with the inverted blocks
-__device__ __forceinline__ void bdiag_apply(double *__restrict__ z, const double *__restrict__ v,
-                                            const double *__restrict__ inv, int64_t ncp)
+__device__ __forceinline__ void bdiag_apply(double *z, const double *v, const double *__restrict__ inv, int64_t ncp)
 {
   for (int64_t cp = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; cp < ncp;
        cp += (int64_t)gridDim.x * blockDim.x) {
