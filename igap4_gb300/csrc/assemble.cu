@@ -8,15 +8,20 @@
 //               geometry, physical derivatives, interpolated state, law.
 //   Phase B1 -- M[(d,k),(c,e)] = sum_l Dw[(d,k),(e,l)] R[c,l]   (27 x 81)
 //   Phase B2 -- thread (b<=c) accumulates K[(b,.),(c,.)] += R[b,k] M[.,(c,.)]
-//   Scatter  -- colour-partitioned: elements of one colour
-//               (ex mod 3, ey mod 3, ez mod 3) share no control point, so the
-//               CSR slots and residual rows they add into are disjoint.
+//   Output   -- the element's sums and matrix blocks go to element buffers,
+//               all elements in one launch, and a gather adds them (gather.cu);
+//               without room for the buffers, and in batches, a scatter
+//               colour by colour: elements of one colour (ex mod 3, ey mod 3,
+//               ez mod 3) share no control point, so the CSR slots and
+//               residual rows they add into are disjoint.  The sums carry the
+//               same bits either way.
 // Slots are computed arithmetically from the clipped structured stencil.
 #include <cuda_runtime.h>
 #include <stdlib.h>
 #include "common.cuh"
 #include "laws.cuh"
 #include "element.cuh"
+#include "gather.cuh"
 #include "law_thread.cuh"
 
 namespace igap {
@@ -114,10 +119,13 @@ __device__ __forceinline__ double *dw_ptr(typename ElemCfg<TAN>::Smem &S, int w)
   else return nullptr;
 }
 
-// One element: load, quadrature (phase A, B1, B2) and the scatter into RR /
-// vals.  COH: the read-modify-write of RR / vals bypasses L1 (a batched
-// launch orders colours inside one kernel, through L2).
-template <int LAWK, bool RES, bool TAN, bool COH>
+// Where an element's results go: added into RR / vals (a colour launch), the
+// same with reads that bypass L1 (a batched launch orders colours inside one
+// kernel, through L2), or stored to the element's buffers RR[81] / vals[EBUF].
+enum ElemOut { OUT_ADD, OUT_ADD_COHERENT, OUT_BUFFER };
+
+// One element: load, quadrature (phase A, B1, B2) and the output.
+template <int LAWK, bool RES, bool TAN, ElemOut OUT>
 __device__ __forceinline__ void element_body(typename ElemCfg<TAN>::Smem &S, LawSmem<LAWK> &LS, const DevMesh &m,
                                              const DevLaw &L, int ex, int ey, int ez,
                                              const double *__restrict__ Uhist, double *__restrict__ RR,
@@ -258,7 +266,15 @@ __device__ __forceinline__ void element_body(typename ElemCfg<TAN>::Smem &S, Law
         acc[3 * d + e] = k1 + l2 * k2;
       }
   }
+  if constexpr (OUT == OUT_BUFFER) {
+    if (RES && tid < NE) RR[tid] = racc;
+    if (TAN && tid < NPAIR)
+#pragma unroll
+      for (int i = 0; i < 9; i++) vals[9 * tid + i] = acc[i];  // the pair tables run row by row, as pair_index
+    return;
+  }
   // scatter (conflict-free within a colour)
+  constexpr bool COH = OUT == OUT_ADD_COHERENT;
   const int nbv[3] = {m.nbasis[0], nb1, nb2};
   if (RES && tid < NE) {
     const int bb = tid / 3, d = tid % 3;
@@ -301,7 +317,23 @@ __global__ void __launch_bounds__(ElemCfg<TAN>::NT, ElemCfg<TAN>::MINB)
   // element of this colour
   const int b = blockIdx.x;
   const int iz = b % ncz, iy = (b / ncz) % ncy, ix = b / (ncz * ncy);
-  element_body<LAWK, RES, TAN, false>(S, LS, m, L, cx + 3 * ix, cy + 3 * iy, cz + 3 * iz, Uhist, RR, vals);
+  element_body<LAWK, RES, TAN, OUT_ADD>(S, LS, m, L, cx + 3 * ix, cy + 3 * iy, cz + 3 * iz, Uhist, RR, vals);
+}
+
+// Every element in one launch, results to the element buffers.
+template <int LAWK, bool RES, bool TAN>
+__global__ void __launch_bounds__(ElemCfg<TAN>::NT, ElemCfg<TAN>::MINB)
+    element_buffer_kernel(DevMesh m, DevLaw L, const double *__restrict__ Uhist, double *__restrict__ rbuf,
+                          double *__restrict__ ebuf)
+{
+  using Smem = typename ElemCfg<TAN>::Smem;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem &S = *reinterpret_cast<Smem *>(smem_raw);
+  LawSmem<LAWK> &LS = *reinterpret_cast<LawSmem<LAWK> *>(smem_raw + sizeof(Smem));
+  const int64_t e = blockIdx.x;
+  const int ez = (int)(e % m.nelem[2]), ey = (int)((e / m.nelem[2]) % m.nelem[1]),
+            ex = (int)(e / ((int64_t)m.nelem[1] * m.nelem[2]));
+  element_body<LAWK, RES, TAN, OUT_BUFFER>(S, LS, m, L, ex, ey, ez, Uhist, rbuf + e * NE, ebuf + e * EBUF);
 }
 
 // ------------------------------------------------- batched (persistent)
@@ -389,7 +421,7 @@ __global__ void __launch_bounds__(ElemCfg<TAN>::NT, ElemCfg<TAN>::MINB)
       }
       __syncthreads();
       if (s_abort) break;
-      element_body<LAWK, RES, TAN, true>(S, LS, m, L, w.ex, w.eyz >> 16, w.eyz & 0xffff, Uhist, RR, vals);
+      element_body<LAWK, RES, TAN, OUT_ADD_COHERENT>(S, LS, m, L, w.ex, w.eyz >> 16, w.eyz & 0xffff, Uhist, RR, vals);
       __syncthreads();
       if (tid == 0) release_add(a.done + w.inst, 1);
     }
@@ -852,15 +884,20 @@ int launch_law_points(Context *c, bool do_res, bool do_tan, DevLaw &L)
   return IGAPGPU_OK;
 }
 
+// Residual and/or tangent of the FP64 element kernel: through the element
+// buffers in one launch and a gather, else (no room for them) colour by colour.
 template <int LAWK, bool RES, bool TAN>
-static int run_colours(Context *c, const DevLaw &L, double *RR, double *vals)
+static int run_elements(Context *c, const DevLaw &L, double *RR, double *vals)
 {
   const DevMesh m = c->devmesh();
   const size_t smem = sizeof(typename ElemCfg<TAN>::Smem) + sizeof(LawSmem<LAWK>);
+  const bool buffered = (!RES || ensure_rbuf(c)) && (!TAN || ensure_ebuf(c));
   auto kern = element_kernel<LAWK, RES, TAN>;
+  auto bkern = element_buffer_kernel<LAWK, RES, TAN>;
   static bool attr_set = false;
   if (!attr_set) {
     IGAP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    IGAP_CUDA(cudaFuncSetAttribute(bkern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set = true;
   }
   cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -869,24 +906,39 @@ static int run_colours(Context *c, const DevLaw &L, double *RR, double *vals)
     IGAP_CUDA(cudaEventCreate(&e1));
     IGAP_CUDA(cudaEventRecord(e0, c->stream));
   }
-  for (int cx = 0; cx < 3; cx++)
-    for (int cy = 0; cy < 3; cy++)
-      for (int cz = 0; cz < 3; cz++) {
-        const int ncx = (c->nelem[0] - cx + 2) / 3, ncy = (c->nelem[1] - cy + 2) / 3,
-                  ncz = (c->nelem[2] - cz + 2) / 3;
-        const int nblk = ncx * ncy * ncz;
-        if (nblk <= 0) continue;
-        kern<<<nblk, ElemCfg<TAN>::NT, smem, c->stream>>>(m, L, cx, cy, cz, ncy, ncz, c->d_Uhist, RR, vals);
-        count_launch();
-        IGAP_CHECK_LAUNCH();
-        if (c->prof) {
-          c->prof_launches[0]++;
-          c->prof_elements[0] += nblk;
-        }
-      }
+  auto count = [&](int64_t nblk) {
+    count_launch();
+    if (c->prof) {
+      c->prof_launches[0]++;
+      c->prof_elements[0] += nblk;
+    }
+  };
+  if (buffered) {
+    bkern<<<(unsigned)c->nelem_total, ElemCfg<TAN>::NT, smem, c->stream>>>(m, L, c->d_Uhist, c->d_rbuf, c->d_ebuf);
+    IGAP_CHECK_LAUNCH();
+    count(c->nelem_total);
+  } else {
+    if (RES)
+      IGAP_CUDA(cudaMemcpyAsync(RR, c->d_Fneu, sizeof(double) * c->ndof, cudaMemcpyDeviceToDevice, c->stream));
+    if (TAN) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
+    for (int col = 0; col < 27; col++) {
+      const int cx = col / 9, cy = (col / 3) % 3, cz = col % 3;
+      const int ncx = (c->nelem[0] - cx + 2) / 3, ncy = (c->nelem[1] - cy + 2) / 3, ncz = (c->nelem[2] - cz + 2) / 3;
+      const int nblk = ncx * ncy * ncz;
+      if (nblk <= 0) continue;
+      kern<<<nblk, ElemCfg<TAN>::NT, smem, c->stream>>>(m, L, cx, cy, cz, ncy, ncz, c->d_Uhist, RR, vals);
+      IGAP_CHECK_LAUNCH();
+      count(nblk);
+    }
+  }
   if (c->prof) {
     IGAP_CUDA(cudaEventRecord(e1, c->stream));
     c->prof_ev[0].emplace_back(e0, e1);
+  }
+  if (buffered) {
+    int r = RES ? launch_residual_gather(c, RR) : IGAPGPU_OK;
+    if (!r && TAN) r = launch_tangent_gather(c, vals);
+    return r;
   }
   return IGAPGPU_OK;
 }
@@ -970,15 +1022,10 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
   if (rc) return rc;
   if (c->batch) return launch_batch_assembly(c, do_res, do_tan, RR, vals);
   if (c->porder == 3) return launch_assembly_p3(c, do_res, do_tan, RR, vals);
-  if (do_res) {
-    IGAP_CUDA(cudaMemcpyAsync(RR, c->d_Fneu, sizeof(double) * c->ndof, cudaMemcpyDeviceToDevice,
-                              c->stream));
-  }
-  if (do_tan) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
 #define IGAP_DISPATCH(LK)                                                   \
-  if (do_res && do_tan) rc = run_colours<LK, true, true>(c, L, RR, vals);   \
-  else if (do_res) rc = run_colours<LK, true, false>(c, L, RR, vals);       \
-  else rc = run_colours<LK, false, true>(c, L, RR, vals);
+  if (do_res && do_tan) rc = run_elements<LK, true, true>(c, L, RR, vals);   \
+  else if (do_res) rc = run_elements<LK, true, false>(c, L, RR, vals);       \
+  else rc = run_elements<LK, false, true>(c, L, RR, vals);
   // split precision: the tangent goes to the tensor cores (TF32x3);
   // FP64-quality tensor-core precision: the linear law's tangent from BF16
   // slices when they were built, else the FP64 kernel; the residual of both
@@ -996,6 +1043,7 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
   const bool law_df = do_res && c->law_df && c->pre_state == 1;
   const bool df_res = do_res && c->prec != IGAPGPU_PREC_FP64 && (c->d_rpc || law_df);
   if (df_res) {
+    IGAP_CUDA(cudaMemcpyAsync(RR, c->d_Fneu, sizeof(double) * c->ndof, cudaMemcpyDeviceToDevice, c->stream));
     rc = law_df ? launch_res_law_df(c, c->d_preR, RR) : launch_res_df(c, RR);
     if (rc) return rc;
   }
@@ -1016,6 +1064,7 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
 #undef IGAP_DISPATCH
   if (rc) return rc;
   if (do_tan && !fp64_tan) {
+    IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
     IGAP_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     rc = oz_tan ? launch_tc_ozaki(c, vals) : launch_tc_tangent(c, vals, L);
     if (rc) return rc;

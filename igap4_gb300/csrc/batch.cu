@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gather.cuh"
 
 namespace igap {
 
@@ -53,6 +54,7 @@ struct Batch {
   int64_t *d_eoff = nullptr;  // [n+1] element offsets (double-FP32 residual)
   float2 *d_rel = nullptr;    // [elements][81] element residual pairs
   int *d_einst = nullptr;     // [elements] instance of each element
+  int *d_cpinst = nullptr;    // [control points] instance of each (element buffers)
   int rdf_state = -1;         // -1 not decided, 0 off, 1 on
   size_t ctrl_bytes() const { return sizeof(int) * (64 + 2 * (size_t)ninst); }
 };
@@ -304,11 +306,18 @@ void batch_release(Context *c)
   if (!b) return;
   for (Context *s : b->subs) context_free(s);
   void *bufs[] = {b->d_mesh, b->d_law, b->d_items, b->d_ctrl, b->d_need, b->d_dir_inst, b->d_nbs, b->d_off,
-                  b->d_norms, b->d_eoff, b->d_einst, b->d_rel};
+                  b->d_norms, b->d_eoff, b->d_einst, b->d_cpinst, b->d_rel};
   for (void *p : bufs)
     if (p) cudaFree(p);
   delete b;
   c->batch = nullptr;
+}
+
+void batch_gather_map(Context *c, GatherMap *a)
+{
+  a->meshes = c->batch->d_mesh;
+  a->eoff = c->batch->d_eoff;
+  a->cpinst = c->batch->d_cpinst;
 }
 
 // Segment norms: one block per instance, fixed reduction tree.

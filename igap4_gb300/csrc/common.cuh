@@ -169,6 +169,9 @@ struct Context {
   double *d_preR = nullptr;    // law outputs of every point (nonlinear laws, when it fits)
   double *d_preD = nullptr;
   int pre_state = -1;          // -1 not decided, 0 off, 1 on
+  double *d_ebuf = nullptr;    // element matrices [element][EBUF] (gather.cu)
+  double *d_rbuf = nullptr;    // element residuals [element][NE]
+  int ebuf_state = -1, rbuf_state = -1;  // -1 not decided, 0 off, 1 on
   double *d_dens = nullptr;    // per-element density sums + result (igapgpu_density, lazy)
   int *d_dsparse = nullptr;    // sparse constant tangent: dptr | dcol | sptr | sl
   double *d_dval = nullptr;

@@ -1,0 +1,185 @@
+// Element buffers to global vectors: every element's 81 residual sums and the
+// 378 blocks b <= c of its (symmetric) element matrix are written once, all
+// elements in one launch, and a gather adds them per DOF and per CSR slot
+// (the additive phase of src/assmcore_iga.c:240-259, :745-764).
+//
+// The scatter it replaces needs one launch per colour: 27 launches, each as
+// long as its slowest element and, below about 4,000 elements, with fewer
+// elements than SMs.  The gather writes each slot once (no zeroing, no
+// read-modify-write) and adds the contributions in colour order
+// (9 (ex mod 3) + 3 (ey mod 3) + ez mod 3), so the sums carry the same bits as
+// the colour launches.  Two memory passes of 27 KB per element.
+#include <cuda_runtime.h>
+#include <stdlib.h>
+
+#include "common.cuh"
+#include "element.cuh"
+#include "gather.cuh"
+
+namespace igap {
+
+namespace {
+constexpr int TG_THREADS = 128;
+constexpr int TG_NJ = 125;  // control points in a row's stencil
+
+// Elements of one direction that hold both control points i and j, by
+// residue: lo..hi consecutive, at most three.
+struct Range {
+  int lo, n;
+};
+__device__ __forceinline__ Range shared_elements(int i, int j, int ne)
+{
+  const int lo = max(max(i, j) - P, 0), hi = min(min(i, j), ne - 1);
+  return {lo, hi - lo + 1};
+}
+// k-th element of the range in the order of the residues mod 3
+__device__ __forceinline__ int by_residue(Range r, int e)
+{
+  // rank of element e among the range's elements, ordered by e mod 3
+  int rank = 0;
+  for (int k = r.lo; k < r.lo + r.n; k++) rank += (k % 3) < (e % 3) ? 1 : 0;
+  return rank;
+}
+}  // namespace
+
+// One block per control point: a table of the (element, pair) blocks of every
+// slot group (column control point) in shared memory, then a thread per entry
+// of the 3 x 3 blocks (nine consecutive threads read one 72-byte block).
+__global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a, const double *__restrict__ ebuf,
+                                                                    double *__restrict__ vals)
+{
+  __shared__ int tab[TG_NJ * 27];  // (element offset in the patch * 378 + pair) * 2 + transposed
+  __shared__ int64_t ebase[27];    // buffer offset of each element of the patch, -1: outside
+  const int64_t cp = blockIdx.x;
+  const int inst = a.cpinst ? __ldg(a.cpinst + cp) : 0;
+  const DevMesh &m = a.meshes ? a.meshes[inst] : a.m;
+  const int64_t e0 = a.eoff ? __ldg(a.eoff + inst) : 0;
+  const int64_t cpl = cp - m.dof_off / 3;
+  const int nb1 = m.nbasis[1], nb2 = m.nbasis[2];
+  const int ne0 = m.nelem[0], ne1 = m.nelem[1], ne2 = m.nelem[2];
+  const int iz = (int)(cpl % nb2), iy = (int)((cpl / nb2) % nb1), ix = (int)(cpl / ((int64_t)nb1 * nb2));
+  const int lox = max(ix - P, 0), loy = max(iy - P, 0), loz = max(iz - P, 0);
+  const int cy = min(iy + P, nb1 - 1) - loy + 1, cz = min(iz + P, nb2 - 1) - loz + 1;
+  const int nj = (min(ix + P, m.nbasis[0] - 1) - lox + 1) * cy * cz;
+  if (threadIdx.x < 27) {
+    const int ex = ix - threadIdx.x / 9, ey = iy - (threadIdx.x / 3) % 3, ez = iz - threadIdx.x % 3;
+    const bool in = ex >= 0 && ex < ne0 && ey >= 0 && ey < ne1 && ez >= 0 && ez < ne2;
+    ebase[threadIdx.x] = in ? (e0 + ((int64_t)ex * ne1 + ey) * ne2 + ez) * EBUF : -1;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 27 * NB; t += TG_THREADS) {
+    const int b = t / NB, c = t % NB;  // b: this control point's number in the element (and the element's place)
+    if (ebase[b] < 0) continue;
+    const int ex = ix - b / 9, ey = iy - (b / 3) % 3, ez = iz - b % 3;
+    const int jx = ex + c / 9, jy = ey + (c / 3) % 3, jz = ez + c % 3;
+    const Range rx = shared_elements(ix, jx, ne0), ry = shared_elements(iy, jy, ne1), rz = shared_elements(iz, jz, ne2);
+    const int rank = (by_residue(rx, ex) * ry.n + by_residue(ry, ey)) * rz.n + by_residue(rz, ez);
+    const int j = ((jx - lox) * cy + (jy - loy)) * cz + (jz - loz);
+    const int lo = min(b, c), hi = max(b, c);
+    tab[j * 27 + rank] = (b * NPAIRS + pair_index(lo, hi)) * 2 + (b > c ? 1 : 0);
+  }
+  __syncthreads();
+  const int64_t r0 = __ldg(a.rowptr + 3 * cp);
+  for (int t = threadIdx.x; t < 9 * nj; t += TG_THREADS) {
+    const int j = t / 9, q = t % 9, d = q / 3, e = q % 3;
+    const int jz = loz + j % cz, jy = loy + (j / cz) % cy, jx = lox + j / (cz * cy);
+    const int n = shared_elements(ix, jx, ne0).n * shared_elements(iy, jy, ne1).n * shared_elements(iz, jz, ne2).n;
+    const int qt = 3 * e + d;
+    double s = 0.0;
+#pragma unroll 3
+    for (int k = 0; k < n; k++) {
+      const int v = tab[j * 27 + k];
+      const int bp = v >> 1, b = bp / NPAIRS;
+      s += __ldg(ebuf + ebase[b] + (int64_t)(bp - b * NPAIRS) * 9 + ((v & 1) ? qt : q));
+    }
+    vals[r0 + (int64_t)d * 3 * nj + 3 * j + e] = s;
+  }
+}
+
+// RR = load + the element sums of every element that holds the control point.
+__global__ void __launch_bounds__(256) residual_gather_kernel(GatherMap a, const double *__restrict__ rbuf,
+                                                              const double *__restrict__ load, double *__restrict__ RR)
+{
+  const int64_t dof = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (dof >= a.ndof) return;
+  const int64_t cp = dof / 3;
+  const int d = (int)(dof % 3);
+  const int inst = a.cpinst ? __ldg(a.cpinst + cp) : 0;
+  const DevMesh &m = a.meshes ? a.meshes[inst] : a.m;
+  const int64_t e0 = a.eoff ? __ldg(a.eoff + inst) : 0;
+  const int64_t cpl = cp - m.dof_off / 3;
+  const int nb1 = m.nbasis[1], nb2 = m.nbasis[2];
+  const int i[3] = {(int)(cpl / ((int64_t)nb1 * nb2)), (int)((cpl / nb2) % nb1), (int)(cpl % nb2)};
+  double s = load[dof];
+#pragma unroll
+  for (int r = 0; r < 27; r++) {
+    const int rr[3] = {r / 9, (r / 3) % 3, r % 3};
+    int64_t el = 0;
+    int b = 0;
+    bool in = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      // the element of this residue among i - 2 .. i
+      const int e = i[k] - (i[k] + 3 - rr[k]) % 3;
+      in = in && e >= 0 && e < m.nelem[k];
+      el = el * m.nelem[k] + e;
+      b = b * 3 + i[k] - e;
+    }
+    if (in) s += __ldg(rbuf + (e0 + el) * NE + 3 * b + d);
+  }
+  RR[dof] = s;
+}
+
+static GatherMap gather_map(Context *c)
+{
+  GatherMap a;
+  a.m = c->devmesh();
+  a.rowptr = c->d_rowptr;
+  a.ndof = c->ndof;
+  a.meshes = nullptr;
+  a.eoff = nullptr;
+  a.cpinst = nullptr;
+  if (c->batch) batch_gather_map(c, &a);
+  return a;
+}
+
+int launch_tangent_gather(Context *c, double *vals)
+{
+  tangent_gather_kernel<<<(unsigned)(c->ndof / 3), TG_THREADS, 0, c->stream>>>(gather_map(c), c->d_ebuf, vals);
+  count_launch();
+  IGAP_CHECK_LAUNCH();
+  return IGAPGPU_OK;
+}
+
+int launch_residual_gather(Context *c, double *RR)
+{
+  residual_gather_kernel<<<(unsigned)((c->ndof + 255) / 256), 256, 0, c->stream>>>(gather_map(c), c->d_rbuf, c->d_Fneu,
+                                                                                  RR);
+  count_launch();
+  IGAP_CHECK_LAUNCH();
+  return IGAPGPU_OK;
+}
+
+// Allocated at the first use outside a capture; a buffer that would leave less
+// than 4 GB free is not, and the colour launches stay in use.
+static bool ensure_buffer(Context *c, double **p, int *state, size_t per_element)
+{
+  if (*state >= 0) return *state == 1;
+  if (c->capturing) return false;
+  *state = 0;
+  const size_t bytes = sizeof(double) * per_element * (size_t)c->nelem_total;
+  size_t freeb = 0, totb = 0;
+  if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess || bytes + ((size_t)4 << 30) > freeb) return false;
+  if (cudaMalloc(p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+    return false;
+  }
+  *state = 1;
+  return true;
+}
+
+bool ensure_ebuf(Context *c) { return ensure_buffer(c, &c->d_ebuf, &c->ebuf_state, EBUF); }
+bool ensure_rbuf(Context *c) { return ensure_buffer(c, &c->d_rbuf, &c->rbuf_state, NE); }
+
+}  // namespace igap

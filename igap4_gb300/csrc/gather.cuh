@@ -1,0 +1,30 @@
+// Element buffers and their gather (gather.cu).
+#pragma once
+#include "common.cuh"
+
+namespace igap {
+
+constexpr int NPAIRS = NB * (NB + 1) / 2;  // 378 basis pairs b <= c
+constexpr int EBUF = NPAIRS * 9;           // doubles of one element's matrix: 3 x 3 blocks [pair][d][e]
+
+// Number of pair (b, c), b <= c, row by row.
+__host__ __device__ constexpr int pair_index(int b, int c) { return b * NB - b * (b - 1) / 2 + c - b; }
+
+struct GatherMap {
+  DevMesh m;
+  const int64_t *rowptr;
+  int64_t ndof;
+  // batches: mesh and first element of every instance, instance of every control point
+  const DevMesh *meshes;
+  const int64_t *eoff;
+  const int *cpinst;
+};
+
+// Buffers of the context ([element][EBUF], [element][NE]); false: not available.
+bool ensure_ebuf(Context *c);
+bool ensure_rbuf(Context *c);
+int launch_tangent_gather(Context *c, double *vals);
+int launch_residual_gather(Context *c, double *RR);
+void batch_gather_map(Context *c, GatherMap *a);
+
+}  // namespace igap
