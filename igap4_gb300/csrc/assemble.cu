@@ -1047,7 +1047,9 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
     rc = law_df ? launch_res_law_df(c, c->d_preR, RR) : launch_res_df(c, RR);
     if (rc) return rc;
   }
-  const bool k_res = do_res && !df_res, k_tan = fp64_tan;
+  // the linear law's FP64 tangent on the tensor cores where its slices are built
+  const bool x_tan = fp64_tan && ensure_exact(c);
+  const bool k_res = do_res && !df_res, k_tan = fp64_tan && !x_tan;
   if (k_res || k_tan) {
     const bool do_res_k = k_res, do_tan_k = k_tan;
     {
@@ -1063,6 +1065,7 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
   }
 #undef IGAP_DISPATCH
   if (rc) return rc;
+  if (x_tan && (rc = launch_exact_tangent(c, vals))) return rc;
   if (do_tan && !fp64_tan) {
     IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
     IGAP_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));

@@ -54,6 +54,7 @@ struct Batch {
   int64_t *d_eoff = nullptr;  // [n+1] element offsets (double-FP32 residual)
   float2 *d_rel = nullptr;    // [elements][81] element residual pairs
   int *d_einst = nullptr;     // [elements] instance of each element
+  int tables = -1;            // the two tables and d_eoff: -1 not built, 0 no memory, 1 built
   int *d_cpinst = nullptr;    // [control points] instance of each (element buffers)
   int rdf_state = -1;         // -1 not decided, 0 off, 1 on
   size_t ctrl_bytes() const { return sizeof(int) * (64 + 2 * (size_t)ninst); }
@@ -168,6 +169,54 @@ static int check_err_word(Context *c)
   return IGAPGPU_OK;
 }
 
+// Instance of every element and control point, for kernels over the whole
+// batch; built once.
+static bool batch_tables(Context *c)
+{
+  Batch *b = c->batch;
+  if (b->tables >= 0) return b->tables == 1;
+  if (c->capturing) return false;
+  b->tables = 0;
+  const int64_t nel = b->elem_off[b->ninst], ncp = c->ndof / 3;
+  std::vector<int> einst((size_t)nel), cpinst((size_t)ncp);
+  for (int i = 0; i < b->ninst; i++) {
+    std::fill(einst.begin() + b->elem_off[i], einst.begin() + b->elem_off[i + 1], i);
+    std::fill(cpinst.begin() + b->dof_off[i] / 3, cpinst.begin() + b->dof_off[i + 1] / 3, i);
+  }
+  if (cudaMalloc(&b->d_eoff, sizeof(int64_t) * (b->ninst + 1)) == cudaSuccess &&
+      cudaMalloc(&b->d_einst, sizeof(int) * (size_t)nel) == cudaSuccess &&
+      cudaMalloc(&b->d_cpinst, sizeof(int) * (size_t)ncp) == cudaSuccess &&
+      cudaMemcpy(b->d_eoff, b->elem_off.data(), sizeof(int64_t) * (b->ninst + 1), cudaMemcpyHostToDevice) ==
+          cudaSuccess &&
+      cudaMemcpy(b->d_einst, einst.data(), sizeof(int) * (size_t)nel, cudaMemcpyHostToDevice) == cudaSuccess &&
+      cudaMemcpy(b->d_cpinst, cpinst.data(), sizeof(int) * (size_t)ncp, cudaMemcpyHostToDevice) == cudaSuccess) {
+    b->tables = 1;
+    return true;
+  }
+  cudaGetLastError();
+  void **bufs[] = {(void **)&b->d_eoff, (void **)&b->d_einst, (void **)&b->d_cpinst};
+  for (void **p : bufs) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+  return false;
+}
+
+bool batch_instances(Context *c, std::vector<Context *> *subs, std::vector<int64_t> *off)
+{
+  Batch *b = c->batch;
+  if (!batch_tables(c)) return false;
+  *subs = b->subs;
+  off->assign(b->elem_off.begin(), b->elem_off.end() - 1);
+  return true;
+}
+
+void batch_law_map(Context *c, const DevLaw **laws, const int **einst)
+{
+  *laws = c->batch->d_law;
+  *einst = c->batch->d_einst;
+}
+
 // The linear law's residual in the split mode in double-FP32 arithmetic
 // (res_df.cu) when every instance has its FP64 geometry cache and the
 // element-residual buffer fits (IGAPGPU_RES_DF=0 keeps the FP64 kernel).
@@ -182,25 +231,12 @@ static void batch_res_df_setup(Context *c)
   bool ok = !(env && env[0] == '0') && c->law == IGAPGPU_LAW_LINGRAD;
   for (Context *s : b->subs) ok = ok && s->d_geo != nullptr;
   if (!ok) return;
-  const int64_t nel = b->elem_off[b->ninst];
-  std::vector<int> einst((size_t)nel);
-  for (int i = 0; i < b->ninst; i++)
-    for (int64_t g = b->elem_off[i]; g < b->elem_off[i + 1]; g++) einst[(size_t)g] = i;
-  if (cudaMalloc(&b->d_eoff, sizeof(int64_t) * (b->ninst + 1)) == cudaSuccess &&
-      cudaMalloc(&b->d_einst, sizeof(int) * (size_t)nel) == cudaSuccess &&
-      cudaMalloc(&b->d_rel, sizeof(float2) * NE * (size_t)nel) == cudaSuccess &&
-      cudaMemcpy(b->d_eoff, b->elem_off.data(), sizeof(int64_t) * (b->ninst + 1), cudaMemcpyHostToDevice) ==
-          cudaSuccess &&
-      cudaMemcpy(b->d_einst, einst.data(), sizeof(int) * (size_t)nel, cudaMemcpyHostToDevice) == cudaSuccess) {
+  if (!batch_tables(c)) return;
+  if (cudaMalloc(&b->d_rel, sizeof(float2) * NE * (size_t)b->elem_off[b->ninst]) == cudaSuccess) {
     b->rdf_state = 1;
     return;
   }
   cudaGetLastError();
-  void *bufs[] = {b->d_eoff, b->d_einst, b->d_rel};
-  for (void *p : bufs)
-    if (p) cudaFree(p);
-  b->d_eoff = nullptr;
-  b->d_einst = nullptr;
   b->d_rel = nullptr;
 }
 
@@ -228,9 +264,18 @@ static int batch_kernels(Context *c, bool do_res, bool do_tan, double *RR, doubl
       if (r) return r;
     }
   }
-  if ((do_res || fp64_tan) && (which & 1)) {
+  // the linear law's FP64 tangent of the whole queue on the tensor cores
+  bool fp64_queue = fp64_tan;
+  if (fp64_tan && nitems == b->nitems && ensure_exact(c)) {
+    fp64_queue = false;
+    if (which & 1) {
+      int r = launch_exact_tangent(c, vals);
+      if (r) return r;
+    }
+  }
+  if ((do_res || fp64_queue) && (which & 1)) {
     int grid = 0;
-    int r = fp64_grid(c, do_res, fp64_tan, &grid);
+    int r = fp64_grid(c, do_res, fp64_queue, &grid);
     if (r) return r;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (c->prof) {
@@ -238,7 +283,7 @@ static int batch_kernels(Context *c, bool do_res, bool do_tan, double *RR, doubl
       IGAP_CUDA(cudaEventCreate(&e1));
       IGAP_CUDA(cudaEventRecord(e0, c->stream));
     }
-    r = launch_element_batch(c, batch_args(c, 0, nitems), c->law, do_res, fp64_tan, grid, c->d_Uhist, RR,
+    r = launch_element_batch(c, batch_args(c, 0, nitems), c->law, do_res, fp64_queue, grid, c->d_Uhist, RR,
                              vals);
     if (r) return r;
     if (c->prof) {
@@ -275,7 +320,8 @@ int launch_batch_assembly(Context *c, bool do_res, bool do_tan, double *RR, doub
   Batch *b = c->batch;
   if (do_res)
     IGAP_CUDA(cudaMemcpyAsync(RR, c->d_Fneu, sizeof(double) * c->ndof, cudaMemcpyDeviceToDevice, c->stream));
-  if (do_tan) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
+  const bool gathered = do_tan && c->prec != IGAPGPU_PREC_SPLIT && ensure_exact(c);  // every slot written
+  if (do_tan && !gathered) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
   int r = batch_kernels(c, do_res, do_tan, RR, vals, b->nitems);
   if (r) return r;
   if (do_res && (r = launch_dirichlet_residual(c, RR))) return r;
@@ -654,7 +700,7 @@ int igapgpu_batch_autotune(igapgpu_t c, int reps, double frac, igapgpu_batch_sch
   Batch *b = c->batch;
   const bool split = c->prec == IGAPGPU_PREC_SPLIT;
   // the FP64 kernel computes the residual (and, in FP64 mode, the tangent)
-  const bool tan64 = !split;
+  const bool tan64 = !split && !ensure_exact(c);
   int occ = 1;
   int r = element_batch_occupancy(c->law, true, tan64, &occ);
   if (r) return r;

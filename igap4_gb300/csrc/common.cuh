@@ -172,6 +172,11 @@ struct Context {
   double *d_ebuf = nullptr;    // element matrices [element][EBUF] (gather.cu)
   double *d_rbuf = nullptr;    // element residuals [element][NE]
   int ebuf_state = -1, rbuf_state = -1;  // -1 not decided, 0 off, 1 on
+  void *d_xops = nullptr;      // linear law: 9-bit slices of the Gram operands (FP64 tensor-core tangent)
+  short *d_xexp = nullptr;     // their row exponents
+  double *d_xrow = nullptr;    // row 80 of every element's operand
+  int exact_state = -1;        // -1 not decided, 0 off, 1 on
+  bool exact_ran = false;      // a launch whose error word has not been read yet
   double *d_dens = nullptr;    // per-element density sums + result (igapgpu_density, lazy)
   int *d_dsparse = nullptr;    // sparse constant tangent: dptr | dcol | sptr | sl
   double *d_dval = nullptr;
@@ -266,6 +271,8 @@ Context *new_context(const igapgpu_mesh_desc *mesh, const igapgpu_phys_desc *phy
                      const igapgpu_bc_desc *bc, int nquad);
 int context_init(Context *c, const igapgpu_mesh_desc *mesh);
 int context_free(Context *c);
+// after a synchronisation: the error word of asynchronous kernels with bounded waits
+int check_async_error(Context *c);
 
 // assemble.cu
 int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *vals);
@@ -300,6 +307,9 @@ int launch_assembly_p3(Context *c, bool do_res, bool do_tan, double *RR, double 
 // tc_ozaki.cu (linear law, BF16 slices, FP64-quality)
 int ensure_ozaki_operands(Context *c);
 int launch_tc_ozaki(Context *c, double *vals);
+// tc_exact.cu (linear law, FP64 tangent from exact BF16 slices)
+bool ensure_exact(Context *c);
+int launch_exact_tangent(Context *c, double *vals);
 // res_df.cu (linear law residual in double-FP32 arithmetic)
 int ensure_res_pairs(Context *c);
 int launch_res_df(Context *c, double *RR);
@@ -337,6 +347,9 @@ int launch_batch_assembly(Context *c, bool do_res, bool do_tan, double *RR, doub
 void batch_release(Context *c);
 int batch_set_neumann(Context *c, const double *table);
 int batch_prepare_split(Context *c);
+// instances and their first elements; false without memory for the element tables
+bool batch_instances(Context *c, std::vector<Context *> *subs, std::vector<int64_t> *off);
+void batch_law_map(Context *c, const DevLaw **laws, const int **einst);
 // element kernels over a batch work queue (assemble.cu, tc_tangent.cu)
 int launch_element_batch(Context *c, const BatchArgs &a, int law, bool do_res, bool do_tan, int grid,
                          const double *Uhist, double *RR, double *vals);

@@ -183,7 +183,7 @@ static int free_ctx(Context *c)
   void *bufs[] = {c->d_wq, c->d_xq, c->d_w, c->d_X, c->d_Uhist, c->d_RR, c->d_vals,
                   c->d_rowptr, c->d_cols, c->d_Dconst, c->d_Fneu, c->d_dir_rows, c->d_dir_g,
                   c->d_stage_a, c->d_stage_b, c->d_stage_v, c->d_V, c->d_Z, c->d_work,
-                  c->d_diag, c->d_bdiag, c->d_cinv, c->d_asmz, c->d_red, c->d_partial, c->d_err, c->d_geo, c->d_geof, c->d_gop, c->d_oz, c->d_ozexp, c->d_rpc, c->d_rel, c->d_upair, c->d_lin, c->d_preR, c->d_preD, c->d_ebuf, c->d_rbuf, c->d_dens, c->d_dsparse, c->d_dval, c->d_sval, c->d_bct, c->d_neu};
+                  c->d_diag, c->d_bdiag, c->d_cinv, c->d_asmz, c->d_red, c->d_partial, c->d_err, c->d_geo, c->d_geof, c->d_gop, c->d_oz, c->d_ozexp, c->d_rpc, c->d_rel, c->d_upair, c->d_lin, c->d_preR, c->d_preD, c->d_ebuf, c->d_rbuf, c->d_xops, c->d_xexp, c->d_xrow, c->d_dens, c->d_dsparse, c->d_dval, c->d_sval, c->d_bct, c->d_neu};
   for (void *b : bufs)
     if (b) cudaFree(b);
   for (int d = 0; d < 3; d++) {
@@ -523,6 +523,19 @@ Context *new_context(const igapgpu_mesh_desc *mesh, const igapgpu_phys_desc *phy
   return c;
 }
 
+int check_async_error(Context *c)
+{
+  if (!c->exact_ran) return IGAPGPU_OK;
+  c->exact_ran = false;
+  int herr = 0;
+  IGAP_CUDA(cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  IGAP_CUDA(cudaStreamSynchronize(c->stream));
+  if (!herr) return IGAPGPU_OK;
+  IGAP_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
+  set_error("tensor-core tangent: a bounded mbarrier wait expired (code %d)", herr);
+  return IGAPGPU_ERR_TIMEOUT;
+}
+
 int context_init(Context *c, const igapgpu_mesh_desc *mesh) { return init_impl(c, mesh); }
 int context_free(Context *c) { return free_ctx(c); }
 
@@ -725,7 +738,10 @@ static int assemble_common(igapgpu_t c, const double *U, double *RR, double *val
   if (do_tan && v_dev == c->d_vals) c->matrix_valid = true;
   if (rr_host) IGAP_CUDA(cudaMemcpyAsync(RR, rr_dev, sizeof(double) * c->ndof, cudaMemcpyDeviceToHost, c->stream));
   if (v_host) IGAP_CUDA(cudaMemcpyAsync(vals, v_dev, sizeof(double) * c->nnz, cudaMemcpyDeviceToHost, c->stream));
-  if (rr_host || v_host || (U && !is_device_ptr(U))) IGAP_CUDA(cudaStreamSynchronize(c->stream));
+  if (rr_host || v_host || (U && !is_device_ptr(U))) {
+    IGAP_CUDA(cudaStreamSynchronize(c->stream));
+    return check_async_error(c);
+  }
   return IGAPGPU_OK;
 }
 
@@ -856,7 +872,7 @@ int igapgpu_synchronize(igapgpu_t c)
 {
   if (!c) return IGAPGPU_ERR_ARG;
   IGAP_CUDA(cudaStreamSynchronize(c->stream));
-  return IGAPGPU_OK;
+  return check_async_error(c);
 }
 
 }  // extern "C"

@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a,
   }
   __syncthreads();
   const int64_t r0 = __ldg(a.rowptr + 3 * cp);
+  const bool failed = a.err && *a.err;
   for (int t = threadIdx.x; t < 9 * nj; t += TG_THREADS) {
     const int j = t / 9, q = t % 9, d = q / 3, e = q % 3;
     const int jz = loz + j % cz, jy = loy + (j / cz) % cy, jx = lox + j / (cz * cy);
@@ -92,7 +93,7 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a,
       const int bp = v >> 1, b = bp / NPAIRS;
       s += __ldg(ebuf + ebase[b] + (int64_t)(bp - b * NPAIRS) * 9 + ((v & 1) ? qt : q));
     }
-    vals[r0 + (int64_t)d * 3 * nj + 3 * j + e] = s;
+    vals[r0 + (int64_t)d * 3 * nj + 3 * j + e] = failed ? __longlong_as_double(0x7ff8000000000000ll) : s;
   }
 }
 
@@ -139,13 +140,16 @@ static GatherMap gather_map(Context *c)
   a.meshes = nullptr;
   a.eoff = nullptr;
   a.cpinst = nullptr;
+  a.err = nullptr;
   if (c->batch) batch_gather_map(c, &a);
   return a;
 }
 
-int launch_tangent_gather(Context *c, double *vals)
+int launch_tangent_gather(Context *c, double *vals, const int *err)
 {
-  tangent_gather_kernel<<<(unsigned)(c->ndof / 3), TG_THREADS, 0, c->stream>>>(gather_map(c), c->d_ebuf, vals);
+  GatherMap a = gather_map(c);
+  a.err = err;
+  tangent_gather_kernel<<<(unsigned)(c->ndof / 3), TG_THREADS, 0, c->stream>>>(a, c->d_ebuf, vals);
   count_launch();
   IGAP_CHECK_LAUNCH();
   return IGAPGPU_OK;

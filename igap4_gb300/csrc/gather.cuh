@@ -18,12 +18,13 @@ struct GatherMap {
   const DevMesh *meshes;
   const int64_t *eoff;
   const int *cpinst;
+  const int *err;  // error word of the element kernel: NaN is written when it is set (or null)
 };
 
 // Buffers of the context ([element][EBUF], [element][NE]); false: not available.
 bool ensure_ebuf(Context *c);
 bool ensure_rbuf(Context *c);
-int launch_tangent_gather(Context *c, double *vals);
+int launch_tangent_gather(Context *c, double *vals, const int *err = nullptr);
 int launch_residual_gather(Context *c, double *RR);
 void batch_gather_map(Context *c, GatherMap *a);
 

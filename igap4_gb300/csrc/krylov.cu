@@ -639,7 +639,7 @@ int igapgpu_solve(igapgpu_t c, double *U, const igapgpu_solver_opts *opts, igapg
   }
   IGAP_CUDA(cudaStreamSynchronize(c->stream));
   if (st) *st = S;
-  return IGAPGPU_OK;
+  return check_async_error(c);
 }
 
 }  // extern "C"
