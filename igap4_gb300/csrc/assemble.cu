@@ -1067,9 +1067,10 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
   if (rc) return rc;
   if (x_tan && (rc = launch_exact_tangent(c, vals))) return rc;
   if (do_tan && !fp64_tan) {
-    IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
+    const bool gathered = !oz_tan && tc_law_applies(c, L);  // every slot is written
+    if (!gathered) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
     IGAP_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    rc = oz_tan ? launch_tc_ozaki(c, vals) : launch_tc_tangent(c, vals, L);
+    rc = oz_tan ? launch_tc_ozaki(c, vals) : gathered ? launch_tc_law(c, vals, L) : launch_tc_tangent(c, vals, L);
     if (rc) return rc;
     if (!c->capturing) {  // a graph replay checks the error word itself
       int herr = 0;

@@ -171,7 +171,8 @@ struct Context {
   int pre_state = -1;          // -1 not decided, 0 off, 1 on
   double *d_ebuf = nullptr;    // element matrices [element][EBUF] (gather.cu)
   double *d_rbuf = nullptr;    // element residuals [element][NE]
-  int ebuf_state = -1, rbuf_state = -1;  // -1 not decided, 0 off, 1 on
+  float *d_fbuf = nullptr;     // FP32 element matrices [element][27][243] (split tangent of the reference's laws)
+  int ebuf_state = -1, rbuf_state = -1, fbuf_state = -1;  // -1 not decided, 0 off, 1 on
   void *d_xops = nullptr;      // linear law: 9-bit slices of the Gram operands (FP64 tensor-core tangent)
   short *d_xexp = nullptr;     // their row exponents
   double *d_xrow = nullptr;    // row 80 of every element's operand
@@ -293,6 +294,9 @@ int launch_geometry_cache(Context *c);
 int launch_geometry_cache_f32(Context *c);
 // tc_tangent.cu
 int launch_tc_tangent(Context *c, double *vals, const DevLaw &L);
+// tc_law.cu (the reference's laws from precomputed FP32 law outputs)
+bool tc_law_applies(Context *c, const DevLaw &L);
+int launch_tc_law(Context *c, double *vals, const DevLaw &L);
 // tc_gram.cu (linear isotropic law with the FP32 geometry cache)
 int launch_tc_gram(Context *c, double *vals);
 // cached: every instance has its Gram operands (d_gop); persistent CTAs per SM of nsm

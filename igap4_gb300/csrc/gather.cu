@@ -40,51 +40,86 @@ __device__ __forceinline__ int by_residue(Range r, int e)
   for (int k = r.lo; k < r.lo + r.n; k++) rank += (k % 3) < (e % 3) ? 1 : 0;
   return rank;
 }
-}  // namespace
 
-// One block per control point: a table of the (element, pair) blocks of every
-// slot group (column control point) in shared memory, then a thread per entry
-// of the 3 x 3 blocks (nine consecutive threads read one 72-byte block).
-__global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a, const double *__restrict__ ebuf,
-                                                                    double *__restrict__ vals)
+// A control point's place in its lattice and the elements around it.
+struct Patch {
+  int ix, iy, iz, lox, loy, loz, cy, cz, nj;
+  int ne0, ne1, ne2;
+};
+
+__device__ __forceinline__ Patch patch_of(const DevMesh &m, int64_t cpl)
 {
-  __shared__ int tab[TG_NJ * 27];  // (element offset in the patch * 378 + pair) * 2 + transposed
-  __shared__ int64_t ebase[27];    // buffer offset of each element of the patch, -1: outside
-  const int64_t cp = blockIdx.x;
-  const int inst = a.cpinst ? __ldg(a.cpinst + cp) : 0;
-  const DevMesh &m = a.meshes ? a.meshes[inst] : a.m;
-  const int64_t e0 = a.eoff ? __ldg(a.eoff + inst) : 0;
-  const int64_t cpl = cp - m.dof_off / 3;
+  Patch p;
   const int nb1 = m.nbasis[1], nb2 = m.nbasis[2];
-  const int ne0 = m.nelem[0], ne1 = m.nelem[1], ne2 = m.nelem[2];
-  const int iz = (int)(cpl % nb2), iy = (int)((cpl / nb2) % nb1), ix = (int)(cpl / ((int64_t)nb1 * nb2));
-  const int lox = max(ix - P, 0), loy = max(iy - P, 0), loz = max(iz - P, 0);
-  const int cy = min(iy + P, nb1 - 1) - loy + 1, cz = min(iz + P, nb2 - 1) - loz + 1;
-  const int nj = (min(ix + P, m.nbasis[0] - 1) - lox + 1) * cy * cz;
+  p.ne0 = m.nelem[0];
+  p.ne1 = m.nelem[1];
+  p.ne2 = m.nelem[2];
+  p.iz = (int)(cpl % nb2);
+  p.iy = (int)((cpl / nb2) % nb1);
+  p.ix = (int)(cpl / ((int64_t)nb1 * nb2));
+  p.lox = max(p.ix - P, 0);
+  p.loy = max(p.iy - P, 0);
+  p.loz = max(p.iz - P, 0);
+  p.cy = min(p.iy + P, nb1 - 1) - p.loy + 1;
+  p.cz = min(p.iz + P, nb2 - 1) - p.loz + 1;
+  p.nj = (min(p.ix + P, m.nbasis[0] - 1) - p.lox + 1) * p.cy * p.cz;
+  return p;
+}
+
+// Per column control point j of the row, the (element, function) pairs that
+// contribute, in colour order: tab[27 j + rank] = entry(b, c), ebase[b] the
+// buffer offset of the patch's element in which the row's control point is
+// function b (-1 outside the lattice).
+template <typename F>
+__device__ __forceinline__ void gather_table(const Patch &p, int64_t e0, int64_t per_element, int *tab, int64_t *ebase,
+                                             F entry)
+{
   if (threadIdx.x < 27) {
-    const int ex = ix - threadIdx.x / 9, ey = iy - (threadIdx.x / 3) % 3, ez = iz - threadIdx.x % 3;
-    const bool in = ex >= 0 && ex < ne0 && ey >= 0 && ey < ne1 && ez >= 0 && ez < ne2;
-    ebase[threadIdx.x] = in ? (e0 + ((int64_t)ex * ne1 + ey) * ne2 + ez) * EBUF : -1;
+    const int ex = p.ix - threadIdx.x / 9, ey = p.iy - (threadIdx.x / 3) % 3, ez = p.iz - threadIdx.x % 3;
+    const bool in = ex >= 0 && ex < p.ne0 && ey >= 0 && ey < p.ne1 && ez >= 0 && ez < p.ne2;
+    ebase[threadIdx.x] = in ? (e0 + ((int64_t)ex * p.ne1 + ey) * p.ne2 + ez) * per_element : -1;
   }
   __syncthreads();
   for (int t = threadIdx.x; t < 27 * NB; t += TG_THREADS) {
-    const int b = t / NB, c = t % NB;  // b: this control point's number in the element (and the element's place)
+    const int b = t / NB, c = t % NB;
     if (ebase[b] < 0) continue;
-    const int ex = ix - b / 9, ey = iy - (b / 3) % 3, ez = iz - b % 3;
+    const int ex = p.ix - b / 9, ey = p.iy - (b / 3) % 3, ez = p.iz - b % 3;
     const int jx = ex + c / 9, jy = ey + (c / 3) % 3, jz = ez + c % 3;
-    const Range rx = shared_elements(ix, jx, ne0), ry = shared_elements(iy, jy, ne1), rz = shared_elements(iz, jz, ne2);
+    const Range rx = shared_elements(p.ix, jx, p.ne0), ry = shared_elements(p.iy, jy, p.ne1),
+                rz = shared_elements(p.iz, jz, p.ne2);
     const int rank = (by_residue(rx, ex) * ry.n + by_residue(ry, ey)) * rz.n + by_residue(rz, ez);
-    const int j = ((jx - lox) * cy + (jy - loy)) * cz + (jz - loz);
-    const int lo = min(b, c), hi = max(b, c);
-    tab[j * 27 + rank] = (b * NPAIRS + pair_index(lo, hi)) * 2 + (b > c ? 1 : 0);
+    const int j = ((jx - p.lox) * p.cy + (jy - p.loy)) * p.cz + (jz - p.loz);
+    tab[j * 27 + rank] = entry(b, c);
   }
   __syncthreads();
+}
+
+__device__ __forceinline__ int contributions(const Patch &p, int j)
+{
+  const int jz = p.loz + j % p.cz, jy = p.loy + (j / p.cz) % p.cy, jx = p.lox + j / (p.cz * p.cy);
+  return shared_elements(p.ix, jx, p.ne0).n * shared_elements(p.iy, jy, p.ne1).n * shared_elements(p.iz, jz, p.ne2).n;
+}
+}  // namespace
+
+// One block per control point: the table of its slots, then a thread per
+// entry of the 3 x 3 blocks (nine consecutive threads read one 72-byte block).
+__global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a, const double *__restrict__ ebuf,
+                                                                    double *__restrict__ vals)
+{
+  __shared__ int tab[TG_NJ * 27];  // (function b * 378 + pair) * 2 + transposed
+  __shared__ int64_t ebase[27];
+  const int64_t cp = blockIdx.x;
+  const int inst = a.cpinst ? __ldg(a.cpinst + cp) : 0;
+  const DevMesh &m = a.meshes ? a.meshes[inst] : a.m;
+  const Patch p = patch_of(m, cp - m.dof_off / 3);
+  gather_table(p, a.eoff ? __ldg(a.eoff + inst) : 0, EBUF, tab, ebase, [](int b, int c) {
+    return (b * NPAIRS + pair_index(min(b, c), max(b, c))) * 2 + (b > c ? 1 : 0);
+  });
   const int64_t r0 = __ldg(a.rowptr + 3 * cp);
   const bool failed = a.err && *a.err;
-  for (int t = threadIdx.x; t < 9 * nj; t += TG_THREADS) {
+  for (int t = threadIdx.x; t < 9 * p.nj; t += TG_THREADS) {
     const int j = t / 9, q = t % 9, d = q / 3, e = q % 3;
-    const int jz = loz + j % cz, jy = loy + (j / cz) % cy, jx = lox + j / (cz * cy);
-    const int n = shared_elements(ix, jx, ne0).n * shared_elements(iy, jy, ne1).n * shared_elements(iz, jz, ne2).n;
+    const int n = contributions(p, j);
     const int qt = 3 * e + d;
     double s = 0.0;
 #pragma unroll 3
@@ -93,7 +128,33 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a,
       const int bp = v >> 1, b = bp / NPAIRS;
       s += __ldg(ebuf + ebase[b] + (int64_t)(bp - b * NPAIRS) * 9 + ((v & 1) ? qt : q));
     }
-    vals[r0 + (int64_t)d * 3 * nj + 3 * j + e] = failed ? __longlong_as_double(0x7ff8000000000000ll) : s;
+    vals[r0 + (int64_t)d * 3 * p.nj + 3 * j + e] = failed ? __longlong_as_double(0x7ff8000000000000ll) : s;
+  }
+}
+
+// The same from FP32 element matrices [27 b][3 d][27 c][3 e] (not symmetric to
+// the last bit): a thread per entry of the rows, consecutive threads along
+// the columns, in the buffer as in the CSR rows.
+__global__ void __launch_bounds__(TG_THREADS) tangent_gather_f32_kernel(GatherMap a, const float *__restrict__ fbuf,
+                                                                        double *__restrict__ vals)
+{
+  __shared__ int tab[TG_NJ * 27];  // 27 b + c
+  __shared__ int64_t ebase[27];
+  const int64_t cp = blockIdx.x;
+  const Patch p = patch_of(a.m, cp);
+  gather_table(p, 0, NB * 243, tab, ebase, [](int b, int c) { return NB * b + c; });
+  const int64_t r0 = __ldg(a.rowptr + 3 * cp);
+  const int row = 3 * p.nj;
+  for (int t = threadIdx.x; t < 3 * row; t += TG_THREADS) {
+    const int d = t / row, x = t - d * row, j = x / 3, e = x - 3 * j;
+    const int n = contributions(p, j);
+    double s = 0.0;
+#pragma unroll 3
+    for (int k = 0; k < n; k++) {
+      const int v = tab[j * 27 + k], b = v / NB;
+      s += (double)__ldg(fbuf + ebase[b] + b * 243 + d * 81 + 3 * (v - NB * b) + e);
+    }
+    vals[r0 + t] = s;
   }
 }
 
@@ -155,6 +216,14 @@ int launch_tangent_gather(Context *c, double *vals, const int *err)
   return IGAPGPU_OK;
 }
 
+int launch_tangent_gather_f32(Context *c, double *vals)
+{
+  tangent_gather_f32_kernel<<<(unsigned)(c->ndof / 3), TG_THREADS, 0, c->stream>>>(gather_map(c), c->d_fbuf, vals);
+  count_launch();
+  IGAP_CHECK_LAUNCH();
+  return IGAPGPU_OK;
+}
+
 int launch_residual_gather(Context *c, double *RR)
 {
   residual_gather_kernel<<<(unsigned)((c->ndof + 255) / 256), 256, 0, c->stream>>>(gather_map(c), c->d_rbuf, c->d_Fneu,
@@ -166,12 +235,13 @@ int launch_residual_gather(Context *c, double *RR)
 
 // Allocated at the first use outside a capture; a buffer that would leave less
 // than 4 GB free is not, and the colour launches stay in use.
-static bool ensure_buffer(Context *c, double **p, int *state, size_t per_element)
+template <typename T>
+static bool ensure_buffer(Context *c, T **p, int *state, size_t per_element)
 {
   if (*state >= 0) return *state == 1;
   if (c->capturing) return false;
   *state = 0;
-  const size_t bytes = sizeof(double) * per_element * (size_t)c->nelem_total;
+  const size_t bytes = sizeof(T) * per_element * (size_t)c->nelem_total;
   size_t freeb = 0, totb = 0;
   if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess || bytes + ((size_t)4 << 30) > freeb) return false;
   if (cudaMalloc(p, bytes) != cudaSuccess) {
@@ -184,6 +254,7 @@ static bool ensure_buffer(Context *c, double **p, int *state, size_t per_element
 }
 
 bool ensure_ebuf(Context *c) { return ensure_buffer(c, &c->d_ebuf, &c->ebuf_state, EBUF); }
+bool ensure_fbuf(Context *c) { return ensure_buffer(c, &c->d_fbuf, &c->fbuf_state, NB * 243); }
 bool ensure_rbuf(Context *c) { return ensure_buffer(c, &c->d_rbuf, &c->rbuf_state, NE); }
 
 }  // namespace igap

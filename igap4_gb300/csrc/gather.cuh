@@ -23,8 +23,10 @@ struct GatherMap {
 
 // Buffers of the context ([element][EBUF], [element][NE]); false: not available.
 bool ensure_ebuf(Context *c);
+bool ensure_fbuf(Context *c);  // FP32 [element][27][243]
 bool ensure_rbuf(Context *c);
 int launch_tangent_gather(Context *c, double *vals, const int *err = nullptr);
+int launch_tangent_gather_f32(Context *c, double *vals);
 int launch_residual_gather(Context *c, double *RR);
 void batch_gather_map(Context *c, GatherMap *a);
 
