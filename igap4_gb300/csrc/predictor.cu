@@ -138,6 +138,179 @@ __global__ void __launch_bounds__(256) conv_bwd_weight(const float *__restrict__
   }
 }
 
+// The input and output layers of a BF16 network (9 -> 32 and 32 -> 3) on the
+// FP32 pipe: one output a thread, as above, reads an input and a weight from
+// memory for every FMA (771 us a layer at 130x34x34).  Here a thread holds PT
+// points x CT outputs, the layer's weights are in shared memory as FP32
+// ([tap][ci][CO]), so that an FMA needs 1 / CT of an input load and 1 / PT of
+// a weight load.  Every output takes its products in the order tap, ci, taps
+// outside the lattice left out, as the one-output kernel: the same bits (a
+// BF16 rounding that falls the other way would travel through the layers).
+constexpr int CS_THREADS = 256;
+
+template <int CI, int CO, int PT, int CT>
+__global__ void __launch_bounds__(CS_THREADS) conv_fwd_tile(const __nv_bfloat16 *__restrict__ in,
+                                                            const __nv_bfloat16 *__restrict__ W,
+                                                            const float *__restrict__ bias,
+                                                            __nv_bfloat16 *__restrict__ out, Lattice L, int B, int relu)
+{
+  constexpr int COP = (CO + 3) / 4 * 4, NCG = COP / CT, PG = CS_THREADS / NCG;
+  __shared__ __align__(16) float Ws[27 * CI * COP];
+  for (int i = threadIdx.x; i < 27 * CI * COP; i += CS_THREADS) {
+    const int co = i % COP, tc = i / COP;  // tc = tap * CI + ci
+    Ws[i] = co < CO ? ld(W + (int64_t)co * 27 * CI + tc) : 0.f;
+  }
+  __syncthreads();
+  const int cg = threadIdx.x % NCG, pg = threadIdx.x / NCG;
+  const int64_t total = (int64_t)B * L.P, first = (int64_t)blockIdx.x * (PG * PT) + pg;
+  float acc[PT][CT];
+  const __nv_bfloat16 *x0[PT];
+  int cx[PT], cy[PT], cz[PT];
+#pragma unroll
+  for (int i = 0; i < PT; i++) {
+    const int64_t bp = first + i * PG, p = (bp < total ? bp : 0) % L.P;
+    cz[i] = (int)(p % L.nz);
+    cy[i] = (int)((p / L.nz) % L.ny);
+    cx[i] = bp < total ? (int)(p / ((int64_t)L.ny * L.nz)) : -8;  // every tap outside
+    x0[i] = in + (bp < total ? bp : 0) * CI;
+#pragma unroll
+    for (int c = 0; c < CT; c++) acc[i][c] = cg * CT + c < CO ? bias[cg * CT + c] : 0.f;
+  }
+  for (int t = 0; t < 27; t++) {
+    const int dx = t / 9 - 1, dy = (t / 3) % 3 - 1, dz = t % 3 - 1;
+    const int64_t off = (((int64_t)dx * L.ny + dy) * L.nz + dz) * CI;
+    bool v[PT];
+    const __nv_bfloat16 *x[PT];
+#pragma unroll
+    for (int i = 0; i < PT; i++) {
+      v[i] = (unsigned)(cx[i] + dx) < (unsigned)L.nx && (unsigned)(cy[i] + dy) < (unsigned)L.ny &&
+             (unsigned)(cz[i] + dz) < (unsigned)L.nz;
+      x[i] = v[i] ? x0[i] + off : x0[i];
+    }
+    const float *w = Ws + t * CI * COP + cg * CT;
+    constexpr int STEP = CI % 8 == 0 ? 8 : CI;  // 16-byte loads of 8 channels where rows are aligned
+#pragma unroll 1
+    for (int c0 = 0; c0 < CI; c0 += STEP) {
+      float xv[PT][STEP];
+#pragma unroll
+      for (int i = 0; i < PT; i++) {
+        if constexpr (STEP == 8) {
+          const uint4 u = __ldg(reinterpret_cast<const uint4 *>(x[i] + c0));
+          const uint32_t h[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            xv[i][2 * k] = __uint_as_float(h[k] << 16);
+            xv[i][2 * k + 1] = __uint_as_float(h[k] & 0xffff0000u);
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < STEP; k++) xv[i][k] = ld(x[i] + c0 + k);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < STEP; k++) {
+        float wv[CT];
+#pragma unroll
+        for (int c = 0; c < CT; c += 4) {
+          const float4 u = *reinterpret_cast<const float4 *>(w + (c0 + k) * COP + c);
+          wv[c] = u.x;
+          wv[c + 1] = u.y;
+          wv[c + 2] = u.z;
+          wv[c + 3] = u.w;
+        }
+#pragma unroll
+        for (int i = 0; i < PT; i++)
+          if (v[i])
+#pragma unroll
+            for (int c = 0; c < CT; c++) acc[i][c] = fmaf(wv[c], xv[i][k], acc[i][c]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < PT; i++) {
+    const int64_t bp = first + i * PG;
+    if (bp >= total) continue;
+#pragma unroll
+    for (int c = 0; c < CT; c++) {
+      if (cg * CT + c >= CO) continue;
+      float a = acc[i][c];
+      if (relu && a < 0.f) a = 0.f;
+      out[bp * CO + cg * CT + c] = cvt<__nv_bfloat16>(a);
+    }
+  }
+}
+
+// Data gradient of the 32 -> 3 output layer the same way: PT points x CT of
+// the 32 input channels a thread, products in the order tap, co (FP32 output
+// gradient, BF16 weights in shared memory as FP32).
+template <int PT, int CT>
+__global__ void __launch_bounds__(CS_THREADS) conv_bwd_data_out(const float *__restrict__ dZ,
+                                                                const __nv_bfloat16 *__restrict__ W,
+                                                                float *__restrict__ dIn, Lattice L, int B)
+{
+  constexpr int CO = 3, CI = 32, NCG = CI / CT, PG = CS_THREADS / NCG;
+  __shared__ __align__(16) float Ws[27 * CO * CI];
+  for (int i = threadIdx.x; i < 27 * CO * CI; i += CS_THREADS) {
+    const int ci = i % CI, co = (i / CI) % CO, t = i / (CI * CO);
+    Ws[i] = ld(W + ((int64_t)co * 27 + t) * CI + ci);
+  }
+  __syncthreads();
+  const int cg = threadIdx.x % NCG, pg = threadIdx.x / NCG;
+  const int64_t total = (int64_t)B * L.P, first = (int64_t)blockIdx.x * (PG * PT) + pg;
+  float acc[PT][CT];
+  int64_t row[PT];
+  int cx[PT], cy[PT], cz[PT];
+#pragma unroll
+  for (int i = 0; i < PT; i++) {
+    const int64_t bp = first + i * PG, p = (bp < total ? bp : 0) % L.P;
+    cz[i] = (int)(p % L.nz);
+    cy[i] = (int)((p / L.nz) % L.ny);
+    cx[i] = bp < total ? (int)(p / ((int64_t)L.ny * L.nz)) : -8;
+    row[i] = bp < total ? bp : 0;
+#pragma unroll
+    for (int c = 0; c < CT; c++) acc[i][c] = 0.f;
+  }
+  for (int t = 0; t < 27; t++) {
+    const int dx = 1 - t / 9, dy = 1 - (t / 3) % 3, dz = 1 - t % 3;  // q = p - offset(t)
+    const int64_t off = ((int64_t)dx * L.ny + dy) * L.nz + dz;
+    bool v[PT];
+    float z[PT][CO];
+#pragma unroll
+    for (int i = 0; i < PT; i++) {
+      v[i] = (unsigned)(cx[i] + dx) < (unsigned)L.nx && (unsigned)(cy[i] + dy) < (unsigned)L.ny &&
+             (unsigned)(cz[i] + dz) < (unsigned)L.nz;
+      const float *src = dZ + (v[i] ? row[i] + off : row[i]) * CO;
+#pragma unroll
+      for (int co = 0; co < CO; co++) z[i][co] = __ldg(src + co);
+    }
+#pragma unroll
+    for (int co = 0; co < CO; co++) {
+      float wv[CT];
+#pragma unroll
+      for (int c = 0; c < CT; c += 4) {
+        const float4 u = *reinterpret_cast<const float4 *>(Ws + (t * CO + co) * CI + cg * CT + c);
+        wv[c] = u.x;
+        wv[c + 1] = u.y;
+        wv[c + 2] = u.z;
+        wv[c + 3] = u.w;
+      }
+#pragma unroll
+      for (int i = 0; i < PT; i++)
+        if (v[i])
+#pragma unroll
+          for (int c = 0; c < CT; c++) acc[i][c] = fmaf(wv[c], z[i][co], acc[i][c]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < PT; i++) {
+    const int64_t bp = first + i * PG;
+    if (bp >= total) continue;
+    float4 *o = reinterpret_cast<float4 *>(dIn + bp * CI + cg * CT);
+#pragma unroll
+    for (int c = 0; c < CT; c += 4) o[c / 4] = make_float4(acc[i][c], acc[i][c + 1], acc[i][c + 2], acc[i][c + 3]);
+  }
+}
+
 // ------------------------------------------- tensor-core convolution (tcgen05)
 // The 32 -> 32 channel layers as an implicit GEMM on the tensor cores:
 // for a tile of 128 consecutive lattice points of one sample,
@@ -685,6 +858,23 @@ int net_forward_t(igapgpu_net *n, int B)
       if (r) return r;
       continue;
     }
+    if constexpr (sizeof(T) == 2) {
+      const __nv_bfloat16 *x = (const __nv_bfloat16 *)n->act[l], *w = (const __nv_bfloat16 *)n->Wt + n->woff[l];
+      __nv_bfloat16 *y = (__nv_bfloat16 *)n->act[l + 1];
+      const int64_t pts = (int64_t)B * L.P;
+      if (kCin[l] == 9 && kCout[l] == 32) {
+        conv_fwd_tile<9, 32, 4, 8><<<(unsigned)((pts + 255) / 256), CS_THREADS, 0, n->stream>>>(x, w, n->bias + n->boff[l], y,
+                                                                                              L, B, l < NL - 1);
+        count_launch();
+        continue;
+      }
+      if (kCin[l] == 32 && kCout[l] == 3) {
+        conv_fwd_tile<32, 3, 2, 4><<<(unsigned)((pts + 511) / 512), CS_THREADS, 0, n->stream>>>(x, w, n->bias + n->boff[l], y,
+                                                                                              L, B, l < NL - 1);
+        count_launch();
+        continue;
+      }
+    }
     const int64_t tot = (int64_t)B * L.P * kCout[l];
     conv_fwd<T><<<(unsigned)((tot + 255) / 256), 256, 0, n->stream>>>(
         (const T *)n->act[l], kCin[l], (const T *)n->Wt + n->woff[l], n->bias + n->boff[l], (T *)n->act[l + 1],
@@ -732,6 +922,10 @@ int net_backward_t(igapgpu_net *n, int B)
       if (tcd) {
         const int r = launch_conv_tc<1>(n, n->dZh, (const __nv_bfloat16 *)n->Wt + n->woff[l], nullptr, dnext, B, 0);
         if (r) return r;
+      } else if (sizeof(T) == 2 && kCout[l] == 3 && kCin[l] == 32) {
+        conv_bwd_data_out<2, 16><<<(unsigned)(((int64_t)B * L.P + 255) / 256), CS_THREADS, 0, n->stream>>>(
+            dcur, (const __nv_bfloat16 *)n->Wt + n->woff[l], dnext, L, B);
+        count_launch();
       } else {
         conv_bwd_data<T><<<(unsigned)((nin + 255) / 256), 256, 0, n->stream>>>(dcur, kCout[l], (const T *)n->Wt + n->woff[l],
                                                                                dnext, kCin[l], L, B);
