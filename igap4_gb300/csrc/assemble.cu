@@ -480,45 +480,57 @@ int launch_geometry_cache(Context *c)
 }
 
 // ----------------------------------------------------------- Neumann
-// One thread per face control point of one face; both orders and all dofs.
-__global__ void neumann_kernel(int face, const int *bc_type, const double *neumann,
-                               const double *tabn0, const double *tabn1, const double *wq, int nq,
-                               int ne_a, int ne_b, int nb_a, int nb_b, int64_t st_a, int64_t st_b,
-                               int64_t st_n, int lay0, int lay1, double nfac0, double nfac1,
-                               double *F)
+// Traction load of every DOF: the faces in order, both orders, as the face
+// loop adds them (src/assmcore_iga.c:333-401).  The traction is constant on a
+// face, so the face integral of N_a N_b is the product of two 1-D integrals
+// (four points of at most three elements each); one thread per DOF, the tables
+// by value.  A launch per face with the 144-point double sum took 228 us each
+// at 32x8x8 whatever the traction.
+struct NeumannTable {
+  int bc_type[6 * NFACE];
+  double traction[6 * NFACE];
+  double nfac[NFACE][2];
+  const double *tabn[3];  // plain Cox-de Boor
+  int ne[3], nb[3];
+};
+
+// int N_i over the direction's elements
+__device__ __forceinline__ double basis_integral(const double *tab, const double *wq, int nq, int ne, int i)
 {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nb_a * nb_b) return;
-  const int ia = t / nb_b, ib = t % nb_b;
-  for (int order = 0; order < 2; order++)
-    for (int d = 0; d < 3; d++) {
-      const int key = 6 * face + 3 * order + d;
-      if (bc_type[key] != 1) continue;
-      const double tr = neumann[key];
-      double v0 = 0.0, v1 = 0.0;
-      for (int ea = max(0, ia - P); ea <= min(ne_a - 1, ia); ea++)
-        for (int eb = max(0, ib - P); eb <= min(ne_b - 1, ib); eb++) {
-          double s0 = 0.0, s1 = 0.0;
-          for (int qa = 0; qa < nq; qa++)
-            for (int qb = 0; qb < nq; qb++) {
-              const double *ta = tabn0 + ((size_t)ea * nq + qa) * TAB;
-              const double *tb = tabn1 + ((size_t)eb * nq + qb) * TAB;
-              const double Nab = ta[ia - ea] * tb[ib - eb];
-              const double wt = wq[qa] * wq[qb] * ta[3 * P1 + 1] * tb[3 * P1 + 1];
-              if (order == 0) {
-                s0 -= wt * Nab * tr;
-              } else {
-                s0 -= wt * (Nab * nfac0) * tr;
-                s1 -= wt * (Nab * nfac1) * tr;
-              }
-            }
-          v0 += s0;
-          v1 += s1;
-        }
-      const int64_t base = st_a * ia + st_b * ib;
-      F[3 * (base + st_n * lay0) + d] += v0;
-      if (order == 1) F[3 * (base + st_n * lay1) + d] += v1;
+  double v = 0.0;
+  for (int e = max(0, i - P); e <= min(ne - 1, i); e++) {
+    double s = 0.0;
+    for (int q = 0; q < nq; q++) {
+      const double *t = tab + ((size_t)e * nq + q) * TAB;
+      s = fma(__ldg(wq + q) * __ldg(t + 3 * P1 + 1), __ldg(t + i - e), s);
     }
+    v += s;
+  }
+  return v;
+}
+
+__global__ void neumann_kernel(NeumannTable T, const double *wq, int nq, int64_t ndof, double *F)
+{
+  const int64_t dof = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (dof >= ndof) return;
+  const int d = (int)(dof % 3);
+  int i[3];
+  cp_coords(dof / 3, T.nb, i[0], i[1], i[2]);
+  double f = 0.0;
+  for (int face = 0; face < NFACE; face++) {
+    const int dn = face / 2, da = dn == 0 ? 1 : 0, db = dn == 2 ? 1 : 2;
+    const int layer = face % 2 == 0 ? i[dn] : T.nb[dn] - 1 - i[dn];
+    if (layer > 1) continue;
+    for (int order = 0; order < 2; order++) {
+      const int key = 6 * face + 3 * order + d;
+      const double tr = T.traction[key];
+      if (T.bc_type[key] != 1 || tr == 0.0 || (order == 0 && layer == 1)) continue;
+      const double ab = basis_integral(T.tabn[da], wq, nq, T.ne[da], i[da]) *
+                        basis_integral(T.tabn[db], wq, nq, T.ne[db], i[db]);
+      f -= (order == 0 ? ab : ab * T.nfac[face][layer]) * tr;
+    }
+  }
+  F[dof] = f;
 }
 
 // ---------------------------------------------------------- Dirichlet
@@ -531,19 +543,21 @@ __global__ void dirichlet_residual_kernel(const int64_t *rows, const double *g, 
   RR[r] = U[r] - g[t];
 }
 
-// MatZeroRowsColumns(diag = 1): row r and column r of every Dirichlet DOF.
+// MatZeroRowsColumns(diag = 1): row r and column r of every Dirichlet DOF.  A
+// warp per row (up to 375 entries; a thread per row took 138 us for the 216
+// rows of the 16x4x4 beam).
 __global__ void dirichlet_matrix_kernel(const int64_t *rows, int64_t n, const int64_t *rowptr,
                                         const int32_t *cols, int nb0, int nb1, int nb2,
                                         double *vals)
 {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= n) return;
   const int nb[3] = {nb0, nb1, nb2};
   const int64_t r = rows[t];
   int ix, iy, iz;
   cp_coords(r / 3, nb, ix, iy, iz);
   const int dr = (int)(r % 3);
-  for (int64_t s = rowptr[r]; s < rowptr[r + 1]; s++) {
+  for (int64_t s = rowptr[r] + (threadIdx.x & 31); s < rowptr[r + 1]; s += 32) {
     const int32_t c = cols[s];
     vals[s] = (c == r) ? 1.0 : 0.0;
     if (c == r) continue;
@@ -560,7 +574,7 @@ __global__ void dirichlet_matrix_batch_kernel(const int64_t *rows, const int *in
                                               const int64_t *rowptr, const int32_t *cols, const int *nbs,
                                               const int64_t *dof_off, double *vals)
 {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= n) return;
   const int i = inst[t];
   const int nb[3] = {nbs[3 * i], nbs[3 * i + 1], nbs[3 * i + 2]};
@@ -569,7 +583,7 @@ __global__ void dirichlet_matrix_batch_kernel(const int64_t *rows, const int *in
   int ix, iy, iz;
   cp_coords(rl / 3, nb, ix, iy, iz);
   const int dr = (int)(rl % 3);
-  for (int64_t s = rowptr[r]; s < rowptr[r + 1]; s++) {
+  for (int64_t s = rowptr[r] + (threadIdx.x & 31); s < rowptr[r + 1]; s += 32) {
     const int32_t c = cols[s];
     vals[s] = (c == r) ? 1.0 : 0.0;
     if (c == r) continue;
@@ -584,7 +598,7 @@ int launch_dirichlet_matrix_batch(Context *c, const int *d_inst, const int *d_nb
                                   double *vals)
 {
   if (c->n_dir == 0) return IGAPGPU_OK;
-  dirichlet_matrix_batch_kernel<<<(unsigned)((c->n_dir + 127) / 128), 128, 0, c->stream>>>(
+  dirichlet_matrix_batch_kernel<<<(unsigned)((c->n_dir + 3) / 4), 128, 0, c->stream>>>(
       c->d_dir_rows, d_inst, c->n_dir, c->d_rowptr, c->d_cols, d_nbs, d_off, vals);
   count_launch();
   IGAP_CHECK_LAUNCH();
@@ -1132,33 +1146,21 @@ int launch_pattern_cols(Context *c)
 
 int launch_neumann(Context *c, const double nfac[NFACE][2])
 {
-  if (!c->d_bct) {
-    IGAP_CUDA(cudaMalloc(&c->d_bct, 36 * sizeof(int)));
-    IGAP_CUDA(cudaMalloc(&c->d_neu, 36 * sizeof(double)));
+  NeumannTable T;
+  for (int k = 0; k < 6 * NFACE; k++) {
+    T.bc_type[k] = c->bc.bc_type[k];
+    T.traction[k] = c->bc.neumann[k];
   }
-  int *d_bct = c->d_bct;
-  double *d_neu = c->d_neu;
-  IGAP_CUDA(cudaMemcpyAsync(d_bct, c->bc.bc_type, 36 * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  IGAP_CUDA(cudaMemcpyAsync(d_neu, c->bc.neumann, 36 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  IGAP_CUDA(cudaMemsetAsync(c->d_Fneu, 0, sizeof(double) * c->ndof, c->stream));
-  const int64_t sx = (int64_t)c->nbasis[1] * c->nbasis[2], sy = c->nbasis[2], sz = 1;
-  for (int face = 0; face < NFACE; face++) {
-    int da, db, dn;
-    int64_t sa, sb, sn;
-    if (face / 2 == 0) { da = 1; db = 2; dn = 0; sa = sy; sb = sz; sn = sx; }
-    else if (face / 2 == 1) { da = 0; db = 2; dn = 1; sa = sx; sb = sz; sn = sy; }
-    else { da = 0; db = 1; dn = 2; sa = sx; sb = sy; sn = sz; }
-    const int lay0 = (face % 2 == 0) ? 0 : c->nbasis[dn] - 1;
-    const int lay1 = (face % 2 == 0) ? 1 : c->nbasis[dn] - 2;
-    const int n = c->nbasis[da] * c->nbasis[db];
-    neumann_kernel<<<(n + 127) / 128, 128, 0, c->stream>>>(
-        face, d_bct, d_neu, c->d_tabn[da], c->d_tabn[db], c->d_wq, c->nquad, c->nelem[da],
-        c->nelem[db], c->nbasis[da], c->nbasis[db], sa, sb, sn, lay0, lay1, nfac[face][0],
-        nfac[face][1], c->d_Fneu);
-    count_launch();
-    IGAP_CHECK_LAUNCH();
+  for (int f = 0; f < NFACE; f++)
+    for (int l = 0; l < 2; l++) T.nfac[f][l] = nfac[f][l];
+  for (int d = 0; d < 3; d++) {
+    T.tabn[d] = c->d_tabn[d];
+    T.ne[d] = c->nelem[d];
+    T.nb[d] = c->nbasis[d];
   }
-  IGAP_CUDA(cudaStreamSynchronize(c->stream));
+  neumann_kernel<<<(unsigned)((c->ndof + 127) / 128), 128, 0, c->stream>>>(T, c->d_wq, c->nquad, c->ndof, c->d_Fneu);
+  count_launch();
+  IGAP_CHECK_LAUNCH();
   return IGAPGPU_OK;
 }
 
@@ -1192,7 +1194,7 @@ int launch_dirichlet_matrix(Context *c, double *vals)
 {
   if (c->porder == 3) return launch_dirichlet_matrix_p3(c, vals);
   if (c->n_dir == 0) return IGAPGPU_OK;
-  dirichlet_matrix_kernel<<<(unsigned)((c->n_dir + 127) / 128), 128, 0, c->stream>>>(
+  dirichlet_matrix_kernel<<<(unsigned)((c->n_dir + 3) / 4), 128, 0, c->stream>>>(
       c->d_dir_rows, c->n_dir, c->d_rowptr, c->d_cols, c->nbasis[0], c->nbasis[1], c->nbasis[2],
       vals);
   count_launch();
