@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "element.cuh"
 #include "gather.cuh"
+#include "gram_common.cuh"
 
 namespace igap {
 
@@ -66,38 +67,47 @@ __device__ __forceinline__ Patch patch_of(const DevMesh &m, int64_t cpl)
   return p;
 }
 
-// Per column control point j of the row, the (element, function) pairs that
-// contribute, in colour order: tab[27 j + rank] = entry(b, c), ebase[b] the
-// buffer offset of the patch's element in which the row's control point is
-// function b (-1 outside the lattice).
+// Shared tables of one row of control points.  Per column control point j, the
+// (element, function) pairs that contribute, in colour order: tab[27 j + rank],
+// the row control point's function number b in bits 16.. (it names the element
+// of the patch, whose buffer offset is ebase[b]), the entry's offset below.
+struct GatherTab {
+  int tab[TG_NJ * 27];
+  int64_t ebase[27];             // -1: outside the lattice
+  unsigned char cnt[TG_NJ];      // contributions of a column
+  // per direction and (a, c): rank among the shared elements, column offset,
+  // number of shared elements
+  unsigned char rank[3][9], off[3][9], n[3][9];
+};
+
 template <typename F>
-__device__ __forceinline__ void gather_table(const Patch &p, int64_t e0, int64_t per_element, int *tab, int64_t *ebase,
-                                             F entry)
+__device__ __forceinline__ void gather_table(GatherTab &G, const Patch &p, int64_t e0, int64_t per_element, F entry)
 {
   if (threadIdx.x < 27) {
-    const int ex = p.ix - threadIdx.x / 9, ey = p.iy - (threadIdx.x / 3) % 3, ez = p.iz - threadIdx.x % 3;
+    const int t = threadIdx.x;
+    const int ex = p.ix - t / 9, ey = p.iy - (t / 3) % 3, ez = p.iz - t % 3;
     const bool in = ex >= 0 && ex < p.ne0 && ey >= 0 && ey < p.ne1 && ez >= 0 && ez < p.ne2;
-    ebase[threadIdx.x] = in ? (e0 + ((int64_t)ex * p.ne1 + ey) * p.ne2 + ez) * per_element : -1;
+    G.ebase[t] = in ? (e0 + ((int64_t)ex * p.ne1 + ey) * p.ne2 + ez) * per_element : -1;
+    // direction t / 9, element i - a, column function c
+    const int dir = t / 9, a = (t / 3) % 3, c = t % 3;
+    const int i = dir == 0 ? p.ix : dir == 1 ? p.iy : p.iz, lo = dir == 0 ? p.lox : dir == 1 ? p.loy : p.loz;
+    const int ne = dir == 0 ? p.ne0 : dir == 1 ? p.ne1 : p.ne2;
+    const Range r = shared_elements(i, i - a + c, ne);
+    G.rank[dir][3 * a + c] = (unsigned char)by_residue(r, i - a);
+    G.n[dir][3 * a + c] = (unsigned char)max(r.n, 0);
+    G.off[dir][3 * a + c] = (unsigned char)(i - a + c - lo);
   }
   __syncthreads();
   for (int t = threadIdx.x; t < 27 * NB; t += TG_THREADS) {
     const int b = t / NB, c = t % NB;
-    if (ebase[b] < 0) continue;
-    const int ex = p.ix - b / 9, ey = p.iy - (b / 3) % 3, ez = p.iz - b % 3;
-    const int jx = ex + c / 9, jy = ey + (c / 3) % 3, jz = ez + c % 3;
-    const Range rx = shared_elements(p.ix, jx, p.ne0), ry = shared_elements(p.iy, jy, p.ne1),
-                rz = shared_elements(p.iz, jz, p.ne2);
-    const int rank = (by_residue(rx, ex) * ry.n + by_residue(ry, ey)) * rz.n + by_residue(rz, ez);
-    const int j = ((jx - p.lox) * p.cy + (jy - p.loy)) * p.cz + (jz - p.loz);
-    tab[j * 27 + rank] = entry(b, c);
+    if (G.ebase[b] < 0) continue;
+    const int x = b / 9 * 3 + c / 9, y = (b / 3) % 3 * 3 + (c / 3) % 3, z = b % 3 * 3 + c % 3;
+    const int ny = G.n[1][y], nz = G.n[2][z];
+    const int j = (G.off[0][x] * p.cy + G.off[1][y]) * p.cz + G.off[2][z];
+    G.tab[j * 27 + (G.rank[0][x] * ny + G.rank[1][y]) * nz + G.rank[2][z]] = b << 16 | entry(b, c);
+    G.cnt[j] = (unsigned char)(G.n[0][x] * ny * nz);  // the same value from every pair of the column
   }
   __syncthreads();
-}
-
-__device__ __forceinline__ int contributions(const Patch &p, int j)
-{
-  const int jz = p.loz + j % p.cz, jy = p.loy + (j / p.cz) % p.cy, jx = p.lox + j / (p.cz * p.cy);
-  return shared_elements(p.ix, jx, p.ne0).n * shared_elements(p.iy, jy, p.ne1).n * shared_elements(p.iz, jz, p.ne2).n;
 }
 }  // namespace
 
@@ -106,27 +116,25 @@ __device__ __forceinline__ int contributions(const Patch &p, int j)
 __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a, const double *__restrict__ ebuf,
                                                                     double *__restrict__ vals)
 {
-  __shared__ int tab[TG_NJ * 27];  // (function b * 378 + pair) * 2 + transposed
-  __shared__ int64_t ebase[27];
+  __shared__ GatherTab G;
   const int64_t cp = blockIdx.x;
   const int inst = a.cpinst ? __ldg(a.cpinst + cp) : 0;
   const DevMesh &m = a.meshes ? a.meshes[inst] : a.m;
   const Patch p = patch_of(m, cp - m.dof_off / 3);
-  gather_table(p, a.eoff ? __ldg(a.eoff + inst) : 0, EBUF, tab, ebase, [](int b, int c) {
-    return (b * NPAIRS + pair_index(min(b, c), max(b, c))) * 2 + (b > c ? 1 : 0);
+  gather_table(G, p, a.eoff ? __ldg(a.eoff + inst) : 0, EBUF, [](int b, int c) {  // block offset, bit 15: transposed
+    return 9 * pair_index(min(b, c), max(b, c)) | (b > c ? 0x8000 : 0);
   });
   const int64_t r0 = __ldg(a.rowptr + 3 * cp);
   const bool failed = a.err && *a.err;
   for (int t = threadIdx.x; t < 9 * p.nj; t += TG_THREADS) {
-    const int j = t / 9, q = t % 9, d = q / 3, e = q % 3;
-    const int n = contributions(p, j);
-    const int qt = 3 * e + d;
+    const int j = t / 9, q = t - 9 * j, d = q / 3, e = q - 3 * d;
+    const int n = G.cnt[j], qt = 3 * e + d;
+    const int *tab = G.tab + j * 27;
     double s = 0.0;
-#pragma unroll 3
+#pragma unroll 4
     for (int k = 0; k < n; k++) {
-      const int v = tab[j * 27 + k];
-      const int bp = v >> 1, b = bp / NPAIRS;
-      s += __ldg(ebuf + ebase[b] + (int64_t)(bp - b * NPAIRS) * 9 + ((v & 1) ? qt : q));
+      const int v = tab[k];
+      s += __ldg(ebuf + G.ebase[v >> 16] + (v & 0x7fff) + ((v & 0x8000) ? qt : q));
     }
     vals[r0 + (int64_t)d * 3 * p.nj + 3 * j + e] = failed ? __longlong_as_double(0x7ff8000000000000ll) : s;
   }
@@ -138,21 +146,21 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a,
 __global__ void __launch_bounds__(TG_THREADS) tangent_gather_f32_kernel(GatherMap a, const float *__restrict__ fbuf,
                                                                         double *__restrict__ vals)
 {
-  __shared__ int tab[TG_NJ * 27];  // 27 b + c
-  __shared__ int64_t ebase[27];
+  __shared__ GatherTab G;
   const int64_t cp = blockIdx.x;
   const Patch p = patch_of(a.m, cp);
-  gather_table(p, 0, NB * 243, tab, ebase, [](int b, int c) { return NB * b + c; });
+  gather_table(G, p, 0, NB * 243, [](int b, int c) { return 243 * b + 3 * c; });
   const int64_t r0 = __ldg(a.rowptr + 3 * cp);
   const int row = 3 * p.nj;
   for (int t = threadIdx.x; t < 3 * row; t += TG_THREADS) {
     const int d = t / row, x = t - d * row, j = x / 3, e = x - 3 * j;
-    const int n = contributions(p, j);
+    const int n = G.cnt[j];
+    const int *tab = G.tab + j * 27;
     double s = 0.0;
-#pragma unroll 3
+#pragma unroll 4
     for (int k = 0; k < n; k++) {
-      const int v = tab[j * 27 + k], b = v / NB;
-      s += (double)__ldg(fbuf + ebase[b] + b * 243 + d * 81 + 3 * (v - NB * b) + e);
+      const int v = tab[k];
+      s += f32_to_f64(__ldg(fbuf + G.ebase[v >> 16] + (v & 0xffff) + 81 * d + e));  // widened on the integer pipe
     }
     vals[r0 + t] = s;
   }
