@@ -1061,9 +1061,11 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
     rc = law_df ? launch_res_law_df(c, c->d_preR, RR) : launch_res_df(c, RR);
     if (rc) return rc;
   }
-  // the linear law's FP64 tangent on the tensor cores where its slices are built
+  // the linear law's FP64 tangent and residual on the tensor cores where its
+  // slices are built
   const bool x_tan = fp64_tan && ensure_exact(c);
-  const bool k_res = do_res && !df_res, k_tan = fp64_tan && !x_tan;
+  const bool x_res = do_res && !df_res && ensure_exact(c);
+  const bool k_res = do_res && !df_res && !x_res, k_tan = fp64_tan && !x_tan;
   if (k_res || k_tan) {
     const bool do_res_k = k_res, do_tan_k = k_tan;
     {
@@ -1079,7 +1081,7 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
   }
 #undef IGAP_DISPATCH
   if (rc) return rc;
-  if (x_tan && (rc = launch_exact_tangent(c, vals))) return rc;
+  if ((x_tan || x_res) && (rc = launch_exact(c, x_res ? RR : nullptr, x_tan ? vals : nullptr))) return rc;
   if (do_tan && !fp64_tan) {
     const bool gathered = !oz_tan && tc_law_applies(c, L);  // every slot is written
     if (!gathered) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));

@@ -211,9 +211,12 @@ bool batch_instances(Context *c, std::vector<Context *> *subs, std::vector<int64
   return true;
 }
 
-void batch_law_map(Context *c, const DevLaw **laws, const int **einst)
+void batch_element_map(Context *c, const DevLaw **laws, const DevMesh **meshes, const int64_t **eoff,
+                       const int **einst)
 {
   *laws = c->batch->d_law;
+  *meshes = c->batch->d_mesh;
+  *eoff = c->batch->d_eoff;
   *einst = c->batch->d_einst;
 }
 
@@ -264,14 +267,14 @@ static int batch_kernels(Context *c, bool do_res, bool do_tan, double *RR, doubl
       if (r) return r;
     }
   }
-  // the linear law's FP64 tangent of the whole queue on the tensor cores
+  // the linear law's FP64 assembly of the whole queue on the tensor cores
   bool fp64_queue = fp64_tan;
-  if (fp64_tan && nitems == b->nitems && ensure_exact(c)) {
-    fp64_queue = false;
+  if ((do_res || fp64_tan) && nitems == b->nitems && ensure_exact(c)) {
     if (which & 1) {
-      int r = launch_exact_tangent(c, vals);
+      int r = launch_exact(c, do_res ? RR : nullptr, fp64_tan ? vals : nullptr);
       if (r) return r;
     }
+    do_res = fp64_queue = false;
   }
   if ((do_res || fp64_queue) && (which & 1)) {
     int grid = 0;
@@ -318,10 +321,12 @@ static int batch_kernels(Context *c, bool do_res, bool do_tan, double *RR, doubl
 int launch_batch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *vals)
 {
   Batch *b = c->batch;
-  if (do_res)
+  // the exact kernel's gathers write every row and slot
+  const bool x_res = do_res && !batch_res_df(c) && ensure_exact(c);
+  const bool x_tan = do_tan && c->prec != IGAPGPU_PREC_SPLIT && ensure_exact(c);
+  if (do_res && !x_res)
     IGAP_CUDA(cudaMemcpyAsync(RR, c->d_Fneu, sizeof(double) * c->ndof, cudaMemcpyDeviceToDevice, c->stream));
-  const bool gathered = do_tan && c->prec != IGAPGPU_PREC_SPLIT && ensure_exact(c);  // every slot written
-  if (do_tan && !gathered) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
+  if (do_tan && !x_tan) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
   int r = batch_kernels(c, do_res, do_tan, RR, vals, b->nitems);
   if (r) return r;
   if (do_res && (r = launch_dirichlet_residual(c, RR))) return r;

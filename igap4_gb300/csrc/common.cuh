@@ -311,9 +311,9 @@ int launch_assembly_p3(Context *c, bool do_res, bool do_tan, double *RR, double 
 // tc_ozaki.cu (linear law, BF16 slices, FP64-quality)
 int ensure_ozaki_operands(Context *c);
 int launch_tc_ozaki(Context *c, double *vals);
-// tc_exact.cu (linear law, FP64 tangent from exact BF16 slices)
+// tc_exact.cu (linear law, FP64 tangent and residual from exact BF16 slices)
 bool ensure_exact(Context *c);
-int launch_exact_tangent(Context *c, double *vals);
+int launch_exact(Context *c, double *RR, double *vals);
 // res_df.cu (linear law residual in double-FP32 arithmetic)
 int ensure_res_pairs(Context *c);
 int launch_res_df(Context *c, double *RR);
@@ -353,7 +353,8 @@ int batch_set_neumann(Context *c, const double *table);
 int batch_prepare_split(Context *c);
 // instances and their first elements; false without memory for the element tables
 bool batch_instances(Context *c, std::vector<Context *> *subs, std::vector<int64_t> *off);
-void batch_law_map(Context *c, const DevLaw **laws, const int **einst);
+void batch_element_map(Context *c, const DevLaw **laws, const DevMesh **meshes, const int64_t **eoff,
+                       const int **einst);
 // element kernels over a batch work queue (assemble.cu, tc_tangent.cu)
 int launch_element_batch(Context *c, const BatchArgs &a, int law, bool do_res, bool do_tan, int grid,
                          const double *Uhist, double *RR, double *vals);

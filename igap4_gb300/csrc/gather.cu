@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) residual_gather_kernel(GatherMap a, const
     }
     if (in) s += __ldg(rbuf + (e0 + el) * NE + 3 * b + d);
   }
-  RR[dof] = s;
+  RR[dof] = a.err && *a.err ? __longlong_as_double(0x7ff8000000000000ll) : s;
 }
 
 static GatherMap gather_map(Context *c)
@@ -232,9 +232,11 @@ int launch_tangent_gather_f32(Context *c, double *vals)
   return IGAPGPU_OK;
 }
 
-int launch_residual_gather(Context *c, double *RR)
+int launch_residual_gather(Context *c, double *RR, const int *err)
 {
-  residual_gather_kernel<<<(unsigned)((c->ndof + 255) / 256), 256, 0, c->stream>>>(gather_map(c), c->d_rbuf, c->d_Fneu,
+  GatherMap a = gather_map(c);
+  a.err = err;
+  residual_gather_kernel<<<(unsigned)((c->ndof + 255) / 256), 256, 0, c->stream>>>(a, c->d_rbuf, c->d_Fneu,
                                                                                   RR);
   count_launch();
   IGAP_CHECK_LAUNCH();

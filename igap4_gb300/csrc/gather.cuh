@@ -27,7 +27,7 @@ bool ensure_fbuf(Context *c);  // FP32 [element][27][243]
 bool ensure_rbuf(Context *c);
 int launch_tangent_gather(Context *c, double *vals, const int *err = nullptr);
 int launch_tangent_gather_f32(Context *c, double *vals);
-int launch_residual_gather(Context *c, double *RR);
+int launch_residual_gather(Context *c, double *RR, const int *err = nullptr);
 void batch_gather_map(Context *c, GatherMap *a);
 
 }  // namespace igap

@@ -520,7 +520,7 @@ int assembly_graph(Context *c, bool do_res, bool do_tan)
   IGAP_CUDA(cudaGraphLaunch(c->asm_graph[key], c->stream));
   count_launch((int)c->asm_graph_nodes[key]);
   if (do_tan) c->matrix_valid = true;
-  if (do_tan && c->exact_state == 1) c->exact_ran = true;
+  if (c->exact_state == 1) c->exact_ran = true;
   if (waits) {
     int herr = 0;
     IGAP_CUDA(cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));

@@ -49,7 +49,7 @@ namespace igap {
 namespace {
 constexpr int CY_THREADS = 1024, CY_WARPS = CY_THREADS / 32;
 constexpr int CY_VB = 4;             // basis vectors per item of the projection
-constexpr int CY_RMAX = 1024;        // row chunks per group of vectors
+constexpr int CY_RMAX = 256;         // row chunks per group of vectors
 constexpr int CY_MAX_RESTART = 200;  // T (m (m - 1) / 2 doubles) in shared memory
 constexpr uint32_t CY_WAIT_LIMIT = 1u << 24;
 
@@ -90,24 +90,26 @@ struct CycleSmem {
   // packed rows of T (row i: entries c < i at i (i - 1) / 2) follow
 };
 
-// All blocks arrive and wait.  Release/acquire at GPU scope by thread 0, the
-// block barriers around it order the other threads.
+// All blocks arrive and wait.  Fences at GPU scope by thread 0 (one before the
+// arrival, one after the relaxed polls), the block barriers around them order
+// the other threads.
 __device__ __forceinline__ bool grid_sync(const CycleArgs &a, CycleSmem &S, unsigned &target)
 {
   __syncthreads();
   target += gridDim.x;
   if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+    asm volatile("fence.acq_rel.gpu;\n\tred.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
     int ok = 0;
     for (uint32_t it = 0; it < CY_WAIT_LIMIT; it++) {
       unsigned v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
       if ((int)(v - target) >= 0) {
         ok = 1;
         break;
       }
       if ((it & 1023u) == 1023u && *(volatile int *)a.err) break;
     }
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
     if (!ok) atomicExch(a.err, 4);
     S.ok = ok;
   }
@@ -219,6 +221,32 @@ __device__ __forceinline__ double multiply_any(const CycleArgs &a, const double 
   return a.n / 3 < (int64_t)gridDim.x * CY_WARPS * 2 ? multiply<32, RES>(a, x, w) : multiply<16, RES>(a, x, w);
 }
 
+// Folds NS sums (4 or 8) over the lanes of a warp: each exchange halves the
+// number of sums a lane carries (NS - 1 additions, then one per remaining
+// step).  s[0] becomes sum number `id` in every lane; the lanes with
+// (lane & (32 / NS - 1)) == 0 name each once.
+template <int NS>
+__device__ __forceinline__ int fold(double (&s)[2 * CY_VB], int lane)
+{
+  int id = 0;
+#pragma unroll
+  for (int o = 16, cnt = NS; o > 0; o >>= 1) {
+    if (cnt > 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int q = 0; q < cnt / 2; q++) {
+        const double keep = up ? s[q + cnt / 2] : s[q], give = up ? s[q] : s[q + cnt / 2];
+        s[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+      if (up) id += cnt / 2;
+      cnt /= 2;
+    } else {
+      s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+    }
+  }
+  return id;
+}
+
 // Partial dot products of the basis vectors 0..j with w (and, with LROW, with
 // v_j): item (group of CY_VB vectors, row chunk) per warp.
 template <bool LROW>
@@ -248,25 +276,8 @@ __device__ __forceinline__ void project_partial(const CycleArgs &a, int j, int R
         if (LROW) s[CY_VB + q] = fma(u, vk, s[CY_VB + q]);
       }
     }
-    // fold the sums over the lanes: each exchange halves the number of sums a
-    // lane carries
-    int id = 0;
     constexpr int NS = LROW ? 8 : 4;
-#pragma unroll
-    for (int o = 16, cnt = NS; o > 0; o >>= 1) {
-      if (cnt > 1) {
-        const bool up = lane & o;
-#pragma unroll
-        for (int q = 0; q < cnt / 2; q++) {
-          const double keep = up ? s[q + cnt / 2] : s[q], give = up ? s[q] : s[q + cnt / 2];
-          s[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-        }
-        if (up) id += cnt / 2;
-        cnt /= 2;
-      } else {
-        s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
-      }
-    }
+    const int id = fold<NS>(s, lane);
     const int q = id % CY_VB, kind = id / CY_VB;
     if ((lane & (32 / NS - 1)) == 0 && i0 + q <= j)
       a.part[((size_t)kind * (a.m + 1) + i0 + q) * CY_RMAX + r] = s[0];
@@ -278,23 +289,19 @@ template <bool LROW>
 __device__ __forceinline__ void project_total(const CycleArgs &a, CycleSmem &S, int j, int R)
 {
   const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x >> 5; i <= j; i += CY_WARPS) {
-    const double *p = a.part + (size_t)i * CY_RMAX, *pl = p + (size_t)(a.m + 1) * CY_RMAX;
-    double s = 0.0, t = 0.0;
-    for (int r = lane; r < R; r += 32) {
-      s += __ldcg(p + r);
-      if (LROW) t += __ldcg(pl + r);
-    }
-    if (LROW) {  // the halves of the warp carry one sum each
-      const bool up = lane & 16;
-      s = (up ? t : s) + __shfl_xor_sync(0xffffffffu, up ? s : t, 16);
-    } else {
-      s += __shfl_xor_sync(0xffffffffu, s, 16);
-    }
+  constexpr int NS = LROW ? 8 : 4;
+  for (int g = threadIdx.x >> 5; g * CY_VB <= j; g += CY_WARPS) {
+    double s[2 * CY_VB];
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) S.r[i] = s;
-    if (LROW && lane == 16) S.l[i] = s;
+    for (int q = 0; q < 2 * CY_VB; q++) s[q] = 0.0;
+#pragma unroll
+    for (int q = 0; q < NS; q++) {
+      const int i = min(g * CY_VB + q % CY_VB, j);
+      const double *p = a.part + ((size_t)(q / CY_VB) * (a.m + 1) + i) * CY_RMAX;
+      for (int r = lane; r < R; r += 32) s[q] += __ldcg(p + r);
+    }
+    const int id = fold<NS>(s, lane), i = g * CY_VB + id % CY_VB;
+    if ((lane & (32 / NS - 1)) == 0 && i <= j) (id < CY_VB ? S.r : S.l)[i] = s[0];
   }
   __syncthreads();
 }
@@ -510,7 +517,7 @@ __global__ void __launch_bounds__(CY_THREADS, 1) gmres_cycle_kernel(CycleArgs a)
     // orthogonalise
     const int ngroup = (j + CY_VB) / CY_VB;
     int R = (int)(gridDim.x * CY_WARPS) / ngroup;
-    const int64_t rmax = (a.n + 127) / 128;
+    const int64_t rmax = (a.n + 159) / 160;
     R = R < CY_RMAX ? R : CY_RMAX;
     R = R < rmax ? R : (int)rmax;
     R = R > 0 ? R : 1;

@@ -152,20 +152,6 @@ __host__ __device__ inline int64_t cell_count(const CellGeom &g)
   return (int64_t)g.nc[0] * g.nc[1] * g.nc[2];
 }
 
-// Control points of cell `cell` (x-major, z fastest) and their count.
-__device__ __forceinline__ int cell_points(const CellGeom &g, int64_t cell, int64_t cps[8])
-{
-  const int gz = (int)(cell % g.nc[2]);
-  const int64_t t = cell / g.nc[2];
-  const int gy = (int)(t % g.nc[1]), gx = (int)(t / g.nc[1]);
-  int n = 0;
-  for (int jx = 2 * gx; jx < 2 * gx + 2 && jx < g.nb[0]; jx++)
-    for (int jy = 2 * gy; jy < 2 * gy + 2 && jy < g.nb[1]; jy++)
-      for (int jz = 2 * gz; jz < 2 * gz + 2 && jz < g.nb[2]; jz++)
-        cps[n++] = ((int64_t)jx * g.nb[1] + jy) * g.nb[2] + jz;
-  return n;
-}
-
 constexpr int CB_WARPS = 4;  // cells per block of the inversion
 
 static __global__ void __launch_bounds__(32 * CB_WARPS) cblock_invert_kernel(const int64_t *__restrict__ rowptr,
@@ -178,19 +164,20 @@ static __global__ void __launch_bounds__(32 * CB_WARPS) cblock_invert_kernel(con
   const int64_t cell = (int64_t)blockIdx.x * CB_WARPS + warp;
   if (cell >= ncell) return;  // whole warp
   double(*A)[2 * CBS + 1] = Aug[warp];
-  int64_t cps[8];
-  const int np = cell_points(g, cell, cps);
-  const int bs = 3 * np;
+  // first control point and extents of the cell (clipped at the far faces)
+  const int z0 = 2 * (int)(cell % g.nc[2]), y0 = 2 * (int)(cell / g.nc[2] % g.nc[1]),
+            x0 = 2 * (int)(cell / ((int64_t)g.nc[1] * g.nc[2]));
+  const int nz = min(2, g.nb[2] - z0), ny = min(2, g.nb[1] - y0), nyz = ny * nz;
+  const int bs = 3 * min(2, g.nb[0] - x0) * nyz;
+#pragma unroll 4
   for (int t = lane; t < CBS * 2 * CBS; t += 32) {
     const int a = t / (2 * CBS), b = t % (2 * CBS);
     double v = 0.0;
     if (a < bs && b < bs) {
       const int p = a / 3, d = a % 3, q = b / 3, e = b % 3;
-      int ix, iy, iz, jx, jy, jz;
-      cp_coords(cps[p], g.nb, ix, iy, iz);
-      cp_coords(cps[q], g.nb, jx, jy, jz);
-      const int64_t r = 3 * cps[p] + d;
-      v = vals[rowptr[r] + 3 * stencil_pos(ix, iy, iz, jx, jy, jz, g.nb) + e];
+      const int ix = x0 + p / nyz, iy = y0 + p / nz % ny, iz = z0 + p % nz;
+      const int64_t r = 3 * (((int64_t)ix * g.nb[1] + iy) * g.nb[2] + iz) + d;
+      v = vals[rowptr[r] + 3 * stencil_pos(ix, iy, iz, x0 + q / nyz, y0 + q / nz % ny, z0 + q % nz, g.nb) + e];
     } else if (b >= CBS) {
       v = (b - CBS == a) ? 1.0 : 0.0;
     }
@@ -244,34 +231,37 @@ static __global__ void __launch_bounds__(32 * CB_WARPS) cblock_invert_kernel(con
         v = A[a][CBS + b];
       } else if (a == b) {  // fallback: inverse of the diagonal
         const int p = a / 3, d = a % 3;
-        int ix, iy, iz;
-        cp_coords(cps[p], g.nb, ix, iy, iz);
-        const int64_t r = 3 * cps[p] + d;
+        const int ix = x0 + p / nyz, iy = y0 + p / nz % ny, iz = z0 + p % nz;
+        const int64_t r = 3 * (((int64_t)ix * g.nb[1] + iy) * g.nb[2] + iz) + d;
         const double dg = vals[rowptr[r] + 3 * stencil_pos(ix, iy, iz, ix, iy, iz, g.nb) + d];
         v = dg != 0.0 ? 1.0 / dg : 1.0;
       }
     }
-    o[t] = v;
+    o[b * CBS + a] = v;  // column by column: the application reads a column across the lanes
   }
 }
 
 // z = B^-1 v with the inverted cell blocks: a warp per cell, lane a < bs
-// computes the cell's DOF a (grid-stride over cells).  v may have been
+// computes the cell's DOF a (grid-stride over cells); the block's columns
+// come as coalesced loads independent of each other, v through shuffles.  v may have been
 // written earlier in the same kernel (no read-only loads of v here and below).
 __device__ __forceinline__ void cblock_apply(double *z, const double *v, const double *__restrict__ inv, const CellGeom &g, int64_t ncell)
 {
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t cell = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); cell < ncell; cell += nw) {
-    int64_t cps[8];
-    const int np = cell_points(g, cell, cps);
-    const int bs = 3 * np;
-    if (lane < bs) {
-      const double *row = inv + (size_t)cell * CBS * CBS + (size_t)lane * CBS;
-      double s = 0.0;
-      for (int b = 0; b < bs; b++) s = fma(row[b], v[3 * cps[b / 3] + b % 3], s);
-      z[3 * cps[lane / 3] + lane % 3] = s;
-    }
+    const int z0 = 2 * (int)(cell % g.nc[2]), y0 = 2 * (int)(cell / g.nc[2] % g.nc[1]),
+              x0 = 2 * (int)(cell / ((int64_t)g.nc[1] * g.nc[2]));
+    const int nz = min(2, g.nb[2] - z0), ny = min(2, g.nb[1] - y0), nyz = ny * nz;
+    const int bs = 3 * min(2, g.nb[0] - x0) * nyz;
+    const int p = lane / 3;
+    const int64_t dof = 3 * (((int64_t)(x0 + p / nyz) * g.nb[1] + y0 + p / nz % ny) * g.nb[2] + z0 + p % nz) + lane % 3;
+    const double vl = lane < bs ? v[dof] : 0.0;
+    const double *col = inv + (size_t)cell * CBS * CBS + (lane < CBS ? lane : 0);
+    double s = 0.0;
+#pragma unroll 12
+    for (int b = 0; b < CBS; b++) s = fma(__ldg(col + b * CBS), __shfl_sync(0xffffffffu, vl, b), s);
+    if (lane < bs) z[dof] = s;
   }
 }
 

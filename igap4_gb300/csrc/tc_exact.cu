@@ -1,5 +1,5 @@
-// FP64 tangent of the linear isotropic strain-gradient law on the tensor
-// cores.  The tangent of the law is a function of the Gram matrix
+// FP64 tangent and residual of the linear isotropic strain-gradient law on
+// the tensor cores.  The tangent of the law is a function of the Gram matrix
 // G = S S^T of the sqrt(w)-weighted derivatives (tc_gram.cu):
 //   K[(b,d),(c,e)] = lam G[(b,d),(c,e)] + mu G[(b,e),(c,d)] + delta_de mu tr G_bc.
 // The FP64 pipe (2 FMA per clock and SM) bounds the direct sum: 0.94 M FMA,
@@ -28,6 +28,9 @@
 //  * tensor memory holds 512 columns: acc2, acc4, acc6, acc78 with N = 80 and
 //    X3, X5 with N = 96.  Column 80 of the symmetric ones is their row 80;
 //    the entry (80, 80) is a 256-term FP64 dot product of the row itself.
+// Residual: exact for constants as the quadrature loop is not (the state enters
+// as differences from the element's middle function: a translation of 5 beside
+// displacements of 1e-3 costs the quadrature loop 2e-13).
 // Measured: against 64-bit reference sums the error is the FP64 kernel's (7e-16
 // at 16x4x4, 3e-15 at 63x17x15 distorted, both from the geometry; the two
 // tangents differ by 2e-16). Residual and tangent at 16x4x4 0.74 -> 0.30 ms,
@@ -43,7 +46,10 @@
 //     G_rc = Y[r][c] + Y[c][r]; the tensor memory is free for the next element
 //     after that,
 //   warps 2-13: a thread per basis pair b <= c forms its 3 x 3 block of K in
-//     FP64; the element's blocks leave by one bulk copy.
+//     FP64; the element's blocks leave by one bulk copy, and the residual of
+//     the linear law is K_e u_e from the blocks in shared memory (6,561 FMA an
+//     element under the next element's MMAs; the quadrature loop takes 93,312
+//     on the FP64 pipe).
 // Every mbarrier wait is bounded; a CTA that gives up sets the error word
 // (the gather then writes NaN), waits (bounded) for its copies and MMAs in
 // flight and frees its tensor memory.
@@ -75,7 +81,7 @@ constexpr int XS_EXP = 88;
 constexpr uint32_t XS_TMEM_COLS = 512;
 constexpr uint32_t XS_ACC2 = 0, XS_ACC4 = 80, XS_ACC6 = 160, XS_ACC78 = 240, XS_X3 = 320, XS_X5 = 416;
 constexpr uint32_t XS_WAIT_LIMIT = 1u << 26;
-constexpr int XO_THREADS = 256;                  // operand kernel
+constexpr int XO_THREADS = 512;                  // operand kernel
 static_assert(XS_STAGE % 16 == 0 && XS_CH_BYTES % 16 == 0, "bulk copies and descriptors need 16-byte alignment");
 static_assert(EBUF * sizeof(double) % 16 == 0, "bulk stores move multiples of 16 bytes");
 
@@ -85,6 +91,7 @@ struct XsSmem {
   long long Y[XS_ROWS * XS_YP];
   unsigned char pb[NPAIRS], pc[NPAIRS];
   double g80;
+  double u[NE], rsum[4][NE];
   int ex[XS_EXP];
   uint64_t full[XS_NS], empty[XS_NS], accfull, accempty;
   uint32_t cp_n[XS_NS], mm_n[XS_NS], accf_n;
@@ -97,11 +104,17 @@ struct ExactArgs {
   const unsigned char *ops;   // [element][chunk][XS_CH_BYTES]
   const short *expo;          // [element][XS_EXP]
   const double *row80;        // [element][chunk * 32] row 80 of S
-  double *ebuf;
+  double *ebuf;               // element matrices out (or null)
+  const double *U;            // current state: element residuals K_e u_e to rbuf (or null)
+  double *rbuf;
+  DevMesh m;
   int64_t nelem;
   int nchunk;
   double lam, mu;
-  const DevLaw *laws;         // batches: law of every instance, instance of every element
+  // batches: law, mesh and first element of every instance, instance of every element
+  const DevLaw *laws;
+  const DevMesh *meshes;
+  const int64_t *eoff;
   const int *einst;
   int *err;
 };
@@ -199,14 +212,18 @@ __global__ void __launch_bounds__(XO_THREADS) exact_operand_kernel(const double 
         if (lane == 0) atomicExch(bad, 1);
         E = 0;
       }
+      // |x|^2 from the leading 24 bits, scaled on the integer pipe (|x| < 2^-100 counts as zero)
       float n2 = 0.f;
-      const double sc = __hiloint2double((1023 + 8 - E) << 20, 0);
       for (int k = lane; k < K; k += 32) {
-        const float x = (float)(S[r * ld + k] * sc);
+        const double v = S[r * ld + k];
+        const int fe = ((__double2hiint(v) >> 20) & 0x7ff) - 1023 + 8 - E + 127;
+        const float x = fe > 27 ? __uint_as_float((uint32_t)fe << 23 | ((uint32_t)__double2hiint(v) & 0xfffffu) << 3 |
+                                                  (uint32_t)__double2loint(v) >> 29)
+                                : 0.f;
         n2 = fmaf(x, x, n2);
       }
       for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
-      if (n2 > 4.18e6f) E++;  // 2048^2 less the rounding of this sum
+      if (n2 > 4.18e6f) E++;  // 2048^2 less the truncation of x and the rounding of this sum
       if (lane == 0) rexp[r] = E;
     }
     for (int r = XS_ROWS + tid; r < XS_EXP; r += XO_THREADS) rexp[r] = 0;
@@ -386,10 +403,22 @@ __global__ void __launch_bounds__(XS_THREADS, 1) exact_tangent_kernel(ExactArgs 
     for (int j = 0; j < nmine && ok; j++) {
       const int64_t e = blockIdx.x + (int64_t)j * gridDim.x;
       double lam = a.lam, mu = a.mu;
+      const int inst = a.laws ? __ldg(a.einst + e) : 0;
       if (a.laws) {
-        const DevLaw &L = a.laws[__ldg(a.einst + e)];
-        lam = __ldg(&L.par[0]);
-        mu = __ldg(&L.par[1]);
+        lam = __ldg(&a.laws[inst].par[0]);
+        mu = __ldg(&a.laws[inst].par[1]);
+      }
+      if (a.U && t >= 32 && t < 32 + NE) {  // the element's state
+        const DevMesh &m = a.laws ? a.meshes[inst] : a.m;
+        const int64_t el = a.laws ? e - __ldg(a.eoff + inst) : e;
+        const int b = (t - 32) / 3, d = (t - 32) % 3;
+        const int ez = (int)(el % m.nelem[2]), ey = (int)((el / m.nelem[2]) % m.nelem[1]),
+                  ex = (int)(el / ((int64_t)m.nelem[1] * m.nelem[2]));
+        const int64_t cp = ((int64_t)(ex + b / 9) * m.nbasis[1] + (ey + (b / 3) % 3)) * m.nbasis[2] + (ez + b % 3);
+        // less the middle function's value: constants drop out of the law, and
+        // what a rigid translation would lose by cancellation is not formed
+        const int64_t mid = ((int64_t)(ex + 1) * m.nbasis[1] + (ey + 1)) * m.nbasis[2] + (ez + 1);
+        S.u[t - 32] = __ldg(a.U + m.dof_off + 3 * cp + d) - __ldg(a.U + m.dof_off + 3 * mid + d);
       }
       if (t < 32) {  // entry (80, 80)
         const double *row = a.row80 + (size_t)e * nchunk * 32;
@@ -480,7 +509,23 @@ __global__ void __launch_bounds__(XS_THREADS, 1) exact_tangent_kernel(ExactArgs 
       }
       tc::fence_proxy_async();
       asm volatile("bar.sync 1, 384;" ::: "memory");
-      if (t == 0) tc::bulk_s2g(a.ebuf + e * EBUF, S.Kb, (uint32_t)(EBUF * sizeof(double)));
+      if (t == 0 && a.ebuf) tc::bulk_s2g(a.ebuf + e * EBUF, S.Kb, (uint32_t)(EBUF * sizeof(double)));
+      if (a.U) {  // row r of K_e u_e, the 27 functions in four parts
+        if (t < 4 * NE) {
+          const int r = t % NE, part = t / NE, b = r / 3, d = r - 3 * b;
+          double s = 0.0;
+          for (int c = 7 * part; c < min(7 * part + 7, NB); c++) {
+            const bool up = b <= c;
+            const double *k = S.Kb + 9 * (up ? pair_index(b, c) : pair_index(c, b)) + (up ? 3 * d : d);
+            const int st = up ? 1 : 3;
+#pragma unroll
+            for (int q = 0; q < 3; q++) s = fma(k[st * q], S.u[3 * c + q], s);
+          }
+          S.rsum[part][r] = s;
+        }
+        asm volatile("bar.sync 1, 384;" ::: "memory");
+        if (t < NE) a.rbuf[e * NE + t] = (S.rsum[0][t] + S.rsum[1][t]) + (S.rsum[2][t] + S.rsum[3][t]);
+      }
     }
     if (t == 0) tc::bulk_wait_all();
     if (!ok) S.abort = 1;
@@ -535,10 +580,10 @@ bool ensure_exact(Context *c)
   const size_t bytes = nel * nchunk * XS_CH_BYTES, rbytes = nel * nchunk * 32 * sizeof(double);
   size_t freeb = 0, totb = 0;
   if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess ||
-      bytes + rbytes + nel * (XS_EXP * sizeof(short) + EBUF * sizeof(double)) + ((size_t)4 << 30) > freeb)
+      bytes + rbytes + nel * (XS_EXP * sizeof(short) + (EBUF + NE) * sizeof(double)) + ((size_t)4 << 30) > freeb)
     return false;
   int *d_bad = nullptr;
-  bool ok = ensure_ebuf(c) && cudaMalloc(&c->d_xops, bytes) == cudaSuccess &&
+  bool ok = ensure_ebuf(c) && ensure_rbuf(c) && cudaMalloc(&c->d_xops, bytes) == cudaSuccess &&
             cudaMalloc(&c->d_xexp, nel * XS_EXP * sizeof(short)) == cudaSuccess &&
             cudaMalloc(&c->d_xrow, rbytes) == cudaSuccess && cudaMalloc(&d_bad, sizeof(int)) == cudaSuccess;
   const size_t smem = sizeof(double) * XS_ROWS * (nchunk * 32 + 1);
@@ -569,8 +614,9 @@ bool ensure_exact(Context *c)
   return true;
 }
 
-// Element matrices of every element into the element buffers, then the gather.
-int launch_exact_tangent(Context *c, double *vals)
+// Element matrices and / or residuals of every element into the element
+// buffers, then the gathers (RR, vals null: not wanted).
+int launch_exact(Context *c, double *RR, double *vals)
 {
   int dev = 0, nsm = 0;
   IGAP_CUDA(cudaGetDevice(&dev));
@@ -580,15 +626,20 @@ int launch_exact_tangent(Context *c, double *vals)
   a.ops = (const unsigned char *)c->d_xops;
   a.expo = c->d_xexp;
   a.row80 = c->d_xrow;
-  a.ebuf = c->d_ebuf;
+  a.ebuf = vals ? c->d_ebuf : nullptr;
+  a.U = RR ? c->d_Uhist : nullptr;
+  a.rbuf = c->d_rbuf;
+  a.m = c->devmesh();
   a.nelem = c->nelem_total;
   a.nchunk = (npts + PW - 1) / PW;
   a.lam = c->par[0];
   a.mu = c->par[1];
   a.laws = nullptr;
+  a.meshes = nullptr;
+  a.eoff = nullptr;
   a.einst = nullptr;
   a.err = c->d_err;
-  if (c->batch) batch_law_map(c, &a.laws, &a.einst);
+  if (c->batch) batch_element_map(c, &a.laws, &a.meshes, &a.eoff, &a.einst);
   const size_t smem = sizeof(XsSmem) + 1024;
   static bool attr_set = false;
   if (!attr_set) {
@@ -612,7 +663,8 @@ int launch_exact_tangent(Context *c, double *vals)
     c->prof_elements[0] += c->nelem_total;
   }
   c->exact_ran = true;
-  return launch_tangent_gather(c, vals, c->d_err);
+  const int r = RR ? launch_residual_gather(c, RR, c->d_err) : IGAPGPU_OK;
+  return r || !vals ? r : launch_tangent_gather(c, vals, c->d_err);
 }
 
 }  // namespace igap
