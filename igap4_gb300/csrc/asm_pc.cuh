@@ -183,7 +183,7 @@ static __global__ void __launch_bounds__(AS_THREADS) asm_setup_kernel(const int6
 // stride), lane c < 3 (cell points) computes the cell's DOF c in FP64 from
 // the FP32 rows.
 __device__ __forceinline__ void asm_apply(double *z, const double *v, const float *__restrict__ Z, const CellGeom &g,
-                                          int64_t ncell)
+                                          int64_t ncell, double scale = 1.0)
 {
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -195,7 +195,7 @@ __device__ __forceinline__ void asm_apply(double *z, const double *v, const floa
       const float *row = Z + (size_t)cell * AS_NC * AS_N + (size_t)lane * AS_N;
       double s = 0.0;
       for (int b = 0; b < 3 * ne; b++) s = fma((double)row[b], v[3 * cps[b / 3] + b % 3], s);
-      z[3 * cps[core[lane / 3]] + lane % 3] = s;
+      z[3 * cps[core[lane / 3]] + lane % 3] = scale * s;
     }
   }
 }

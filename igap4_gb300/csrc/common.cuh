@@ -337,7 +337,7 @@ int setup_pc(Context *c, int pc, const double **pcd);
 // krylov_cycle.cu: GMRES restart cycles as one cooperative kernel each
 bool cycle_applies(const Context *c, int m);
 int ksp_cycles(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int m, int pc, const double *pcd,
-               double *V, double *Z, double *w, bool cap, int *its, double *rnorm);
+               double *V, double *Z, double *w, double *wd, bool cap, int *its, double *rnorm);
 int launch_diag_reciprocal(Context *c, double *inv);
 void cycle_release(Context *c);
 struct CellGeom;

@@ -18,9 +18,16 @@
 //    step and is kept in every block's shared memory, and h = T V^T w;
 //  * opts.orth = 1 (classical Gram-Schmidt twice) runs the same two passes
 //    twice with T = I;
-//  * the Givens chain of a column runs on one warp while the other warps
-//    multiply for the next step; the cycle stops one multiply later than the
-//    test, with the same iterate;
+//  * the convergence test needs only the last rotated entry of a column, a
+//    dot product of the column with one row of the accumulated rotations,
+//    which every block carries; the rotations themselves are applied to all
+//    columns at once at the end of the cycle.  One warp does the test while
+//    the others multiply for the next step; the cycle stops one multiply later
+//    than the test, with the same iterate (the chain of rotations per step
+//    held up every barrier by 14 k clocks);
+//  * three grid barriers a step (3.5 k clocks each): the vector is normalised
+//    while the multiply gathers it, the preconditioned copy (Jacobi) having
+//    been written beside the update; the block preconditioners take a fourth;
 //  * the FP64 pipe (2 FMA per clock and SM) bounds the stages, so cross-lane
 //    sums are merged: a warp of the multiply owns the three rows of a control
 //    point (one gather of x for three products), a warp of the projection
@@ -55,22 +62,21 @@ constexpr uint32_t CY_WAIT_LIMIT = 1u << 24;
 
 struct CycleState {
   int its;        // Arnoldi steps of this cycle
-  int stop;       // the cycle ended before its last step (converged or broke down)
   double beta;    // |r| at the start of the cycle
   double rnorm;   // residual estimate
   double rnorm0;  // |r| of the first cycle (negative before it)
   double tol;
 };
 
-struct CycleArgs {
+struct CycleArgs {  // w: two buffers, one the current vector, the other its product
   const int64_t *rowptr;
   const int32_t *cols;
   const double *vals;
   const double *b;
-  double *x, *w, *V, *Z;
+  double *x, *w, *wd, *V, *Z;  // wd: the current vector times the reciprocal diagonal (no or scalar preconditioner)
   const double *pcd;   // Jacobi: reciprocal diagonal; block preconditioners: their blocks
   double *H;           // [m][m + 1] columns
-  double *cs, *sn, *g, *y;
+  double *y;
   double *part;        // projection partial sums [2][vectors][CY_RMAX]
   double *npart;       // norm partial sums [2][blocks]
   CycleState *st;
@@ -85,9 +91,13 @@ struct CycleArgs {
 struct CycleSmem {
   double red[CY_THREADS];
   double r[CY_MAX_RESTART + 1], l[CY_MAX_RESTART + 1], h[CY_MAX_RESTART + 1];
+  // rotations, their diagonal, the rotated right-hand side, the last row of the accumulated rotations
+  double cs[CY_MAX_RESTART + 1], sn[CY_MAX_RESTART + 1], den[CY_MAX_RESTART + 1], g[CY_MAX_RESTART + 2],
+      q[CY_MAX_RESTART + 2];
   double bc;           // a broadcast sum
-  int ok;
-  // packed rows of T (row i: entries c < i at i (i - 1) / 2) follow
+  int ok, stop;
+  // packed rows of T (row i: entries c < i at i (i - 1) / 2) follow; at the end
+  // of the cycle packed columns of H (column c: entries i <= c at c (c + 1) / 2)
 };
 
 // All blocks arrive and wait.  Fences at GPU scope by thread 0 (one before the
@@ -117,17 +127,16 @@ __device__ __forceinline__ bool grid_sync(const CycleArgs &a, CycleSmem &S, unsi
   return S.ok != 0;
 }
 
-// Sum of s over the block in a fixed order: the threads' values through
-// shared memory, then one warp (37 instead of 165 FP64 warp additions).
-// Valid in thread 0.
-__device__ __forceinline__ double block_sum(CycleSmem &S, double s)
+// Sum of s over the first `warps` warps of the block (the others hold none) in
+// a fixed order: through shared memory, then one warp.  Valid in thread 0.
+__device__ __forceinline__ double block_sum(CycleSmem &S, double s, int warps)
 {
-  S.red[threadIdx.x] = s;
+  if (threadIdx.x < 32 * warps) S.red[threadIdx.x] = s;
   __syncthreads();
   double t = 0.0;
   if (threadIdx.x < 32) {
-#pragma unroll
-    for (int k = 0; k < CY_WARPS; k++) t += S.red[threadIdx.x + 32 * k];
+#pragma unroll 4
+    for (int k = 0; k < warps; k++) t += S.red[threadIdx.x + 32 * k];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   }
@@ -172,11 +181,11 @@ __device__ __forceinline__ double fold3(double s0, double s1, double s2, int sub
   return v;
 }
 
-// w = A x (or b - A x with RES) over this grid's groups of G lanes, one
-// control point (three rows sharing their columns) per group; returns this
-// thread's part of |w|^2 with RES.
+// w = scale A x (or w = b - A x and wd = M^-1 w with RES) over this grid's
+// groups of G lanes, one control point (three rows sharing their columns) per
+// group; returns this thread's part of |w|^2 with RES.
 template <int G, bool RES>
-__device__ __forceinline__ double multiply(const CycleArgs &a, const double *x, double *w)
+__device__ __forceinline__ double multiply(const CycleArgs &a, const double *x, double *w, double scale)
 {
   const int64_t ncp = a.n / 3;
   const int sub = threadIdx.x % G;
@@ -207,6 +216,9 @@ __device__ __forceinline__ double multiply(const CycleArgs &a, const double *x, 
       if (RES) {
         v = a.b[row] - v;
         nn = fma(v, v, nn);
+        if (a.pc <= 1) a.wd[row] = a.pc ? v * __ldg(a.pcd + row) : v;
+      } else {
+        v *= scale;
       }
       w[row] = v;
     }
@@ -215,10 +227,11 @@ __device__ __forceinline__ double multiply(const CycleArgs &a, const double *x, 
 }
 
 template <bool RES>
-__device__ __forceinline__ double multiply_any(const CycleArgs &a, const double *x, double *w)
+__device__ __forceinline__ double multiply_any(const CycleArgs &a, const double *x, double *w, double scale)
 {
   // 32 lanes a control point while there are fewer points than groups of 16
-  return a.n / 3 < (int64_t)gridDim.x * CY_WARPS * 2 ? multiply<32, RES>(a, x, w) : multiply<16, RES>(a, x, w);
+  return a.n / 3 < (int64_t)gridDim.x * CY_WARPS * 2 ? multiply<32, RES>(a, x, w, scale)
+                                                     : multiply<16, RES>(a, x, w, scale);
 }
 
 // Folds NS sums (4 or 8) over the lanes of a warp: each exchange halves the
@@ -250,7 +263,7 @@ __device__ __forceinline__ int fold(double (&s)[2 * CY_VB], int lane)
 // Partial dot products of the basis vectors 0..j with w (and, with LROW, with
 // v_j): item (group of CY_VB vectors, row chunk) per warp.
 template <bool LROW>
-__device__ __forceinline__ void project_partial(const CycleArgs &a, int j, int R)
+__device__ __forceinline__ void project_partial(const CycleArgs &a, const double *w, int j, int R)
 {
   const int lane = threadIdx.x & 31;
   const int ngroup = (j + CY_VB) / CY_VB;
@@ -267,7 +280,7 @@ __device__ __forceinline__ void project_partial(const CycleArgs &a, int j, int R
     for (int q = 0; q < 2 * CY_VB; q++) s[q] = 0.0;
 #pragma unroll 2
     for (int64_t k = lo + lane; k < hi; k += 32) {
-      const double wk = __ldcg(a.w + k);
+      const double wk = __ldcg(w + k);
       const double vk = LROW ? __ldcg(vj + k) : 0.0;
 #pragma unroll
       for (int q = 0; q < CY_VB; q++) {
@@ -315,7 +328,7 @@ __device__ __forceinline__ double *t_row(CycleSmem &S, int i)
 __device__ __forceinline__ void solve_t(CycleSmem &S, int j)
 {
   const int width = (j + 32) & ~31;             // threads per slice of the sums
-  const int ns = CY_THREADS / width;            // slices
+  const int ns = min(8, CY_THREADS / width);    // slices: their sums are a serial chain
   const int c = threadIdx.x % width, sl = threadIdx.x / width;
   // t_j[c] = -(l_c + sum_{c < k < j} l_k T[k][c])
   double s = 0.0;
@@ -343,23 +356,27 @@ __device__ __forceinline__ void solve_t(CycleSmem &S, int j)
   __syncthreads();
 }
 
-// w -= V h on this block's rows (h = hs); returns this thread's part of |w|^2.
-// With fewer rows than threads the basis vectors are split over ns threads a
-// row and their sums joined through shared memory.
-__device__ __forceinline__ double update_w(const CycleArgs &a, CycleSmem &S, const double *hs, int j)
+// w -= V h on this block's rows (h = hs) and wd = M^-1 w; returns this thread's
+// part of |w|^2, held by the first `warps` warps.  With fewer rows than threads
+// the basis vectors are split over ns threads a row and their sums joined
+// through shared memory.
+__device__ __forceinline__ double update_w(const CycleArgs &a, CycleSmem &S, double *w, const double *hs, int j,
+                                           int &warps)
 {
   const int64_t per = (a.n + gridDim.x - 1) / gridDim.x;
   const int64_t lo = (int64_t)blockIdx.x * per, hi = lo + per < a.n ? lo + per : a.n;
   double nn = 0.0;
   int width = 32;
   while (width < per && width < CY_THREADS) width *= 2;
+  warps = width / 32;
   const int ns = CY_THREADS / width < 8 ? CY_THREADS / width : 8;
   if (ns == 1) {
     for (int64_t r = lo + threadIdx.x; r < hi; r += CY_THREADS) {
-      double s = __ldcg(a.w + r);
+      double s = __ldcg(w + r);
 #pragma unroll 8
       for (int i = 0; i <= j; i++) s = fma(-hs[i], __ldcg(a.V + (size_t)i * a.n + r), s);
-      a.w[r] = s;
+      w[r] = s;
+      if (a.pc <= 1) a.wd[r] = a.pc ? s * __ldg(a.pcd + r) : s;
       nn = fma(s, s, nn);
     }
     return nn;
@@ -376,106 +393,102 @@ __device__ __forceinline__ double update_w(const CycleArgs &a, CycleSmem &S, con
   }
   __syncthreads();
   if (sl == 0 && r < hi) {
-    double s = __ldcg(a.w + r);
+    double s = __ldcg(w + r);
     for (int q = 0; q < ns; q++) s -= S.red[q * width + c];
-    a.w[r] = s;
+    w[r] = s;
+    if (a.pc <= 1) a.wd[r] = a.pc ? s * __ldg(a.pcd + r) : s;
     nn = s * s;
   }
   __syncthreads();
   return nn;
 }
 
-// v = w / den on this block's rows and, without or with scalar Jacobi
-// preconditioning, z = M^-1 v.
-__device__ __forceinline__ void normalise(const CycleArgs &a, double den, double *v, double *z)
+// v = inv w on this block's rows.
+__device__ __forceinline__ void normalise(const CycleArgs &a, const double *w, double inv, double *v)
 {
   const int64_t per = (a.n + gridDim.x - 1) / gridDim.x;
   const int64_t lo = (int64_t)blockIdx.x * per, hi = lo + per < a.n ? lo + per : a.n;
-  const double inv = 1.0 / den;
-  for (int64_t r = lo + threadIdx.x; r < hi; r += CY_THREADS) {
-    const double t = __ldcg(a.w + r) * inv;
-    v[r] = t;
-    if (a.pc == 0) z[r] = t;
-    else if (a.pc == 1) z[r] = t * __ldg(a.pcd + r);
-  }
+  for (int64_t r = lo + threadIdx.x; r < hi; r += CY_THREADS) v[r] = __ldcg(w + r) * inv;
 }
 
-__device__ __forceinline__ void block_precondition(const CycleArgs &a, const double *v, double *z)
+__device__ __forceinline__ void block_precondition(const CycleArgs &a, const double *v, double *z, double scale)
 {
-  if (a.pc == 2) bdiag_apply(z, v, a.pcd, a.n / 3);
-  else if (a.pc == 3) cblock_apply(z, v, a.pcd, a.cg, cell_count(a.cg));
-  else asm_apply(z, v, reinterpret_cast<const float *>(a.pcd), a.cg, cell_count(a.cg));
+  if (a.pc == 2) bdiag_apply(z, v, a.pcd, a.n / 3, scale);
+  else if (a.pc == 3) cblock_apply(z, v, a.pcd, a.cg, cell_count(a.cg), scale);
+  else asm_apply(z, v, reinterpret_cast<const float *>(a.pcd), a.cg, cell_count(a.cg), scale);
 }
 
-// Givens update of Hessenberg column j by one warp (lane 0 runs the chain on
-// values staged in shared memory) and the convergence test.
-__device__ void givens(const CycleArgs &a, double *sh, int j)
+// Rotation of Hessenberg column j (S.h, norm hn below it) and the convergence
+// test, by one warp of every block: the column's last rotated entry is
+// q . h with q the last row of the accumulated rotations.
+__device__ __forceinline__ void rotate(CycleSmem &S, int j, double hn, double tol)
 {
   const int lane = threadIdx.x & 31;
-  double *h = a.H + (size_t)j * (a.m + 1);
-  double *hh = sh, *cc = sh + CY_MAX_RESTART + 2, *ss = cc + CY_MAX_RESTART + 2;
-  for (int i = lane; i <= j + 1; i += 32) hh[i] = __ldcg(h + i);
-  for (int i = lane; i < j; i += 32) {
-    cc[i] = __ldcg(a.cs + i);
-    ss[i] = __ldcg(a.sn + i);
-  }
-  __syncwarp();
+  double hi = 0.0;
+  for (int i = lane; i <= j; i += 32) hi = fma(S.q[i], S.h[i], hi);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) hi += __shfl_xor_sync(0xffffffffu, hi, o);
+  double den = hypot(hi, hn);
+  const bool breakdown = !(den > 0.0) || !isfinite(den);
+  if (breakdown) den = 1e-300;
+  const double c = hi / den, s = hn / den;
+  for (int i = lane; i <= j; i += 32) S.q[i] *= -s;
   if (lane == 0) {
-    double hi = hh[0];
-    for (int i = 0; i < j; i++) {
-      const double hn = hh[i + 1];
-      hh[i] = fma(ss[i], hn, cc[i] * hi);
-      hi = fma(-ss[i], hi, cc[i] * hn);
-    }
-    const double hl = hh[j + 1];
-    double den = hypot(hi, hl);
-    const bool breakdown = !(den > 0.0) || !isfinite(den);
-    if (breakdown) den = 1e-300;
-    const double c = hi / den, s = hl / den;
-    a.cs[j] = c;
-    a.sn[j] = s;
-    hh[j] = den;
-    hh[j + 1] = 0.0;
-    const double gj = __ldcg(a.g + j), gn = -s * gj;
-    a.g[j] = c * gj;
-    a.g[j + 1] = gn;
-    a.st->rnorm = fabs(gn);
-    a.st->its = j + 1;
-    if (fabs(gn) <= a.st->tol || breakdown || !isfinite(gn)) a.st->stop = 1;
+    S.q[j + 1] = c;
+    S.cs[j] = c;
+    S.sn[j] = s;
+    S.den[j] = den;
+    const double gj = S.g[j], gn = -s * gj;
+    S.g[j] = c * gj;
+    S.g[j + 1] = gn;
+    S.stop = (fabs(gn) <= tol || breakdown || !isfinite(gn)) ? 1 : 0;
   }
-  __syncwarp();
-  for (int i = lane; i <= j + 1; i += 32) h[i] = hh[i];
 }
 
-// y = H(0:k, 0:k)^-1 g by one block, column by column.
+// y = R^-1 g of the k columns by one block: the columns of H to shared memory,
+// every thread rotates one, one warp substitutes backwards.
 __device__ void backsolve(const CycleArgs &a, CycleSmem &S, int k)
 {
-  for (int i = threadIdx.x; i < k; i += CY_THREADS) S.h[i] = __ldcg(a.g + i);
-  for (int i = k - 1; i >= 0; i--) {
-    const double *col = a.H + (size_t)i * (a.m + 1);
-    const double hc = threadIdx.x <= i ? __ldcg(col + threadIdx.x) : 0.0;
-    __syncthreads();
-    if (threadIdx.x == i) S.bc = S.h[i] = S.h[i] / hc;
-    __syncthreads();
-    if (threadIdx.x < i) S.h[threadIdx.x] = fma(-hc, S.bc, S.h[threadIdx.x]);
+  double *R = reinterpret_cast<double *>(&S + 1);
+  __syncthreads();
+  for (int c = threadIdx.x >> 5; c < k; c += CY_WARPS)
+    for (int i = threadIdx.x & 31; i <= c; i += 32) R[c * (c + 1) / 2 + i] = __ldcg(a.H + (size_t)c * (a.m + 1) + i);
+  __syncthreads();
+  if (threadIdx.x < k) {
+    const int c = threadIdx.x;
+    double *col = R + c * (c + 1) / 2, hi = col[0];
+    for (int i = 0; i < c; i++) {
+      const double hn = col[i + 1];
+      col[i] = fma(S.sn[i], hn, S.cs[i] * hi);
+      hi = fma(-S.sn[i], hi, S.cs[i] * hn);
+    }
+    S.den[c] = 1.0 / S.den[c];
+    S.h[c] = S.g[c];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < k; i += CY_THREADS) a.y[i] = S.h[i];
+  if (threadIdx.x < 32)
+    for (int c = k - 1; c >= 0; c--) {
+      const double *col = R + c * (c + 1) / 2;
+      const double y = S.h[c] * S.den[c];
+      __syncwarp();
+      for (int i = threadIdx.x; i < c; i += 32) S.h[i] = fma(-col[i], y, S.h[i]);
+      if (threadIdx.x == 0) a.y[c] = y;
+      __syncwarp();
+    }
 }
 
 __global__ void __launch_bounds__(CY_THREADS, 1) gmres_cycle_kernel(CycleArgs a)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CycleSmem &S = *reinterpret_cast<CycleSmem *>(smem_raw);
-  __shared__ double gsh[3 * (CY_MAX_RESTART + 2)];
-  __shared__ int s_stop;
   unsigned target = 0;
   const int tid = threadIdx.x, warp = tid >> 5;
   const bool last_block = blockIdx.x == gridDim.x - 1;
   CycleState *st = a.st;
+  double *wcur = a.w, *wnext = a.w + a.n;
   // r = b - A x, beta = |r|
   {
-    const double nn = block_sum(S, multiply_any<true>(a, a.x, a.w));
+    const double nn = block_sum(S, multiply_any<true>(a, a.x, wcur, 1.0), CY_WARPS);
     if (tid == 0) a.npart[blockIdx.x] = nn;
   }
   if (!grid_sync(a, S, target)) return;
@@ -489,30 +502,32 @@ __global__ void __launch_bounds__(CY_THREADS, 1) gmres_cycle_kernel(CycleArgs a)
     st->tol = tol;
     st->beta = st->rnorm = beta;
     st->its = 0;
-    st->stop = go ? 0 : 1;
-    a.g[0] = beta;
   }
   if (!go) return;
-  normalise(a, beta, a.V, a.Z);
-  if (!grid_sync(a, S, target)) return;
+  if (tid == 0) {
+    S.g[0] = beta;
+    S.q[0] = 1.0;
+    S.stop = 0;
+  }
   int k = 0;
+  double den = beta;
   for (int j = 0; j < a.steps; j++) {
     double *vj = a.V + (size_t)j * a.n, *zj = a.Z + (size_t)j * a.n;
+    const double inv = 1.0 / den;
     if (a.pc >= 2) {
-      block_precondition(a, vj, zj);
+      block_precondition(a, wcur, zj, inv);
+      normalise(a, wcur, inv, vj);
       if (!grid_sync(a, S, target)) return;
+    } else {
+      normalise(a, wcur, inv, vj);
     }
-    // the previous column's rotation beside the multiply
-    if (j > 0 && last_block && warp == CY_WARPS - 1) givens(a, gsh, j - 1);
-    multiply_any<false>(a, zj, a.w);
+    // the previous column's test beside the multiply
+    if (j > 0 && warp == CY_WARPS - 1) rotate(S, j - 1, den, tol);
+    multiply_any<false>(a, a.pc >= 2 ? zj : a.wd, wnext, a.pc >= 2 ? 1.0 : inv);
     if (!grid_sync(a, S, target)) return;
-    if (j > 0) {
-      if (tid == 0) s_stop = *(volatile int *)&st->stop;
-      __syncthreads();
-      if (s_stop) {
-        k = j;
-        break;
-      }
+    if (S.stop) {
+      k = j;
+      break;
     }
     // orthogonalise
     const int ngroup = (j + CY_VB) / CY_VB;
@@ -522,51 +537,56 @@ __global__ void __launch_bounds__(CY_THREADS, 1) gmres_cycle_kernel(CycleArgs a)
     R = R < rmax ? R : (int)rmax;
     R = R > 0 ? R : 1;
     double nn;
+    int warps;
     if (a.orth == 1) {
-      project_partial<false>(a, j, R);
+      project_partial<false>(a, wnext, j, R);
       if (!grid_sync(a, S, target)) return;
       project_total<false>(a, S, j, R);
-      update_w(a, S, S.r, j);
+      update_w(a, S, wnext, S.r, j, warps);
       if (tid <= j) S.h[tid] = S.r[tid];
       if (!grid_sync(a, S, target)) return;
-      project_partial<false>(a, j, R);
+      project_partial<false>(a, wnext, j, R);
       if (!grid_sync(a, S, target)) return;
       project_total<false>(a, S, j, R);
-      nn = update_w(a, S, S.r, j);
+      nn = update_w(a, S, wnext, S.r, j, warps);
       if (tid <= j) S.h[tid] += S.r[tid];
     } else {
-      project_partial<true>(a, j, R);
+      project_partial<true>(a, wnext, j, R);
       if (!grid_sync(a, S, target)) return;
       project_total<true>(a, S, j, R);
       solve_t(S, j);
-      nn = update_w(a, S, S.h, j);
+      nn = update_w(a, S, wnext, S.h, j, warps);
     }
-    nn = block_sum(S, nn);
+    nn = block_sum(S, nn, warps);
     if (tid == 0) a.npart[gridDim.x * (1 + (j & 1)) + blockIdx.x] = nn;
+    if (last_block && tid <= j) a.H[(size_t)j * (a.m + 1) + tid] = S.h[tid];
     if (!grid_sync(a, S, target)) return;
-    const double hn = total_norm(a, S, 1 + (j & 1));
-    if (last_block) {
-      if (tid <= j) a.H[(size_t)j * (a.m + 1) + tid] = S.h[tid];
-      if (tid == 0) a.H[(size_t)j * (a.m + 1) + j + 1] = hn;
-    }
-    if (j + 1 < a.steps) {
-      normalise(a, hn, vj + a.n, zj + a.n);
-    } else {
-      __syncthreads();
-      if (last_block && warp == CY_WARPS - 1) givens(a, gsh, j);
-      k = j + 1;
-    }
-    if (!grid_sync(a, S, target)) return;
+    den = total_norm(a, S, 1 + (j & 1));
+    double *t = wcur;
+    wcur = wnext;
+    wnext = t;
+    k = j + 1;
   }
-  // x += Z y
-  if (last_block) backsolve(a, S, k);
+  // the last column of a full cycle has not been rotated yet
+  if (!S.stop && warp == CY_WARPS - 1) rotate(S, k - 1, den, tol);
+  __syncthreads();
+  // x += M^-1 V y
+  if (last_block) {
+    backsolve(a, S, k);
+    if (tid == 0) {
+      st->its = k;
+      st->rnorm = fabs(S.g[k]);
+    }
+  }
   if (!grid_sync(a, S, target)) return;
   for (int i = tid; i < k; i += CY_THREADS) S.h[i] = __ldcg(a.y + i);
   __syncthreads();
+  const double *B = a.pc >= 2 ? a.Z : a.V;
   for (int64_t r = (int64_t)blockIdx.x + (int64_t)gridDim.x * tid; r < a.n; r += (int64_t)gridDim.x * CY_THREADS) {
-    double s = a.x[r];
-    for (int i = 0; i < k; i++) s = fma(S.h[i], __ldcg(a.Z + (size_t)i * a.n + r), s);
-    a.x[r] = s;
+    double s = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < k; i++) s = fma(S.h[i], __ldcg(B + (size_t)i * a.n + r), s);
+    a.x[r] += a.pc == 1 ? s * __ldg(a.pcd + r) : s;
   }
 }
 
@@ -589,7 +609,7 @@ __global__ void diag_reciprocal_kernel(const int64_t *rowptr, const int32_t *col
 
 struct CycleWork {
   int m = 0, grid = 0;
-  double *buf = nullptr;      // H, cs, sn, g, y, partial sums
+  double *buf = nullptr;      // H, y, partial sums
   unsigned *ctl = nullptr;    // barrier counter, error word (128 B apart), state
   CycleState *h_st = nullptr; // pinned: state and error word
 };
@@ -616,7 +636,7 @@ static int ensure_cycle(Context *c, int m)
   int dev = 0, nsm = 0;
   IGAP_CUDA(cudaGetDevice(&dev));
   IGAP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const size_t cnt = (size_t)(m + 1) * m + 4 * (size_t)(m + 1) + 2 * (size_t)(m + 1) * CY_RMAX + 3 * (size_t)nsm;
+  const size_t cnt = (size_t)(m + 1) * m + (size_t)(m + 1) + 2 * (size_t)(m + 1) * CY_RMAX + 3 * (size_t)nsm;
   if (cudaMalloc(&cw->buf, sizeof(double) * cnt) != cudaSuccess || cudaMalloc(&cw->ctl, CY_CTL_BYTES) != cudaSuccess ||
       cudaMallocHost(&cw->h_st, CY_CTL_BYTES) != cudaSuccess) {
     cudaGetLastError();
@@ -629,7 +649,7 @@ static int ensure_cycle(Context *c, int m)
   return IGAPGPU_OK;
 }
 
-static size_t cycle_smem(int m) { return sizeof(CycleSmem) + sizeof(double) * ((size_t)m * (m - 1) / 2 + 1); }
+static size_t cycle_smem(int m) { return sizeof(CycleSmem) + sizeof(double) * ((size_t)m * (m + 1) / 2); }
 
 // Whether the cycle kernel takes this solve (19 times faster than the separate
 // launches at 32x8x8, so up to the longest restart that fits): T fits in shared memory, the
@@ -637,11 +657,11 @@ static size_t cycle_smem(int m) { return sizeof(CycleSmem) + sizeof(double) * ((
 bool cycle_applies(const Context *c, int m) { return m <= CY_MAX_RESTART && !spmv_df(c); }
 
 // GMRES cycles on the context matrix; b, x device vectors, pcd the
-// preconditioner's data, V and Z the basis buffers.  `cap`: stop at ksp_max_it
+// preconditioner's data, V and Z the basis buffers, w 2 n and wd n scratch.  `cap`: stop at ksp_max_it
 // inside a cycle and return the true residual norm (else whole cycles and the
 // recurrence's estimate).
 int ksp_cycles(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int m, int pc, const double *pcd,
-               double *V, double *Z, double *w, bool cap, int *its_out, double *rnorm_out)
+               double *V, double *Z, double *w, double *wd, bool cap, int *its_out, double *rnorm_out)
 {
   int r = ensure_cycle(c, m);
   if (r) return r;
@@ -654,14 +674,12 @@ int ksp_cycles(Context *c, const double *b, double *x, const igapgpu_solver_opts
   a.b = b;
   a.x = x;
   a.w = w;
+  a.wd = wd;
   a.V = V;
   a.Z = Z;
   a.pcd = pcd;
   a.H = cw->buf;
-  a.cs = a.H + (size_t)(cw->m + 1) * cw->m;
-  a.sn = a.cs + cw->m + 1;
-  a.g = a.sn + cw->m + 1;
-  a.y = a.g + cw->m + 1;
+  a.y = a.H + (size_t)(cw->m + 1) * cw->m;
   a.part = a.y + cw->m + 1;
   a.npart = a.part + 2 * (size_t)(cw->m + 1) * CY_RMAX;
   a.bar = cw->ctl;

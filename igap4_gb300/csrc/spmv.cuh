@@ -245,7 +245,7 @@ static __global__ void __launch_bounds__(32 * CB_WARPS) cblock_invert_kernel(con
 // computes the cell's DOF a (grid-stride over cells); the block's columns
 // come as coalesced loads independent of each other, v through shuffles.  v may have been
 // written earlier in the same kernel (no read-only loads of v here and below).
-__device__ __forceinline__ void cblock_apply(double *z, const double *v, const double *__restrict__ inv, const CellGeom &g, int64_t ncell)
+__device__ __forceinline__ void cblock_apply(double *z, const double *v, const double *__restrict__ inv, const CellGeom &g, int64_t ncell, double scale = 1.0)
 {
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -261,20 +261,21 @@ __device__ __forceinline__ void cblock_apply(double *z, const double *v, const d
     double s = 0.0;
 #pragma unroll 12
     for (int b = 0; b < CBS; b++) s = fma(__ldg(col + b * CBS), __shfl_sync(0xffffffffu, vl, b), s);
-    if (lane < bs) z[dof] = s;
+    if (lane < bs) z[dof] = scale * s;
   }
 }
 
 // z = B^-1 v with the inverted blocks
-__device__ __forceinline__ void bdiag_apply(double *z, const double *v, const double *__restrict__ inv, int64_t ncp)
+__device__ __forceinline__ void bdiag_apply(double *z, const double *v, const double *__restrict__ inv, int64_t ncp,
+                                            double scale = 1.0)
 {
   for (int64_t cp = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; cp < ncp;
        cp += (int64_t)gridDim.x * blockDim.x) {
     const double *b = inv + 9 * cp;
     const double v0 = v[3 * cp], v1 = v[3 * cp + 1], v2 = v[3 * cp + 2];
-    z[3 * cp] = b[0] * v0 + b[1] * v1 + b[2] * v2;
-    z[3 * cp + 1] = b[3] * v0 + b[4] * v1 + b[5] * v2;
-    z[3 * cp + 2] = b[6] * v0 + b[7] * v1 + b[8] * v2;
+    z[3 * cp] = scale * (b[0] * v0 + b[1] * v1 + b[2] * v2);
+    z[3 * cp + 1] = scale * (b[3] * v0 + b[4] * v1 + b[5] * v2);
+    z[3 * cp + 2] = scale * (b[6] * v0 + b[7] * v1 + b[8] * v2);
   }
 }
 
