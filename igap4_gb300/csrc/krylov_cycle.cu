@@ -307,11 +307,16 @@ __device__ __forceinline__ void project_total(const CycleArgs &a, CycleSmem &S, 
     double s[2 * CY_VB];
 #pragma unroll
     for (int q = 0; q < 2 * CY_VB; q++) s[q] = 0.0;
+    const double *p[NS];
 #pragma unroll
-    for (int q = 0; q < NS; q++) {
-      const int i = min(g * CY_VB + q % CY_VB, j);
-      const double *p = a.part + ((size_t)(q / CY_VB) * (a.m + 1) + i) * CY_RMAX;
-      for (int r = lane; r < R; r += 32) s[q] += __ldcg(p + r);
+    for (int q = 0; q < NS; q++)
+      p[q] = a.part + ((size_t)(q / CY_VB) * (a.m + 1) + min(g * CY_VB + q % CY_VB, j)) * CY_RMAX;
+    for (int r = lane; r < R; r += 32) {
+      double t[NS];  // every sum's load in flight at once
+#pragma unroll
+      for (int q = 0; q < NS; q++) t[q] = __ldcg(p[q] + r);
+#pragma unroll
+      for (int q = 0; q < NS; q++) s[q] += t[q];
     }
     const int id = fold<NS>(s, lane), i = g * CY_VB + id % CY_VB;
     if ((lane & (32 / NS - 1)) == 0 && i <= j) (id < CY_VB ? S.r : S.l)[i] = s[0];
@@ -532,7 +537,7 @@ __global__ void __launch_bounds__(CY_THREADS, 1) gmres_cycle_kernel(CycleArgs a)
     // orthogonalise
     const int ngroup = (j + CY_VB) / CY_VB;
     int R = (int)(gridDim.x * CY_WARPS) / ngroup;
-    const int64_t rmax = (a.n + 159) / 160;
+    const int64_t rmax = (a.n + 159) / 160;  // at least five rows a lane: fewer partial sums for every block to add
     R = R < CY_RMAX ? R : CY_RMAX;
     R = R < rmax ? R : (int)rmax;
     R = R > 0 ? R : 1;

@@ -250,8 +250,8 @@ __device__ __forceinline__ void cblock_apply(double *z, const double *v, const d
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t cell = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); cell < ncell; cell += nw) {
-    const int z0 = 2 * (int)(cell % g.nc[2]), y0 = 2 * (int)(cell / g.nc[2] % g.nc[1]),
-              x0 = 2 * (int)(cell / ((int64_t)g.nc[1] * g.nc[2]));
+    const int ci = (int)cell, cyz = ci / g.nc[2];  // fewer than 2^31 cells (2^31 rows at most)
+    const int z0 = 2 * (ci - cyz * g.nc[2]), x0 = 2 * (cyz / g.nc[1]), y0 = 2 * cyz - x0 * g.nc[1];
     const int nz = min(2, g.nb[2] - z0), ny = min(2, g.nb[1] - y0), nyz = ny * nz;
     const int bs = 3 * min(2, g.nb[0] - x0) * nyz;
     const int p = lane / 3;
