@@ -94,10 +94,12 @@ __global__ void axpy_dev_kernel(double *y, const double *x, const double *palpha
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = fma(a, x[i], y[i]);
 }
+// y = a x + b y; with b = 0 y is only written (it may be uninitialised memory,
+// whose NaN bits 0 y would keep)
 __global__ void axpby_kernel(double *y, const double *x, double a, double b, int64_t n)
 {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = a * x[i] + b * y[i];
+    y[i] = b != 0.0 ? a * x[i] + b * y[i] : a * x[i];
 }
 // y = x / (*pden)  (device scalar)
 __global__ void scale_div_kernel(double *y, const double *x, const double *pden, int64_t n)
