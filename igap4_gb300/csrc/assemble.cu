@@ -594,6 +594,27 @@ __global__ void dirichlet_matrix_batch_kernel(const int64_t *rows, const int *in
   }
 }
 
+__global__ void dirmap_kernel(const int64_t *rows, int64_t n, int *map)
+{
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) map[rows[t]] = (int)t + 1;
+}
+
+int build_dirmap(Context *c)
+{
+  if (cudaMalloc(&c->d_dirmap, sizeof(int) * (size_t)c->ndof) != cudaSuccess) {
+    cudaGetLastError();
+    c->d_dirmap = nullptr;
+    set_error("Dirichlet map: allocation failed");
+    return IGAPGPU_ERR_NOMEM;
+  }
+  IGAP_CUDA(cudaMemsetAsync(c->d_dirmap, 0, sizeof(int) * (size_t)c->ndof, c->stream));
+  dirmap_kernel<<<(unsigned)((c->n_dir + 255) / 256), 256, 0, c->stream>>>(c->d_dir_rows, c->n_dir, c->d_dirmap);
+  count_launch();
+  IGAP_CHECK_LAUNCH();
+  return IGAPGPU_OK;
+}
+
 int launch_dirichlet_matrix_batch(Context *c, const int *d_inst, const int *d_nbs, const int64_t *d_off,
                                   double *vals)
 {
@@ -669,48 +690,53 @@ __global__ void __launch_bounds__(PW * 32, 1)
 // the weighted outputs in the point-minor layout [element][entry][point], so
 // that a warp's stores are contiguous.
 constexpr int LT_NT = 128;
+// Small meshes: 32 points and 8 warps a block, so that the points spread over
+// the SMs and a warp interpolates 4 points instead of 32 one after the other
+// (85 -> 31 us for the 1,024 points of a 4x2x2 mesh).
+constexpr int LT_SMALL_PT = 32, LT_SMALL_NT = 256;
 // T: the law's arithmetic.  The FP32 law keeps its inputs as floats (the
 // same values its phase 2 used to convert them to), and a launch that copies
 // its inputs (PRE) needs no basis or state: the smaller shared-memory
 // footprints let more CTAs share an SM.
-template <typename T, bool PRE = false>
+template <typename T, bool PRE = false, int PT = LT_NT, int NT = LT_NT>
 struct LawThreadSmem {
   static constexpr bool F32 = sizeof(T) == 4;
-  T sm[30 * LT_NT];
-  T sd[30 * LT_NT];
-  double wt[LT_NT];
-  double R[LT_NT / 32][PRE ? 1 : GEO_STRIDE];
-  double U[LT_NT / 32][F32 || PRE ? 1 : 3 * NE];
-  float Uf[LT_NT / 32][F32 && !PRE ? 3 * NE : 1];  // the element's state in FP32 (float law)
+  T sm[30 * PT];
+  T sd[30 * PT];
+  double wt[PT];
+  double R[NT / 32][PRE ? 1 : GEO_STRIDE];
+  double U[NT / 32][F32 || PRE ? 1 : 3 * NE];
+  float Uf[NT / 32][F32 && !PRE ? 3 * NE : 1];  // the element's state in FP32 (float law)
 };
 
 // T: the law's arithmetic (double; float for the tangent of the split mode,
 // whose contraction runs in TF32x3 on the tensor cores).  PRE: phase 1 copies
 // the law's inputs from lin (pair interpolation, law_in_df_kernel) instead of
 // interpolating them.
-template <int LAWK, bool RES, bool TAN, typename T = double, bool PRE = false>
-__global__ void __launch_bounds__(LT_NT)
+template <int LAWK, bool RES, bool TAN, typename T = double, bool PRE = false, int PT = LT_NT, int NT = LT_NT>
+__global__ void __launch_bounds__(NT)
     law_thread_kernel(DevMesh m, DevLaw L, const double *__restrict__ Uhist, double *__restrict__ preR,
                       double *__restrict__ preD, int64_t npt_total, const double *__restrict__ lin)
 {
   constexpr bool TR = LAWK == 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  LawThreadSmem<T, PRE> &S = *reinterpret_cast<LawThreadSmem<T, PRE> *>(smem_raw);
+  LawThreadSmem<T, PRE, PT, NT> &S = *reinterpret_cast<LawThreadSmem<T, PRE, PT, NT> *>(smem_raw);
+  constexpr int PPW = PT / (NT / 32);  // points a warp prepares
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t p0 = (int64_t)blockIdx.x * LT_NT;
+  const int64_t p0 = (int64_t)blockIdx.x * PT;
   const int nh = L.nhist;
   const int nb1 = m.nbasis[1], nb2 = m.nbasis[2];
   const double rho_m = L.par[5], damp = L.par[6], dt = L.par[7];
   int64_t cur_e = -1;
-  for (int j = 0; j < 32; j++) {
-    const int t = warp * 32 + j;
+  for (int j = 0; j < PPW; j++) {
+    const int t = warp * PPW + j;
     const int64_t p = p0 + t;
     if (p >= npt_total) break;  // uniform over the warp
     if constexpr (PRE) {
       const double *src = lin + p * 64;
       if (lane < 30) {
-        S.sm[lane * LT_NT + t] = lawpt::to_t<T>(__ldg(src + lane));
-        if (TR) S.sd[lane * LT_NT + t] = lawpt::to_t<T>(__ldg(src + 30 + lane));
+        S.sm[lane * PT + t] = lawpt::to_t<T>(__ldg(src + lane));
+        if (TR) S.sd[lane * PT + t] = lawpt::to_t<T>(__ldg(src + 30 + lane));
       }
       if (lane == 30) S.wt[t] = __ldg(src + 60);
     } else {
@@ -754,17 +780,17 @@ __global__ void __launch_bounds__(LT_NT)
           }
         }
         if (!TR) {
-          S.sm[lane * LT_NT + t] = lawpt::to_t<T>(s[0]);
+          S.sm[lane * PT + t] = lawpt::to_t<T>(s[0]);
         } else if (k == 0) {
           // the value slots' inertia and damping term enters the residual only
           // (the tangent's value rows are the constant mass): no FP64 divisions
           // in a tangent-only launch
-          S.sm[lane * LT_NT + t] = RES ? lawpt::to_t<T>(damp * (s[0] - s[2]) / (2.0 * dt) +
+          S.sm[lane * PT + t] = RES ? lawpt::to_t<T>(damp * (s[0] - s[2]) / (2.0 * dt) +
                                                         rho_m * (s[0] + s[2] - 2.0 * s[1]) / (dt * dt))
                                        : T(0);
         } else {
-          S.sm[lane * LT_NT + t] = lawpt::to_t<T>(0.5 * (s[1] + s[2]));
-          S.sd[lane * LT_NT + t] = lawpt::to_t<T>(0.5 * (s[0] - s[2]));
+          S.sm[lane * PT + t] = lawpt::to_t<T>(0.5 * (s[1] + s[2]));
+          S.sd[lane * PT + t] = lawpt::to_t<T>(0.5 * (s[0] - s[2]));
         }
       }
       if (lane == 0) S.wt[t] = S.R[warp][NB * NDD];
@@ -773,12 +799,12 @@ __global__ void __launch_bounds__(LT_NT)
   }
   __syncthreads();
   const int64_t p = p0 + tid;
-  if (p < npt_total) {
+  if (tid < PT && p < npt_total) {
     const int64_t e = p / m.npts;
     const int q = (int)(p % m.npts);
     // the float law writes its tangent outputs as floats into the same buffer
     T *outd = reinterpret_cast<T *>(preD) + e * 900 * m.npts + q;
-    gradelast_point<TR ? 4 : 1, RES, TAN, T>(S.sm + tid, S.sd + tid, LT_NT, L.par, S.wt[tid],
+    gradelast_point<TR ? 4 : 1, RES, TAN, T>(S.sm + tid, S.sd + tid, PT, L.par, S.wt[tid],
                                              preR + e * 30 * m.npts + q, outd, m.npts);
   }
 }
@@ -788,6 +814,22 @@ static int run_law_points(Context *c, const DevLaw &L)
 {
   const DevMesh m = c->devmesh();
   if (m.geo) {
+    const int64_t npt = c->nelem_total * m.npts;
+    if constexpr (sizeof(T) == 8 && !PRE)
+      if (npt < 2 * 152 * LT_NT) {  // fewer than two blocks of 128 points an SM
+        const size_t smem = sizeof(LawThreadSmem<T, PRE, LT_SMALL_PT, LT_SMALL_NT>);
+        auto kern = law_thread_kernel<LAWK, RES, TAN, T, PRE, LT_SMALL_PT, LT_SMALL_NT>;
+        static bool attr_set = false;
+        if (!attr_set) {
+          IGAP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+          attr_set = true;
+        }
+        kern<<<(unsigned)((npt + LT_SMALL_PT - 1) / LT_SMALL_PT), LT_SMALL_NT, smem, c->stream>>>(
+            m, L, c->d_Uhist, c->d_preR, c->d_preD, npt, c->d_lin);
+        count_launch();
+        IGAP_CHECK_LAUNCH();
+        return IGAPGPU_OK;
+      }
     const size_t smem = sizeof(LawThreadSmem<T, PRE>);
     auto kern = law_thread_kernel<LAWK, RES, TAN, T, PRE>;
     static bool attr_set = false;
@@ -795,7 +837,6 @@ static int run_law_points(Context *c, const DevLaw &L)
       IGAP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       attr_set = true;
     }
-    const int64_t npt = c->nelem_total * m.npts;
     const int64_t nblk = (npt + LT_NT - 1) / LT_NT;
     kern<<<(unsigned)nblk, LT_NT, smem, c->stream>>>(m, L, c->d_Uhist, c->d_preR, c->d_preD, npt, c->d_lin);
     count_launch();
@@ -898,6 +939,71 @@ int launch_law_points(Context *c, bool do_res, bool do_tan, DevLaw &L)
   return IGAPGPU_OK;
 }
 
+// ------------------------------------- projection of precomputed laws
+// R_bd = sum_q sum_k R_q[b,k] rr_q[d,k] (src/assmcore_iga.c:240-258) from the
+// law outputs of every point: lane = basis function, a warp per point, the
+// warps' sums joined in a fixed order.  FP64-pipe bound (46,656 FMA an
+// element).  `parts` blocks an element while the elements leave SMs idle
+// (40 -> 9 us for the 16 elements of a 4x2x2 mesh).
+constexpr int RP_NT = 256;
+
+__global__ void __launch_bounds__(RP_NT) res_project_kernel(DevMesh m, const double *__restrict__ preR, int parts,
+                                                            double *__restrict__ rbuf)
+{
+  __shared__ double red[RP_NT / 32][NE];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t e = blockIdx.x / parts;
+  const int part = (int)(blockIdx.x % parts);
+  double acc[3] = {0.0, 0.0, 0.0};
+  for (int q = part * (RP_NT / 32) + warp; q < m.npts; q += parts * (RP_NT / 32)) {
+    const double2 *r = reinterpret_cast<const double2 *>(m.geo + (e * m.npts + q) * GEO_STRIDE + NDD * (lane < NB ? lane : 0));
+    double rv[NDD];
+#pragma unroll
+    for (int k = 0; k < NDD / 2; k++) {
+      const double2 v = __ldg(r + k);
+      rv[2 * k] = v.x;
+      rv[2 * k + 1] = v.y;
+    }
+    // the point's outputs a lane each, then through shuffles
+    const double mine = lane < 30 ? __ldg(preR + (e * 30 + lane) * m.npts + q) : 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+#pragma unroll
+      for (int k = 0; k < NDD; k++) acc[d] = fma(rv[k], __shfl_sync(0xffffffffu, mine, NDD * d + k), acc[d]);
+  }
+  if (lane < NB)
+#pragma unroll
+    for (int d = 0; d < 3; d++) red[warp][3 * lane + d] = acc[d];
+  __syncthreads();
+  if (threadIdx.x < NE) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < RP_NT / 32; w++) s += red[w][threadIdx.x];
+    rbuf[blockIdx.x * (int64_t)NE + threadIdx.x] = s;
+  }
+}
+
+static int launch_res_project(Context *c, const DevLaw &L, double *RR)
+{
+  const int parts = res_parts(c->nelem_total);
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  if (c->prof) {
+    IGAP_CUDA(cudaEventCreate(&e0));
+    IGAP_CUDA(cudaEventCreate(&e1));
+    IGAP_CUDA(cudaEventRecord(e0, c->stream));
+  }
+  res_project_kernel<<<(unsigned)(c->nelem_total * parts), RP_NT, 0, c->stream>>>(c->devmesh(), L.preR, parts, c->d_rbuf);
+  count_launch();
+  IGAP_CHECK_LAUNCH();
+  if (c->prof) {
+    IGAP_CUDA(cudaEventRecord(e1, c->stream));
+    c->prof_ev[0].emplace_back(e0, e1);
+    c->prof_launches[0]++;
+    c->prof_elements[0] += c->nelem_total;
+  }
+  return launch_residual_gather(c, RR, parts);
+}
+
 // Residual and/or tangent of the FP64 element kernel: through the element
 // buffers in one launch and a gather, else (no room for them) colour by colour.
 template <int LAWK, bool RES, bool TAN>
@@ -950,11 +1056,13 @@ static int run_elements(Context *c, const DevLaw &L, double *RR, double *vals)
     c->prof_ev[0].emplace_back(e0, e1);
   }
   if (buffered) {
-    int r = RES ? launch_residual_gather(c, RR) : IGAPGPU_OK;
+    int r = RES ? launch_residual_gather(c, RR, 1) : IGAPGPU_OK;
     if (!r && TAN) r = launch_tangent_gather(c, vals);
     return r;
   }
-  return IGAPGPU_OK;
+  int r = RES ? launch_dirichlet_residual(c, RR) : IGAPGPU_OK;
+  if (!r && TAN) r = launch_dirichlet_matrix(c, vals);
+  return r;
 }
 
 static bool pairs_ready = false;
@@ -1059,13 +1167,15 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
   if (df_res) {
     IGAP_CUDA(cudaMemcpyAsync(RR, c->d_Fneu, sizeof(double) * c->ndof, cudaMemcpyDeviceToDevice, c->stream));
     rc = law_df ? launch_res_law_df(c, c->d_preR, RR) : launch_res_df(c, RR);
-    if (rc) return rc;
+    if (rc || (rc = launch_dirichlet_residual(c, RR))) return rc;
   }
   // the linear law's FP64 tangent and residual on the tensor cores where its
   // slices are built
   const bool x_tan = fp64_tan && ensure_exact(c);
   const bool x_res = do_res && !df_res && ensure_exact(c);
-  const bool k_res = do_res && !df_res && !x_res, k_tan = fp64_tan && !x_tan;
+  // the reference laws' residual from precomputed law outputs
+  const bool p_res = do_res && !df_res && c->law != IGAPGPU_LAW_LINGRAD && L.preR && c->d_geo && ensure_rbuf(c);
+  const bool k_res = do_res && !df_res && !x_res && !p_res, k_tan = fp64_tan && !x_tan;
   if (k_res || k_tan) {
     const bool do_res_k = k_res, do_tan_k = k_tan;
     {
@@ -1081,6 +1191,7 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
   }
 #undef IGAP_DISPATCH
   if (rc) return rc;
+  if (p_res && (rc = launch_res_project(c, L, RR))) return rc;
   if ((x_tan || x_res) && (rc = launch_exact(c, x_res ? RR : nullptr, x_tan ? vals : nullptr))) return rc;
   if (do_tan && !fp64_tan) {
     const bool gathered = !oz_tan && tc_law_applies(c, L);  // every slot is written
@@ -1088,6 +1199,7 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
     IGAP_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     rc = oz_tan ? launch_tc_ozaki(c, vals) : gathered ? launch_tc_law(c, vals, L) : launch_tc_tangent(c, vals, L);
     if (rc) return rc;
+    if (!gathered && (rc = launch_dirichlet_matrix(c, vals))) return rc;
     if (!c->capturing) {  // a graph replay checks the error word itself
       int herr = 0;
       IGAP_CUDA(cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1097,14 +1209,6 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
         return IGAPGPU_ERR_TIMEOUT;
       }
     }
-  }
-  if (do_res) {
-    rc = launch_dirichlet_residual(c, RR);
-    if (rc) return rc;
-  }
-  if (do_tan) {
-    rc = launch_dirichlet_matrix(c, vals);
-    if (rc) return rc;
   }
   return IGAPGPU_OK;
 }

@@ -329,8 +329,8 @@ int launch_batch_assembly(Context *c, bool do_res, bool do_tan, double *RR, doub
   if (do_tan && !x_tan) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
   int r = batch_kernels(c, do_res, do_tan, RR, vals, b->nitems);
   if (r) return r;
-  if (do_res && (r = launch_dirichlet_residual(c, RR))) return r;
-  if (do_tan && (r = launch_dirichlet_matrix_batch(c, b->d_dir_inst, b->d_nbs, b->d_off, vals))) return r;
+  if (do_res && !x_res && (r = launch_dirichlet_residual(c, RR))) return r;
+  if (do_tan && !x_tan && (r = launch_dirichlet_matrix_batch(c, b->d_dir_inst, b->d_nbs, b->d_off, vals))) return r;
   return IGAPGPU_OK;
 }
 
@@ -595,6 +595,7 @@ int igapgpu_batch_init(igapgpu_t *out, int ninst, const igapgpu_mesh_desc *meshe
     BCUDA(cudaMemcpy(c->d_dir_rows, dir_rows.data(), sizeof(int64_t) * c->n_dir, cudaMemcpyHostToDevice));
     BCUDA(cudaMemcpy(c->d_dir_g, dir_g.data(), sizeof(double) * c->n_dir, cudaMemcpyHostToDevice));
     BCUDA(cudaMemcpy(b->d_dir_inst, dir_inst.data(), sizeof(int) * c->n_dir, cudaMemcpyHostToDevice));
+    BTRY(build_dirmap(c));
   }
   // per-instance descriptors
   {

@@ -186,6 +186,7 @@ struct Context {
   int64_t n_dir = 0;           // Dirichlet rows (unique, last writer wins)
   int64_t *d_dir_rows = nullptr;
   double *d_dir_g = nullptr;
+  int *d_dirmap = nullptr;     // [ndof] index + 1 in d_dir_rows, 0: free (null without Dirichlet rows)
   double *d_stage_a = nullptr, *d_stage_b = nullptr; // host-pointer staging [ndof]
   double *d_stage_v = nullptr;                       // host-pointer staging [nnz] (lazy)
   bool matrix_valid = false;
@@ -288,6 +289,7 @@ int launch_dirichlet_residual(Context *c, double *RR);
 int launch_impose_dirichlet(Context *c, double *U);
 int launch_pattern_cols(Context *c);
 int launch_pattern_cols_at(Context *c, const int64_t *rowptr, int32_t *cols, int64_t coff);
+int build_dirmap(Context *c);
 int launch_dirichlet_matrix_batch(Context *c, const int *d_inst, const int *d_nbs, const int64_t *d_off,
                                   double *vals);
 int launch_geometry_cache(Context *c);

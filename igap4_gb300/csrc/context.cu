@@ -181,7 +181,7 @@ static int free_ctx(Context *c)
   cycle_release(c);
   batch_release(c);
   void *bufs[] = {c->d_wq, c->d_xq, c->d_w, c->d_X, c->d_Uhist, c->d_RR, c->d_vals,
-                  c->d_rowptr, c->d_cols, c->d_Dconst, c->d_Fneu, c->d_dir_rows, c->d_dir_g,
+                  c->d_rowptr, c->d_cols, c->d_Dconst, c->d_Fneu, c->d_dir_rows, c->d_dir_g, c->d_dirmap,
                   c->d_stage_a, c->d_stage_b, c->d_stage_v, c->d_V, c->d_Z, c->d_work,
                   c->d_diag, c->d_bdiag, c->d_cinv, c->d_asmz, c->d_red, c->d_partial, c->d_err, c->d_geo, c->d_geof, c->d_gop, c->d_oz, c->d_ozexp, c->d_rpc, c->d_rel, c->d_upair, c->d_lin, c->d_preR, c->d_preD, c->d_ebuf, c->d_fbuf, c->d_rbuf, c->d_xops, c->d_xexp, c->d_xrow, c->d_dens, c->d_dsparse, c->d_dval, c->d_sval, c->d_bct, c->d_neu};
   for (void *b : bufs)
@@ -418,6 +418,7 @@ static int init_impl(Context *c, const igapgpu_mesh_desc *mesh)
       if ((r = dev_alloc(&c->d_dir_g, c->n_dir))) return r;
       IGAP_CUDA(cudaMemcpy(c->d_dir_rows, order.data(), sizeof(int64_t) * c->n_dir, cudaMemcpyHostToDevice));
       IGAP_CUDA(cudaMemcpy(c->d_dir_g, gv.data(), sizeof(double) * c->n_dir, cudaMemcpyHostToDevice));
+      if (!c->sub && (r = build_dirmap(c))) return r;
     }
   }
   IGAP_CUDA(cudaStreamSynchronize(c->stream));

@@ -44,7 +44,7 @@ __device__ __forceinline__ int by_residue(Range r, int e)
 
 // A control point's place in its lattice and the elements around it.
 struct Patch {
-  int ix, iy, iz, lox, loy, loz, cy, cz, nj;
+  int ix, iy, iz, lox, loy, loz, cy, cz, nj, nb1, nb2;
   int ne0, ne1, ne2;
 };
 
@@ -52,6 +52,8 @@ __device__ __forceinline__ Patch patch_of(const DevMesh &m, int64_t cpl)
 {
   Patch p;
   const int nb1 = m.nbasis[1], nb2 = m.nbasis[2];
+  p.nb1 = nb1;
+  p.nb2 = nb2;
   p.ne0 = m.nelem[0];
   p.ne1 = m.nelem[1];
   p.ne2 = m.nelem[2];
@@ -75,13 +77,15 @@ struct GatherTab {
   int tab[TG_NJ * 27];
   int64_t ebase[27];             // -1: outside the lattice
   unsigned char cnt[TG_NJ];      // contributions of a column
+  unsigned char fix[TG_NJ];      // its Dirichlet components (bit e)
   // per direction and (a, c): rank among the shared elements, column offset,
   // number of shared elements
   unsigned char rank[3][9], off[3][9], n[3][9];
 };
 
 template <typename F>
-__device__ __forceinline__ void gather_table(GatherTab &G, const Patch &p, int64_t e0, int64_t per_element, F entry)
+__device__ __forceinline__ void gather_table(GatherTab &G, const Patch &p, int64_t e0, int64_t per_element,
+                                             const int *dir, F entry)
 {
   if (threadIdx.x < 27) {
     const int t = threadIdx.x;
@@ -96,6 +100,15 @@ __device__ __forceinline__ void gather_table(GatherTab &G, const Patch &p, int64
     G.rank[dir][3 * a + c] = (unsigned char)by_residue(r, i - a);
     G.n[dir][3 * a + c] = (unsigned char)max(r.n, 0);
     G.off[dir][3 * a + c] = (unsigned char)(i - a + c - lo);
+  }
+  for (int j = threadIdx.x; j < p.nj; j += TG_THREADS) {
+    unsigned f = 0;
+    if (dir) {
+      const int jz = p.loz + j % p.cz, jy = p.loy + (j / p.cz) % p.cy, jx = p.lox + j / (p.cz * p.cy);
+      const int *d = dir + 3 * (((int64_t)jx * p.nb1 + jy) * p.nb2 + jz);
+      for (int e = 0; e < 3; e++) f |= (__ldg(d + e) ? 1u : 0u) << e;
+    }
+    G.fix[j] = (unsigned char)f;
   }
   __syncthreads();
   for (int t = threadIdx.x; t < 27 * NB; t += TG_THREADS) {
@@ -121,11 +134,12 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a,
   const int inst = a.cpinst ? __ldg(a.cpinst + cp) : 0;
   const DevMesh &m = a.meshes ? a.meshes[inst] : a.m;
   const Patch p = patch_of(m, cp - m.dof_off / 3);
-  gather_table(G, p, a.eoff ? __ldg(a.eoff + inst) : 0, EBUF, [](int b, int c) {  // block offset, bit 15: transposed
+  gather_table(G, p, a.eoff ? __ldg(a.eoff + inst) : 0, EBUF, a.dir ? a.dir + m.dof_off : nullptr, [](int b, int c) {  // block offset, bit 15: transposed
     return 9 * pair_index(min(b, c), max(b, c)) | (b > c ? 0x8000 : 0);
   });
   const int64_t r0 = __ldg(a.rowptr + 3 * cp);
   const bool failed = a.err && *a.err;
+  const int self = ((p.ix - p.lox) * p.cy + p.iy - p.loy) * p.cz + p.iz - p.loz, rfix = G.fix[self];
   for (int t = threadIdx.x; t < 9 * p.nj; t += TG_THREADS) {
     const int j = t / 9, q = t - 9 * j, d = q / 3, e = q - 3 * d;
     const int n = G.cnt[j], qt = 3 * e + d;
@@ -136,6 +150,7 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a,
       const int v = tab[k];
       s += __ldg(ebuf + G.ebase[v >> 16] + (v & 0x7fff) + ((v & 0x8000) ? qt : q));
     }
+    if ((rfix >> d | G.fix[j] >> e) & 1) s = j == self && d == e ? 1.0 : 0.0;
     vals[r0 + (int64_t)d * 3 * p.nj + 3 * j + e] = failed ? __longlong_as_double(0x7ff8000000000000ll) : s;
   }
 }
@@ -149,9 +164,10 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_f32_kernel(GatherMa
   __shared__ GatherTab G;
   const int64_t cp = blockIdx.x;
   const Patch p = patch_of(a.m, cp);
-  gather_table(G, p, 0, NB * 243, [](int b, int c) { return 243 * b + 3 * c; });
+  gather_table(G, p, 0, NB * 243, a.dir, [](int b, int c) { return 243 * b + 3 * c; });
   const int64_t r0 = __ldg(a.rowptr + 3 * cp);
   const int row = 3 * p.nj;
+  const int self = ((p.ix - p.lox) * p.cy + p.iy - p.loy) * p.cz + p.iz - p.loz, rfix = G.fix[self];
   for (int t = threadIdx.x; t < 3 * row; t += TG_THREADS) {
     const int d = t / row, x = t - d * row, j = x / 3, e = x - 3 * j;
     const int n = G.cnt[j];
@@ -162,11 +178,13 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_f32_kernel(GatherMa
       const int v = tab[k];
       s += f32_to_f64(__ldg(fbuf + G.ebase[v >> 16] + (v & 0xffff) + 81 * d + e));  // widened on the integer pipe
     }
+    if ((rfix >> d | G.fix[j] >> e) & 1) s = j == self && d == e ? 1.0 : 0.0;
     vals[r0 + t] = s;
   }
 }
 
-// RR = load + the element sums of every element that holds the control point.
+// RR = load + the element sums of every element that holds the control point;
+// U - g on the Dirichlet rows.
 __global__ void __launch_bounds__(256) residual_gather_kernel(GatherMap a, const double *__restrict__ rbuf,
                                                               const double *__restrict__ load, double *__restrict__ RR)
 {
@@ -180,6 +198,11 @@ __global__ void __launch_bounds__(256) residual_gather_kernel(GatherMap a, const
   const int64_t cpl = cp - m.dof_off / 3;
   const int nb1 = m.nbasis[1], nb2 = m.nbasis[2];
   const int i[3] = {(int)(cpl / ((int64_t)nb1 * nb2)), (int)((cpl / nb2) % nb1), (int)(cpl % nb2)};
+  const int fix = a.dir ? __ldg(a.dir + dof) : 0;
+  if (fix) {
+    RR[dof] = a.U[dof] - __ldg(a.dir_g + fix - 1);
+    return;
+  }
   double s = load[dof];
 #pragma unroll
   for (int r = 0; r < 27; r++) {
@@ -195,7 +218,8 @@ __global__ void __launch_bounds__(256) residual_gather_kernel(GatherMap a, const
       el = el * m.nelem[k] + e;
       b = b * 3 + i[k] - e;
     }
-    if (in) s += __ldg(rbuf + (e0 + el) * NE + 3 * b + d);
+    if (in)
+      for (int k = 0; k < a.parts; k++) s += __ldg(rbuf + ((e0 + el) * a.parts + k) * NE + 3 * b + d);
   }
   RR[dof] = a.err && *a.err ? __longlong_as_double(0x7ff8000000000000ll) : s;
 }
@@ -210,6 +234,10 @@ static GatherMap gather_map(Context *c)
   a.eoff = nullptr;
   a.cpinst = nullptr;
   a.err = nullptr;
+  a.dir = c->d_dirmap;
+  a.dir_g = c->d_dir_g;
+  a.U = c->d_Uhist;
+  a.parts = 1;
   if (c->batch) batch_gather_map(c, &a);
   return a;
 }
@@ -232,9 +260,10 @@ int launch_tangent_gather_f32(Context *c, double *vals)
   return IGAPGPU_OK;
 }
 
-int launch_residual_gather(Context *c, double *RR, const int *err)
+int launch_residual_gather(Context *c, double *RR, int parts, const int *err)
 {
   GatherMap a = gather_map(c);
+  a.parts = parts;
   a.err = err;
   residual_gather_kernel<<<(unsigned)((c->ndof + 255) / 256), 256, 0, c->stream>>>(a, c->d_rbuf, c->d_Fneu,
                                                                                   RR);
@@ -265,6 +294,6 @@ static bool ensure_buffer(Context *c, T **p, int *state, size_t per_element)
 
 bool ensure_ebuf(Context *c) { return ensure_buffer(c, &c->d_ebuf, &c->ebuf_state, EBUF); }
 bool ensure_fbuf(Context *c) { return ensure_buffer(c, &c->d_fbuf, &c->fbuf_state, NB * 243); }
-bool ensure_rbuf(Context *c) { return ensure_buffer(c, &c->d_rbuf, &c->rbuf_state, NE); }
+bool ensure_rbuf(Context *c) { return ensure_buffer(c, &c->d_rbuf, &c->rbuf_state, NE * (size_t)res_parts(c->nelem_total)); }
 
 }  // namespace igap

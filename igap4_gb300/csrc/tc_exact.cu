@@ -663,7 +663,7 @@ int launch_exact(Context *c, double *RR, double *vals)
     c->prof_elements[0] += c->nelem_total;
   }
   c->exact_ran = true;
-  const int r = RR ? launch_residual_gather(c, RR, c->d_err) : IGAPGPU_OK;
+  const int r = RR ? launch_residual_gather(c, RR, 1, c->d_err) : IGAPGPU_OK;
   return r || !vals ? r : launch_tangent_gather(c, vals, c->d_err);
 }
 
