@@ -1175,7 +1175,9 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
   const bool x_res = do_res && !df_res && ensure_exact(c);
   // the reference laws' residual from precomputed law outputs
   const bool p_res = do_res && !df_res && c->law != IGAPGPU_LAW_LINGRAD && L.preR && c->d_geo && ensure_rbuf(c);
-  const bool k_res = do_res && !df_res && !x_res && !p_res, k_tan = fp64_tan && !x_tan;
+  // and their FP64 tangent by sum factorisation
+  const bool s_tan = fp64_tan && c->law != IGAPGPU_LAW_LINGRAD && ensure_sumfac(c, L);
+  const bool k_res = do_res && !df_res && !x_res && !p_res, k_tan = fp64_tan && !x_tan && !s_tan;
   if (k_res || k_tan) {
     const bool do_res_k = k_res, do_tan_k = k_tan;
     {
@@ -1192,6 +1194,7 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
 #undef IGAP_DISPATCH
   if (rc) return rc;
   if (p_res && (rc = launch_res_project(c, L, RR))) return rc;
+  if (s_tan && (rc = launch_sumfac(c, L, vals))) return rc;
   if ((x_tan || x_res) && (rc = launch_exact(c, x_res ? RR : nullptr, x_tan ? vals : nullptr))) return rc;
   if (do_tan && !fp64_tan) {
     const bool gathered = !oz_tan && tc_law_applies(c, L);  // every slot is written

@@ -173,6 +173,8 @@ struct Context {
   double *d_rbuf = nullptr;    // element residuals [element][NE]
   float *d_fbuf = nullptr;     // FP32 element matrices [element][27][243] (split tangent of the reference's laws)
   int ebuf_state = -1, rbuf_state = -1, fbuf_state = -1;  // -1 not decided, 0 off, 1 on
+  double *d_sft = nullptr;     // parametric-to-physical derivative maps [element][73][64] (sumfac.cu)
+  int sf_state = -1;           // -1 not decided, 0 off, 1 on
   void *d_xops = nullptr;      // linear law: 9-bit slices of the Gram operands (FP64 tensor-core tangent)
   short *d_xexp = nullptr;     // their row exponents
   double *d_xrow = nullptr;    // row 80 of every element's operand
@@ -313,6 +315,9 @@ int launch_assembly_p3(Context *c, bool do_res, bool do_tan, double *RR, double 
 // tc_ozaki.cu (linear law, BF16 slices, FP64-quality)
 int ensure_ozaki_operands(Context *c);
 int launch_tc_ozaki(Context *c, double *vals);
+// sumfac.cu (the reference's laws' FP64 tangent by sum factorisation)
+bool ensure_sumfac(Context *c, const DevLaw &L);
+int launch_sumfac(Context *c, const DevLaw &L, double *vals);
 // tc_exact.cu (linear law, FP64 tangent and residual from exact BF16 slices)
 bool ensure_exact(Context *c);
 int launch_exact(Context *c, double *RR, double *vals);

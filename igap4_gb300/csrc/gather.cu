@@ -20,7 +20,7 @@
 namespace igap {
 
 namespace {
-constexpr int TG_THREADS = 128;
+constexpr int TG_THREADS = 256;
 constexpr int TG_NJ = 125;  // control points in a row's stencil
 
 // Elements of one direction that hold both control points i and j, by
@@ -184,12 +184,16 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_f32_kernel(GatherMa
 }
 
 // RR = load + the element sums of every element that holds the control point;
-// U - g on the Dirichlet rows.
+// U - g on the Dirichlet rows.  WARP: a warp per DOF, its lanes an element
+// each (small meshes, where 27 loads one after the other are the time); else a
+// thread per DOF.  The additions run in colour order either way.
+template <bool WARP>
 __global__ void __launch_bounds__(256) residual_gather_kernel(GatherMap a, const double *__restrict__ rbuf,
                                                               const double *__restrict__ load, double *__restrict__ RR)
 {
-  const int64_t dof = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (dof >= a.ndof) return;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t dof = WARP ? t >> 5 : t;
+  if (dof >= a.ndof) return;  // whole warps with WARP
   const int64_t cp = dof / 3;
   const int d = (int)(dof % 3);
   const int inst = a.cpinst ? __ldg(a.cpinst + cp) : 0;
@@ -203,9 +207,8 @@ __global__ void __launch_bounds__(256) residual_gather_kernel(GatherMap a, const
     RR[dof] = a.U[dof] - __ldg(a.dir_g + fix - 1);
     return;
   }
-  double s = load[dof];
-#pragma unroll
-  for (int r = 0; r < 27; r++) {
+  // the sum of residue r's element (0 outside the lattice)
+  auto element_sum = [&](int r) {
     const int rr[3] = {r / 9, (r / 3) % 3, r % 3};
     int64_t el = 0;
     int b = 0;
@@ -218,8 +221,24 @@ __global__ void __launch_bounds__(256) residual_gather_kernel(GatherMap a, const
       el = el * m.nelem[k] + e;
       b = b * 3 + i[k] - e;
     }
-    if (in)
-      for (int k = 0; k < a.parts; k++) s += __ldg(rbuf + ((e0 + el) * a.parts + k) * NE + 3 * b + d);
+    double v = 0.0;
+    if (in) {
+      const double *p = rbuf + (e0 + el) * a.parts * NE + 3 * b + d;
+      v = __ldg(p);
+      for (int k = 1; k < a.parts; k++) v += __ldg(p + k * NE);
+    }
+    return v;
+  };
+  double s = load[dof];
+  if constexpr (WARP) {
+    const int lane = threadIdx.x & 31;
+    const double mine = lane < 27 ? element_sum(lane) : 0.0;
+#pragma unroll
+    for (int r = 0; r < 27; r++) s += __shfl_sync(0xffffffffu, mine, r);
+    if (lane) return;
+  } else {
+#pragma unroll
+    for (int r = 0; r < 27; r++) s += element_sum(r);
   }
   RR[dof] = a.err && *a.err ? __longlong_as_double(0x7ff8000000000000ll) : s;
 }
@@ -265,8 +284,10 @@ int launch_residual_gather(Context *c, double *RR, int parts, const int *err)
   GatherMap a = gather_map(c);
   a.parts = parts;
   a.err = err;
-  residual_gather_kernel<<<(unsigned)((c->ndof + 255) / 256), 256, 0, c->stream>>>(a, c->d_rbuf, c->d_Fneu,
-                                                                                  RR);
+  if (c->ndof < 152 * 64 * 2)  // one wave of warps
+    residual_gather_kernel<true><<<(unsigned)((c->ndof + 7) / 8), 256, 0, c->stream>>>(a, c->d_rbuf, c->d_Fneu, RR);
+  else
+    residual_gather_kernel<false><<<(unsigned)((c->ndof + 255) / 256), 256, 0, c->stream>>>(a, c->d_rbuf, c->d_Fneu, RR);
   count_launch();
   IGAP_CHECK_LAUNCH();
   return IGAPGPU_OK;
