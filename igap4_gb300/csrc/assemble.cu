@@ -704,7 +704,7 @@ struct LawThreadSmem {
   T sm[30 * PT];
   T sd[30 * PT];
   double wt[PT];
-  double R[NT / 32][PRE ? 1 : GEO_STRIDE];
+  T R[NT / 32][PRE ? 1 : GEO_STRIDE];  // the point's basis in the law's arithmetic
   double U[NT / 32][F32 || PRE ? 1 : 3 * NE];
   float Uf[NT / 32][F32 && !PRE ? 3 * NE : 1];  // the element's state in FP32 (float law)
 };
@@ -728,6 +728,15 @@ __global__ void __launch_bounds__(NT)
   const int nb1 = m.nbasis[1], nb2 = m.nbasis[2];
   const double rho_m = L.par[5], damp = L.par[6], dt = L.par[7];
   int64_t cur_e = -1;
+  // the next point's basis is on its way while the current one is interpolated
+  constexpr int LD = (GEO_STRIDE + 31) / 32;
+  [[maybe_unused]] double gv[PRE ? 1 : LD];
+  [[maybe_unused]] auto fetch = [&](int64_t p) {
+    const double *g = m.geo + (p < npt_total ? p : npt_total - 1) * GEO_STRIDE;
+#pragma unroll
+    for (int i = 0; i < LD; i++) gv[i] = lane + 32 * i < GEO_STRIDE ? __ldg(g + lane + 32 * i) : 0.0;
+  };
+  if constexpr (!PRE) fetch(p0 + warp * PPW);
   for (int j = 0; j < PPW; j++) {
     const int t = warp * PPW + j;
     const int64_t p = p0 + t;
@@ -754,8 +763,12 @@ __global__ void __launch_bounds__(NT)
         }
         cur_e = e;
       }
-      const double *g = m.geo + p * GEO_STRIDE;
-      for (int i = lane; i < GEO_STRIDE; i += 32) S.R[warp][i] = __ldg(g + i);
+#pragma unroll
+      for (int i = 0; i < LD; i++)
+        if (lane + 32 * i < GEO_STRIDE) S.R[warp][lane + 32 * i] = lawpt::to_t<T>(gv[i]);
+      // the weight (entry NB * NDD) in FP64
+      if (lane == (NB * NDD) % 32) S.wt[t] = gv[(NB * NDD) / 32];
+      if (j + 1 < PPW) fetch(p + 1);
       __syncwarp();
       if (lane < 30) {
         const int d = lane / NDD, k = lane % NDD;
@@ -764,7 +777,7 @@ __global__ void __launch_bounds__(NT)
           float sf[3] = {0.f, 0.f, 0.f};
 #pragma unroll
           for (int b = 0; b < NB; b++) {
-            const float r = f64_to_pair(S.R[warp][NDD * b + k]).x;
+            const float r = S.R[warp][NDD * b + k];
 #pragma unroll
             for (int h = 0; h < 3; h++)
               if (h < nh) sf[h] = fmaf(r, S.Uf[warp][h * NE + 3 * b + d], sf[h]);
@@ -793,7 +806,6 @@ __global__ void __launch_bounds__(NT)
           S.sd[lane * PT + t] = lawpt::to_t<T>(0.5 * (s[0] - s[2]));
         }
       }
-      if (lane == 0) S.wt[t] = S.R[warp][NB * NDD];
       __syncwarp();
     }
   }
