@@ -126,22 +126,37 @@ __device__ __forceinline__ void gather_table(GatherTab &G, const Patch &p, int64
 
 // One block per control point: the table of its slots, then a thread per
 // entry of the 3 x 3 blocks (nine consecutive threads read one 72-byte block).
+// The matrix is symmetric and so are its element blocks: the columns from the
+// diagonal on are summed once and stored in both rows (the FP64 additions and
+// the reads halve).
 __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a, const double *__restrict__ ebuf,
                                                                     double *__restrict__ vals)
 {
   __shared__ GatherTab G;
+  __shared__ int64_t tbase[TG_NJ];  // slot of this control point's column in row 3 j
+  __shared__ int tlen[TG_NJ];       // length of that row
   const int64_t cp = blockIdx.x;
   const int inst = a.cpinst ? __ldg(a.cpinst + cp) : 0;
   const DevMesh &m = a.meshes ? a.meshes[inst] : a.m;
-  const Patch p = patch_of(m, cp - m.dof_off / 3);
+  const int64_t cp0 = m.dof_off / 3;
+  const Patch p = patch_of(m, cp - cp0);
+  const int self = ((p.ix - p.lox) * p.cy + p.iy - p.loy) * p.cz + p.iz - p.loz;
+  for (int j = self + threadIdx.x; j < p.nj; j += TG_THREADS) {
+    const int jz = p.loz + j % p.cz, jy = p.loy + (j / p.cz) % p.cy, jx = p.lox + j / (p.cz * p.cy);
+    const int64_t r = __ldg(a.rowptr + 3 * (cp0 + ((int64_t)jx * p.nb1 + jy) * p.nb2 + jz));
+    const int cx = min(jx + P, m.nbasis[0] - 1) - max(jx - P, 0) + 1, cy = min(jy + P, p.nb1 - 1) - max(jy - P, 0) + 1,
+              cz = min(jz + P, p.nb2 - 1) - max(jz - P, 0) + 1;
+    tbase[j] = r + 3 * (((p.ix - max(jx - P, 0)) * cy + p.iy - max(jy - P, 0)) * cz + p.iz - max(jz - P, 0));
+    tlen[j] = 3 * cx * cy * cz;
+  }
   gather_table(G, p, a.eoff ? __ldg(a.eoff + inst) : 0, EBUF, a.dir ? a.dir + m.dof_off : nullptr, [](int b, int c) {  // block offset, bit 15: transposed
     return 9 * pair_index(min(b, c), max(b, c)) | (b > c ? 0x8000 : 0);
   });
   const int64_t r0 = __ldg(a.rowptr + 3 * cp);
   const bool failed = a.err && *a.err;
-  const int self = ((p.ix - p.lox) * p.cy + p.iy - p.loy) * p.cz + p.iz - p.loz, rfix = G.fix[self];
-  for (int t = threadIdx.x; t < 9 * p.nj; t += TG_THREADS) {
-    const int j = t / 9, q = t - 9 * j, d = q / 3, e = q - 3 * d;
+  const int rfix = G.fix[self];
+  for (int t = threadIdx.x; t < 9 * (p.nj - self); t += TG_THREADS) {
+    const int j = self + t / 9, q = t % 9, d = q / 3, e = q - 3 * d;
     const int n = G.cnt[j], qt = 3 * e + d;
     const int *tab = G.tab + j * 27;
     double s = 0.0;
@@ -151,7 +166,9 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a,
       s += __ldg(ebuf + G.ebase[v >> 16] + (v & 0x7fff) + ((v & 0x8000) ? qt : q));
     }
     if ((rfix >> d | G.fix[j] >> e) & 1) s = j == self && d == e ? 1.0 : 0.0;
-    vals[r0 + (int64_t)d * 3 * p.nj + 3 * j + e] = failed ? __longlong_as_double(0x7ff8000000000000ll) : s;
+    if (failed) s = __longlong_as_double(0x7ff8000000000000ll);
+    vals[r0 + (int64_t)d * 3 * p.nj + 3 * j + e] = s;
+    if (j != self) vals[tbase[j] + (int64_t)e * tlen[j] + d] = s;
   }
 }
 
