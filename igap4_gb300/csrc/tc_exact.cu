@@ -33,8 +33,10 @@
 // displacements of 1e-3 costs the quadrature loop 2e-13).
 // Measured: against 64-bit reference sums the error is the FP64 kernel's (7e-16
 // at 16x4x4, 3e-15 at 63x17x15 distorted, both from the geometry; the two
-// tangents differ by 2e-16). Residual and tangent at 16x4x4 0.74 -> 0.30 ms,
-// 63x17x15 30.1 -> 6.2 ms (the FP64 residual 4.1 ms of it).
+// tangents differ by 2e-16).  Residual and tangent at 16x4x4 7.9 ms (FP64 kernel,
+// colour by colour) -> 79 us, 63x17x15 36.7 -> 2.33 ms, 128x32x32 255.7 ->
+// 18.6 ms; per element and SM 36 k clocks, 27 k of them MMAs (their
+// shared-memory operand reads) and 9 k the accumulators' drain.
 //
 // One persistent CTA per SM over all elements; results go to the element
 // buffers (gather.cu):
@@ -82,6 +84,7 @@ constexpr uint32_t XS_TMEM_COLS = 512;
 constexpr uint32_t XS_ACC2 = 0, XS_ACC4 = 80, XS_ACC6 = 160, XS_ACC78 = 240, XS_X3 = 320, XS_X5 = 416;
 constexpr uint32_t XS_WAIT_LIMIT = 1u << 26;
 constexpr int XO_THREADS = 512;                  // operand kernel
+constexpr int XO_LD = (NB * 9 + 31) / 32;        // its loads per lane and point
 static_assert(XS_STAGE % 16 == 0 && XS_CH_BYTES % 16 == 0, "bulk copies and descriptors need 16-byte alignment");
 static_assert(EBUF * sizeof(double) % 16 == 0, "bulk stores move multiples of 16 bytes");
 
@@ -159,6 +162,10 @@ __device__ __forceinline__ double scaled(long long v, int k)
 
 // Slices of every element, once per context (state independent).  One CTA per
 // element: S in shared memory (row stride K + 1), row exponents, digits.
+// Integer operations and the loads' latency bound it: the digits as bit fields of
+// a biased sum with one exact FMA each, and the next point's loads in flight,
+// take the first assembly at 63x17x15 from 7.2 to 5.3 ms (76 k -> 41 k clocks
+// an element here).
 __global__ void __launch_bounds__(XO_THREADS) exact_operand_kernel(const double *__restrict__ geo, int npts, int nchunk,
                                                                    int64_t nelem, double ell,
                                                                    unsigned char *__restrict__ ops,
@@ -172,6 +179,15 @@ __global__ void __launch_bounds__(XO_THREADS) exact_operand_kernel(const double 
   __shared__ int nrm[XS_EXP][4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int K = nchunk * 32, ld = K + 1;
+  // this lane's values of a point (0: none): place in the cache, second
+  // derivative, its two indices (gradient: index), row 3 b
+  int off[XO_LD];
+#pragma unroll
+  for (int i = 0; i < XO_LD; i++) {
+    const int u = lane + 32 * i, b = u / 9, s = u % 9, h = s - 3;  // h: xx, xy, xz, yy, yz, zz
+    const int i0 = s < 3 ? s : (h < 3 ? 0 : (h < 5 ? 1 : 2)), m0 = s < 3 ? 0 : (h < 3 ? h : (h < 5 ? h - 2 : 2));
+    off[i] = u < NB * 9 ? (NDD * b + 1 + s) | (s >= 3) << 10 | i0 << 11 | m0 << 13 | 3 * b << 15 : 0;
+  }
   for (int64_t e = blockIdx.x; e < nelem; e += gridDim.x) {
     for (int q = tid; q < nchunk * PW; q += XO_THREADS) {
       double w = q < npts ? geo[(e * npts + q) * GEO_STRIDE + NB * NDD] : 0.0;
@@ -184,19 +200,35 @@ __global__ void __launch_bounds__(XO_THREADS) exact_operand_kernel(const double 
     }
     for (int i = tid; i < XS_EXP * 4; i += XO_THREADS) nrm[i / 4][i % 4] = 0;
     __syncthreads();
-    // column of point q: 32 (q / 8) + q % 8 for the gradient, + 8 + 3 (q % 8) + m for the Hessian row's entry m
-    for (int i = tid; i < nchunk * PW * NB * 9; i += XO_THREADS) {
-      const int s = i % 9, b = (i / 9) % NB, q = i / (9 * NB);
-      const int c0 = 32 * (q / PW), p = q % PW;
-      const double v = q < npts ? __ldg(geo + (e * npts + q) * GEO_STRIDE + NDD * b + 1 + s) : 0.0;
-      if (s < 3) {
-        S[(3 * b + s) * ld + c0 + p] = sw[q] * v;
-      } else {
-        const int h = s - 3;  // xx, xy, xz, yy, yz, zz
-        const int i0 = h < 3 ? 0 : (h < 5 ? 1 : 2), m0 = h < 3 ? h : (h < 5 ? h - 2 : 2);
-        const double x = swl[q] * v;
-        S[(3 * b + i0) * ld + c0 + PW + 3 * p + m0] = x;
-        if (i0 != m0) S[(3 * b + m0) * ld + c0 + PW + 3 * p + i0] = x;
+    // column of point q: 32 (q / 8) + q % 8 for the gradient, + 8 + 3 (q % 8) + m for the Hessian row's entry m;
+    // a warp per point, the next point's loads in flight
+    {
+      double v[XO_LD];
+      auto fetch = [&](int q) {
+        const double *g = geo + (e * npts + q) * GEO_STRIDE;
+#pragma unroll
+        for (int i = 0; i < XO_LD; i++) v[i] = q < npts && off[i] ? __ldg(g + (off[i] & 0x3ff)) : 0.0;
+      };
+      fetch(warp);
+      for (int q = warp; q < nchunk * PW; q += XO_THREADS / 32) {
+        double x[XO_LD];
+        const double wq = sw[q], wl = swl[q];
+#pragma unroll
+        for (int i = 0; i < XO_LD; i++) x[i] = v[i] * ((off[i] >> 10) & 1 ? wl : wq);
+        if (q + XO_THREADS / 32 < nchunk * PW) fetch(q + XO_THREADS / 32);
+        const int c0 = 32 * (q / PW), p = q % PW;
+#pragma unroll
+        for (int i = 0; i < XO_LD; i++) {
+          if (!off[i]) continue;
+          double *row = S + (off[i] >> 15) * ld + c0;  // row 3 b
+          const int i0 = (off[i] >> 11) & 3, m0 = (off[i] >> 13) & 3;
+          if (!((off[i] >> 10) & 1)) {
+            row[i0 * ld + p] = x[i];
+          } else {
+            row[i0 * ld + PW + 3 * p + m0] = x[i];
+            if (i0 != m0) row[m0 * ld + PW + 3 * p + i0] = x[i];
+          }
+        }
       }
     }
     __syncthreads();
@@ -239,38 +271,49 @@ __global__ void __launch_bounds__(XO_THREADS) exact_operand_kernel(const double 
         for (int i = 0; i < 4; i++) out[j][i] = 0u;
       if (r < XS_ROWS) {
         const int E = rexp[r];
-        int s2[4] = {0, 0, 0, 0};
+        float s2[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const double v = S[r * ld + kq * 8 + i];
-          const int hw = __double2hiint(v);
-          const int ef = (hw >> 20) & 0x7ff;
-          long long X = 0;
-          if (ef) {
-            // v = m 2^(ef - 1075); x = v 2^(8 - E), 45 fraction bits: m shifted right by E + 1022 - ef >= 0
-            const long long mt = ((long long)((hw & 0xfffff) | 0x100000) << 32) | (uint32_t)__double2loint(v);
-            const int n = E + 1022 - ef;
-            X = n == 0 ? mt : (n < 55 ? (mt + (1ll << (n - 1))) >> n : 0);
-            if (hw < 0) X = -X;
-          }
-          int d[XS_NSL];
+        for (int i = 0; i < 8; i += 2) {
+          float f[2][XS_NSL];
 #pragma unroll
-          for (int j = XS_NSL - 1; j > 0; j--) {
-            d[j] = ((int)(X + 256) & 511) - 256;
-            X = (X - d[j]) >> 9;
-          }
-          d[0] = (int)X;
-          float f = 1.f;
+          for (int u = 0; u < 2; u++) {
+            const double v = S[r * ld + kq * 8 + i + u];
+            const int hw = __double2hiint(v);
+            const int ef = (hw >> 20) & 0x7ff;
+            long long X = 0;
+            if (ef) {
+              // v = m 2^(ef - 1075); x = v 2^(8 - E), 45 fraction bits: m shifted right by E + 1022 - ef >= 0
+              const long long mt = ((long long)((hw & 0xfffff) | 0x100000) << 32) | (uint32_t)__double2loint(v);
+              const int n = E + 1022 - ef;
+              X = n == 0 ? mt : (n < 55 ? (mt + (1ll << (n - 1))) >> n : 0);
+              if (hw < 0) X = -X;
+            }
+            // balanced digits: with 256 added at every digit's place they are the
+            // 9-bit fields less 256.  2^23 + field is a float by its bits, and one
+            // exact FMA takes off the bias and scales.
+            const long long Y = X + 0x1008040201ll * 256;
+            const int top = (int)(Y >> 45);  // D1 itself, -256 .. 256
+            f[u][0] = __uint_as_float(0x4b000000u | (uint32_t)(top + 256)) - 8388864.f;
+            float sc = 1.f / 512.f;
 #pragma unroll
-          for (int j = 0; j < XS_NSL; j++) {
-            if (j < 4) s2[j] += d[j] * d[j];
-            const uint32_t h = __float_as_uint((float)d[j] * f) >> 16;  // exact: at most 8 significant bits
-            out[j][i / 2] |= h << (16 * (i & 1));
-            f *= 1.f / 512.f;
+            for (int j = 1; j < XS_NSL; j++) {
+              const uint32_t d = (uint32_t)(Y >> (9 * (XS_NSL - 1 - j))) & 511u;
+              f[u][j] = __fmaf_rn(__uint_as_float(0x4b000000u | d), sc, -8388864.f * sc);
+              sc *= 1.f / 512.f;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) s2[j] = fmaf(f[u][j], f[u][j], s2[j]);  // exact: below 2^20 units
           }
+#pragma unroll
+          for (int j = 0; j < XS_NSL; j++)  // exact in BF16: at most 8 significant bits
+            out[j][i / 2] = __byte_perm(__float_as_uint(f[0][j]), __float_as_uint(f[1][j]), 0x7632);
         }
+        float un = 1.f;
 #pragma unroll
-        for (int j = 0; j < 4; j++) atomicAdd(&nrm[r][j], s2[j]);
+        for (int j = 0; j < 4; j++) {
+          atomicAdd(&nrm[r][j], (int)(s2[j] * un));
+          un *= 262144.f;
+        }
       }
       unsigned char *o = oe + (size_t)(kq / 4) * XS_CH_BYTES + ((kq / 2) % 2) * XS_KS_BYTES + (r / 8) * 256 +
                          (kq % 2) * 128 + (r % 8) * 16;
@@ -282,12 +325,15 @@ __global__ void __launch_bounds__(XO_THREADS) exact_operand_kernel(const double 
     for (int k = tid; k < K; k += XO_THREADS) row80[e * K + k] = S[80 * ld + k];
     __syncthreads();
     // partial sums of acc4 and X5 below 2^24 units
-    if (tid == 0) {
+    if (warp == 0) {
       float n[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int r = 0; r < XS_ROWS; r++)
+      for (int r = lane; r < XS_ROWS; r += 32)
         for (int j = 0; j < 4; j++) n[j] = fmaxf(n[j], (float)nrm[r][j]);
-      for (int j = 0; j < 4; j++) n[j] = sqrtf(n[j]);
-      if (2.f * n[0] * n[2] + n[1] * n[1] > 1.67e7f || n[0] * n[3] + n[1] * n[2] > 1.67e7f) atomicExch(bad, 1);
+      for (int j = 0; j < 4; j++) {
+        for (int o = 16; o > 0; o >>= 1) n[j] = fmaxf(n[j], __shfl_xor_sync(0xffffffffu, n[j], o));
+        n[j] = sqrtf(n[j]);
+      }
+      if (lane == 0 && (2.f * n[0] * n[2] + n[1] * n[1] > 1.67e7f || n[0] * n[3] + n[1] * n[2] > 1.67e7f)) atomicExch(bad, 1);
     }
     __syncthreads();
   }
