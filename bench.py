@@ -59,6 +59,9 @@ EXEC_FLOP_FP64_ELEM = 378 * 64 * 72 + 64 * 243 + 64 * 3420 + 30_000  # ~2.0 M
 EXEC_FLOP_TC_ELEM = 3 * 2 * 128 * 96 * 256                         # 18.9 M
 # FP64-quality tensor-core kernel: 12 BF16 products of M128 x N96 x K256 per element
 EXEC_FLOP_OZ_ELEM = 12 * 2 * 128 * 96 * 256                        # 75.5 M
+# FP64 tensor-core kernel (exact slices): per K-step of 16 (16 of them) 20 BF16
+# products of N 80 and 3 of N 96, M128
+EXEC_FLOP_XS_ELEM = 16 * 2 * 128 * 16 * (20 * 80 + 3 * 96)         # 123.7 M
 # residual-only FP64 kernel: state interpolation, law and projection per point
 EXEC_FLOP_RES_ELEM = 64 * 3420 + 64 * 243
 # double-FP32 residual kernel (res_df_kernel), FP32-pipe lane instructions per
@@ -72,6 +75,9 @@ ALG_BYTES_RES_DF_ELEM = 64 * 244 * 8 + 81 * 8
 # FP64-quality tangent: per element the slices (8 chunks x 22,528 B), the row
 # exponents (88 B) and the read-modify-write of its 6,561 FP64 CSR slots
 ALG_BYTES_OZ_ELEM = 8 * 22528 + 88 + 2 * 8 * 6561
+# FP64 tensor-core kernel: the six slices (8 chunks x 33,792 B), the row
+# exponents and row 80, the element matrix (27,216 B) and residual written
+ALG_BYTES_XS_ELEM = 8 * 33792 + 88 * 2 + 256 * 8 + 27216 + 2 * 648
 # cached-operand tensor-core tangent: per element the operands (8 chunks x
 # 11,264 B) and the read-modify-write of its 6,561 FP64 CSR slots
 ALG_BYTES_TCS_ELEM = 8 * 11264 + 2 * 8 * 6561
@@ -686,6 +692,20 @@ def main():
                                 "executed_frac is the FP64 pipe fraction")
         return out
 
+    def exact_roofline(kms, kl, kc, step_total_ms):
+        """The FP64 mode's tensor-core kernel (exact BF16 slices of the Gram operands)."""
+        sec, el = kms / max(kl, 1) * 1e-3, kc / max(kl, 1)
+        ach, gbs = EXEC_FLOP_XS_ELEM * el / sec / 1e12, ALG_BYTES_XS_ELEM * el / sec / 1e9
+        return {"bound": "tensor", "achieved": ach, "peak": bf16_peak, "unit": "TFLOP/s", "frac": ach / bf16_peak,
+                "kernel": "exact_tangent_kernel (six 9-bit BF16 slices of the Gram operands, 46 tcgen05.mma kind::f16 "
+                          "per chunk, integer recombination; residual K_e u_e)",
+                "executed_tensor_flop_per_element": EXEC_FLOP_XS_ELEM,
+                "hbm_algorithmic_bytes_per_element": ALG_BYTES_XS_ELEM, "hbm_achieved_gbs": gbs,
+                "hbm_frac": gbs / hbm_peak, "peak_source": "MEASURED_PEAKS.json bf16_tflops and hbm_gbs (copy)",
+                "fp64_equivalent_tflops": (TAN_FLOP_PER_ELEM + RES_FLOP_PER_ELEM) * el / sec / 1e12,
+                "elements_per_launch": el, "avg_launch_ms": sec * 1e3,
+                "kernel_share_of_step": kms / step_total_ms if step_total_ms > 0 else None}
+
     def res_df_roofline(kms, kl, kc, step_total_ms):
         """The double-FP32 residual kernel of the tensor-core modes: bound by the
         FP32 pipe (lane instructions against the measured FMA issue rate)."""
@@ -732,9 +752,12 @@ def main():
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (copy) and bf16_tflops",
                 "avg_launch_ms": per_launch_ms, "elements_per_launch": per_launch_el}
 
+    # the FP64 mode of this law runs on the tensor cores unless switched off
+    exact64 = os.environ.get("IGAPGPU_TC_EXACT") != "0"
     mode_desc = {"fp64q": "double-FP32 residual (FP32 pipe); tangent on the tensor cores from error-free BF16 "
                           "slices (FP64 quality)",
-                 "fp64": "FP64 residual and tangent (FP64 pipe)",
+                 "fp64": "FP64 residual and tangent (tensor cores, exact BF16 slices summed in 64-bit integers)" if exact64
+                 else "FP64 residual and tangent (FP64 pipe)",
                  "split": "double-FP32 residual (FP32 pipe); TF32x3 tensor-core tangent"}
     blocks = {}
     for name, (mms, mstep, mkinds, mlaunch) in runs.items():
@@ -747,7 +770,8 @@ def main():
              "setup_launches": prep_launches.get(name)}
         if name == "fp64":
             b["fp64_kernel_ms_per_step"] = res_ms / a.steps
-            b["fp64_kernel_roofline"] = fp64_roofline(name, res_ms, res_l, res_c, tot)
+            b["fp64_kernel_roofline"] = (exact_roofline(res_ms, res_l, res_c, tot) if exact64
+                                         else fp64_roofline(name, res_ms, res_l, res_c, tot))
         else:
             b["res_kernel_ms_per_step"] = res_ms / a.steps
             b["res_kernel_roofline"] = res_df_roofline(res_ms, res_l, res_c, tot)

@@ -8,7 +8,7 @@
 //   no host synchronisation inside.  Once the residual estimate reaches the
 //   tolerance a device flag predicates the remaining steps of the cycle off.
 //   The host reads one small state record per cycle.
-// * The assembly (colour launches, Dirichlet rows and columns) is captured
+// * The assembly (element kernels, gathers, Dirichlet rows and columns) is captured
 //   once per (residual, tangent, precision) and replayed.
 #include <cuda_runtime.h>
 #include <math.h>

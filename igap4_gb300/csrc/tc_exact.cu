@@ -164,8 +164,8 @@ __device__ __forceinline__ double scaled(long long v, int k)
 // element: S in shared memory (row stride K + 1), row exponents, digits.
 // Integer operations and the loads' latency bound it: the digits as bit fields of
 // a biased sum with one exact FMA each, and the next point's loads in flight,
-// take the first assembly at 63x17x15 from 7.2 to 5.3 ms (76 k -> 41 k clocks
-// an element here).
+// take it from 4.2 to 2.5 ms at 63x17x15 (76 k -> 45 k clocks an element) and the
+// first assembly from 7.2 to 5.3 ms.
 __global__ void __launch_bounds__(XO_THREADS) exact_operand_kernel(const double *__restrict__ geo, int npts, int nchunk,
                                                                    int64_t nelem, double ell,
                                                                    unsigned char *__restrict__ ops,

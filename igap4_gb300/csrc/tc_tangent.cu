@@ -11,7 +11,7 @@
 // (8 points x 5 slots).  Each operand is split into TF32 hi + lo parts and
 // the three products hi.hi + hi.lo + lo.hi accumulate in FP32 in tensor
 // memory; the epilogue reads TMEM and adds into the FP64 CSR values.
-// The residual is not touched here (the FP64 element kernel computes it).
+// The residual is not touched here (it has its own kernels).
 //
 // One persistent CTA per SM walks the elements of one colour, so the CSR
 // scatter is conflict-free as in the FP64 kernel.  The reference's laws with

@@ -259,7 +259,7 @@ const char *igapgpu_last_error(void);
 int64_t igapgpu_launch_count(void);
 
 /* Timing of the element-assembly kernels with CUDA events recorded on the
- * launching stream around each colour batch.  enable=1 resets and starts,
+ * launching stream around the kernels.  enable=1 resets and starts,
  * enable=0 stops; igapgpu_profile_read synchronises and returns the summed
  * kernel time (ms), the number of element-kernel launches and the number of
  * elements they processed since the last reset. */
