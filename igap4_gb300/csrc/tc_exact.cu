@@ -34,9 +34,8 @@
 // Measured: against 64-bit reference sums the error is the FP64 kernel's (7e-16
 // at 16x4x4, 3e-15 at 63x17x15 distorted, both from the geometry; the two
 // tangents differ by 2e-16).  Residual and tangent at 16x4x4 7.9 ms (FP64 kernel,
-// colour by colour) -> 79 us, 63x17x15 36.7 -> 2.33 ms, 128x32x32 255.7 ->
-// 18.6 ms; per element and SM 36 k clocks, 27 k of them MMAs (their
-// shared-memory operand reads) and 9 k the accumulators' drain.
+// colour by colour) -> 76 us, 63x17x15 36.7 -> 2.05 ms.  Per element and SM 31 k
+// clocks, 27 k of them MMAs (73 clocks each: shared-memory operand reads).
 //
 // One persistent CTA per SM over all elements; results go to the element
 // buffers (gather.cu):
@@ -46,7 +45,9 @@
 //   warps 4-6 and 8-10: accumulators -> Y[r][c] in shared memory (int64, units
 //     of 2^-36): c > r the symmetric sums and X, c < r X alone, so that
 //     G_rc = Y[r][c] + Y[c][r]; the tensor memory is free for the next element
-//     after that,
+//     after that.  acc78 is drained first and released alone: its products, 11
+//     of 23, of the next element's staged chunks run while the others are
+//     drained (9 k clocks that the tensor core stood idle: 36 -> 31 k clocks),
 //   warps 2-13: a thread per basis pair b <= c forms its 3 x 3 block of K in
 //     FP64; the element's blocks leave by one bulk copy, and the residual of
 //     the linear law is K_e u_e from the blocks in shared memory (6,561 FMA an
@@ -96,7 +97,7 @@ struct XsSmem {
   double g80;
   double u[NE], rsum[4][NE];
   int ex[XS_EXP];
-  uint64_t full[XS_NS], empty[XS_NS], accfull, accempty;
+  uint64_t full[XS_NS], empty[XS_NS], accfull, accempty, empty78;
   uint32_t cp_n[XS_NS], mm_n[XS_NS], accf_n;
   uint32_t taddr;
   int abort;
@@ -362,6 +363,7 @@ __global__ void __launch_bounds__(XS_THREADS, 1) exact_tangent_kernel(ExactArgs 
     }
     tc::mbar_init(&S.accfull, 1);
     tc::mbar_init(&S.accempty, 192);
+    tc::mbar_init(&S.empty78, 192);
     S.accf_n = 0;
     S.abort = 0;
   }
@@ -396,40 +398,68 @@ __global__ void __launch_bounds__(XS_THREADS, 1) exact_tangent_kernel(ExactArgs 
       const uint32_t id80 = tc::instr_desc(1, 128, 80), id96 = tc::instr_desc(1, 128, 96);
       uint32_t s = 0, mmn[XS_NS] = {}, accn = 0;
       bool ok = true;
+      auto slices = [&](uint32_t st, int ks, uint64_t *d) {
+        const uint32_t base = tc::smem_u32(S.stage[st]);
+#pragma unroll
+        for (int q = 0; q < XS_NSL; q++)
+          d[q] = tc::smem_desc(base + (uint32_t)(q * XS_SLICE_BYTES + ks * XS_KS_BYTES), 128, 256);
+      };
+      auto low = [&](uint32_t st, uint32_t c) {  // the products of acc78
+        for (int ks = 0; ks < 2; ks++) {
+          uint64_t d[XS_NSL];
+          slices(st, ks, d);
+#pragma unroll
+          for (int q = 0; q < 6; q++)
+            tc::mma_bf16(taddr + XS_ACC78, d[q], d[5 - q], id80, c == 0 && ks == 0 && q == 0 ? 0u : 1u);
+#pragma unroll
+          for (int q = 1; q < 6; q++) tc::mma_bf16(taddr + XS_ACC78, d[q], d[6 - q], id80, 1u);
+        }
+      };
+      auto high = [&](uint32_t st, uint32_t c) {  // the others
+        for (int ks = 0; ks < 2; ks++) {
+          uint64_t d[XS_NSL];
+          slices(st, ks, d);
+          const uint32_t first = (c == 0 && ks == 0) ? 0u : 1u;
+          tc::mma_bf16(taddr + XS_ACC2, d[0], d[0], id80, first);
+          tc::mma_bf16(taddr + XS_X3, d[0], d[1], id96, first);
+          tc::mma_bf16(taddr + XS_ACC4, d[0], d[2], id80, first);
+          tc::mma_bf16(taddr + XS_ACC4, d[2], d[0], id80, 1u);
+          tc::mma_bf16(taddr + XS_ACC4, d[1], d[1], id80, 1u);
+          tc::mma_bf16(taddr + XS_X5, d[0], d[3], id96, first);
+          tc::mma_bf16(taddr + XS_X5, d[1], d[2], id96, 1u);
+#pragma unroll
+          for (int q = 0; q < 5; q++) tc::mma_bf16(taddr + XS_ACC6, d[q], d[4 - q], id80, q == 0 ? first : 1u);
+        }
+      };
+      const uint32_t lead = nchunk < (uint32_t)XS_NS ? nchunk : (uint32_t)XS_NS;  // chunks that the stages hold at once
       for (int j = 0; j < nmine && ok; j++) {
-        if (j >= 1 && !xs_wait(&S.accempty, ((uint32_t)j - 1) & 1, abort)) {
-          ok = false;
+        // acc78 is drained first: its products of the staged chunks run while
+        // the other accumulators are drained
+        ok = j == 0 || xs_wait(&S.empty78, ((uint32_t)j - 1) & 1, abort);
+        uint32_t c = 0;
+        for (; c < lead && ok; c++) {
+          const uint32_t st = (s + c) % XS_NS;
+          if (!(ok = xs_wait(&S.full[st], ((s + c) / XS_NS) & 1, abort))) break;
+          tc::fence_after_sync();
+          low(st, c);
+        }
+        ok = ok && (j == 0 || xs_wait(&S.accempty, ((uint32_t)j - 1) & 1, abort));
+        if (!ok) {
+          if (c > 0) {  // the teardown waits for the products issued
+            tc::mma_commit(&S.empty[s % XS_NS]);
+            mmn[s % XS_NS]++;
+          }
           break;
         }
         tc::fence_after_sync();
-        for (uint32_t c = 0; c < nchunk; c++, s++) {
-          const int st = (int)(s % XS_NS);
-          if (!xs_wait(&S.full[st], (s / XS_NS) & 1, abort)) {
-            ok = false;
-            break;
+        for (c = 0; c < nchunk; c++, s++) {
+          const uint32_t st = s % XS_NS;
+          if (c >= lead) {
+            if (!(ok = xs_wait(&S.full[st], (s / XS_NS) & 1, abort))) break;
+            tc::fence_after_sync();
+            low(st, c);
           }
-          tc::fence_after_sync();
-          const uint32_t base = tc::smem_u32(S.stage[st]);
-          for (int ks = 0; ks < 2; ks++) {
-            uint64_t d[XS_NSL];
-#pragma unroll
-            for (int q = 0; q < XS_NSL; q++)
-              d[q] = tc::smem_desc(base + (uint32_t)(q * XS_SLICE_BYTES + ks * XS_KS_BYTES), 128, 256);
-            const uint32_t first = (c == 0 && ks == 0) ? 0u : 1u;
-            tc::mma_bf16(taddr + XS_ACC2, d[0], d[0], id80, first);
-            tc::mma_bf16(taddr + XS_X3, d[0], d[1], id96, first);
-            tc::mma_bf16(taddr + XS_ACC4, d[0], d[2], id80, first);
-            tc::mma_bf16(taddr + XS_ACC4, d[2], d[0], id80, 1u);
-            tc::mma_bf16(taddr + XS_ACC4, d[1], d[1], id80, 1u);
-            tc::mma_bf16(taddr + XS_X5, d[0], d[3], id96, first);
-            tc::mma_bf16(taddr + XS_X5, d[1], d[2], id96, 1u);
-#pragma unroll
-            for (int q = 0; q < 5; q++) tc::mma_bf16(taddr + XS_ACC6, d[q], d[4 - q], id80, q == 0 ? first : 1u);
-#pragma unroll
-            for (int q = 0; q < 6; q++) tc::mma_bf16(taddr + XS_ACC78, d[q], d[5 - q], id80, q == 0 ? first : 1u);
-#pragma unroll
-            for (int q = 1; q < 6; q++) tc::mma_bf16(taddr + XS_ACC78, d[q], d[6 - q], id80, 1u);
-          }
+          high(st, c);
           tc::mma_commit(&S.empty[st]);
           mmn[st]++;
         }
@@ -500,16 +530,28 @@ __global__ void __launch_bounds__(XS_THREADS, 1) exact_tangent_kernel(ExactArgs 
         const int r = quarter * 32 + lane;
         const uint32_t ta = taddr + ((uint32_t)(quarter * 32) << 16);
         const int cb1 = half ? 6 : 3;
+        // acc78 first: its integers wait in Y's slots, and the next element's
+        // products may overwrite it
+        for (int cb = half ? 3 : 0; cb < min(cb1, 5); cb++) {
+          uint32_t v8[16];
+          tc::tmem_ld_32x32b_x16(ta + XS_ACC78 + cb * 16, v8);
+          tc::tmem_wait_ld();
+          if (r < XS_ROWS)
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+              S.Y[r * XS_YP + cb * 16 + i] = units(v8[i], 0x1p36f, 0);
+        }
+        tc::fence_before_sync();
+        mbar_arrive1(&S.empty78);
         for (int cb = half ? 3 : 0; cb < cb1; cb++) {
           uint32_t v3[16], v5[16];
           tc::tmem_ld_32x32b_x16(ta + XS_X3 + cb * 16, v3);
           tc::tmem_ld_32x32b_x16(ta + XS_X5 + cb * 16, v5);
           if (cb < 5) {
-            uint32_t v2[16], v4[16], v6[16], v8[16];
+            uint32_t v2[16], v4[16], v6[16];
             tc::tmem_ld_32x32b_x16(ta + XS_ACC2 + cb * 16, v2);
             tc::tmem_ld_32x32b_x16(ta + XS_ACC4 + cb * 16, v4);
             tc::tmem_ld_32x32b_x16(ta + XS_ACC6 + cb * 16, v6);
-            tc::tmem_ld_32x32b_x16(ta + XS_ACC78 + cb * 16, v8);
             tc::tmem_wait_ld();
             if (r < XS_ROWS)
 #pragma unroll
@@ -517,7 +559,7 @@ __global__ void __launch_bounds__(XS_THREADS, 1) exact_tangent_kernel(ExactArgs 
                 const int c = cb * 16 + i;
                 const long long x = units(v3[i], 0x1p9f, 27) + units(v5[i], 0x1p27f, 9);
                 const long long g = units(v2[i], 1.f, 36) + units(v4[i], 0x1p18f, 18) + units(v6[i], 0x1p36f, 0) +
-                                    units(v8[i], 0x1p36f, 0);
+                                    S.Y[r * XS_YP + c];
                 // the symmetric part once per pair: at c > r, and at row 80 for its column's sake
                 S.Y[r * XS_YP + c] = c == r ? g + 2 * x : ((c > r || r == 80) ? g + x : x);
               }

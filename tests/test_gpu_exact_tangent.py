@@ -52,3 +52,12 @@ def test_matches_oracle():
     A.set_state(U)
     Ko = po.OracleCase(prob).tangent(U)
     assert np.linalg.norm(A.tangent() - Ko) <= 1e-14 * np.linalg.norm(Ko)
+
+
+# 496 elements: three or four per SM; 1, 4 and 8 chunks (fewer than, as many as
+# and more than the copy stages).  Tolerance as above.
+@pytest.mark.parametrize("nquad", [2, 3, 4])
+def test_several_elements_per_block(monkeypatch, nquad):
+    K, Kf = both(monkeypatch, (31, 4, 4), [0.9, 1.2, 0.1], nquad, True, True)
+    assert np.linalg.norm(K - Kf) <= 4e-15 * np.linalg.norm(Kf)
+    assert np.abs(K - Kf).max() <= 4e-15 * np.abs(Kf).max()
