@@ -20,7 +20,10 @@
 namespace igap {
 
 namespace {
-constexpr int TG_THREADS = 256;
+// 567 entries (63 columns from the diagonal on) are three rounds of 192
+// threads, seven blocks per SM: 322 -> 240 us at 63x17x15 (256 threads, four
+// blocks); the FP32 form's 1125 entries take 505 us with 256, 534 with 192
+constexpr int TG_THREADS = 192, TGF_THREADS = 256;
 constexpr int TG_NJ = 125;  // control points in a row's stencil
 
 // Elements of one direction that hold both control points i and j, by
@@ -83,7 +86,7 @@ struct GatherTab {
   unsigned char rank[3][9], off[3][9], n[3][9];
 };
 
-template <typename F>
+template <int NT, typename F>
 __device__ __forceinline__ void gather_table(GatherTab &G, const Patch &p, int64_t e0, int64_t per_element,
                                              const int *dir, F entry)
 {
@@ -101,7 +104,7 @@ __device__ __forceinline__ void gather_table(GatherTab &G, const Patch &p, int64
     G.n[dir][3 * a + c] = (unsigned char)max(r.n, 0);
     G.off[dir][3 * a + c] = (unsigned char)(i - a + c - lo);
   }
-  for (int j = threadIdx.x; j < p.nj; j += TG_THREADS) {
+  for (int j = threadIdx.x; j < p.nj; j += NT) {
     unsigned f = 0;
     if (dir) {
       const int jz = p.loz + j % p.cz, jy = p.loy + (j / p.cz) % p.cy, jx = p.lox + j / (p.cz * p.cy);
@@ -111,7 +114,7 @@ __device__ __forceinline__ void gather_table(GatherTab &G, const Patch &p, int64
     G.fix[j] = (unsigned char)f;
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < 27 * NB; t += TG_THREADS) {
+  for (int t = threadIdx.x; t < 27 * NB; t += NT) {
     const int b = t / NB, c = t % NB;
     if (G.ebase[b] < 0) continue;
     const int x = b / 9 * 3 + c / 9, y = (b / 3) % 3 * 3 + (c / 3) % 3, z = b % 3 * 3 + c % 3;
@@ -129,7 +132,7 @@ __device__ __forceinline__ void gather_table(GatherTab &G, const Patch &p, int64
 // The matrix is symmetric and so are its element blocks: the columns from the
 // diagonal on are summed once and stored in both rows (the FP64 additions and
 // the reads halve).
-__global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a, const double *__restrict__ ebuf,
+__global__ void __launch_bounds__(TG_THREADS, 7) tangent_gather_kernel(GatherMap a, const double *__restrict__ ebuf,
                                                                     double *__restrict__ vals)
 {
   __shared__ GatherTab G;
@@ -149,7 +152,7 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a,
     tbase[j] = r + 3 * (((p.ix - max(jx - P, 0)) * cy + p.iy - max(jy - P, 0)) * cz + p.iz - max(jz - P, 0));
     tlen[j] = 3 * cx * cy * cz;
   }
-  gather_table(G, p, a.eoff ? __ldg(a.eoff + inst) : 0, EBUF, a.dir ? a.dir + m.dof_off : nullptr, [](int b, int c) {  // block offset, bit 15: transposed
+  gather_table<TG_THREADS>(G, p, a.eoff ? __ldg(a.eoff + inst) : 0, EBUF, a.dir ? a.dir + m.dof_off : nullptr, [](int b, int c) {  // block offset, bit 15: transposed
     return 9 * pair_index(min(b, c), max(b, c)) | (b > c ? 0x8000 : 0);
   });
   const int64_t r0 = __ldg(a.rowptr + 3 * cp);
@@ -175,17 +178,17 @@ __global__ void __launch_bounds__(TG_THREADS) tangent_gather_kernel(GatherMap a,
 // The same from FP32 element matrices [27 b][3 d][27 c][3 e] (not symmetric to
 // the last bit): a thread per entry of the rows, consecutive threads along
 // the columns, in the buffer as in the CSR rows.
-__global__ void __launch_bounds__(TG_THREADS) tangent_gather_f32_kernel(GatherMap a, const float *__restrict__ fbuf,
+__global__ void __launch_bounds__(TGF_THREADS) tangent_gather_f32_kernel(GatherMap a, const float *__restrict__ fbuf,
                                                                         double *__restrict__ vals)
 {
   __shared__ GatherTab G;
   const int64_t cp = blockIdx.x;
   const Patch p = patch_of(a.m, cp);
-  gather_table(G, p, 0, NB * 243, a.dir, [](int b, int c) { return 243 * b + 3 * c; });
+  gather_table<TGF_THREADS>(G, p, 0, NB * 243, a.dir, [](int b, int c) { return 243 * b + 3 * c; });
   const int64_t r0 = __ldg(a.rowptr + 3 * cp);
   const int row = 3 * p.nj;
   const int self = ((p.ix - p.lox) * p.cy + p.iy - p.loy) * p.cz + p.iz - p.loz, rfix = G.fix[self];
-  for (int t = threadIdx.x; t < 3 * row; t += TG_THREADS) {
+  for (int t = threadIdx.x; t < 3 * row; t += TGF_THREADS) {
     const int d = t / row, x = t - d * row, j = x / 3, e = x - 3 * j;
     const int n = G.cnt[j];
     const int *tab = G.tab + j * 27;
@@ -290,7 +293,7 @@ int launch_tangent_gather(Context *c, double *vals, const int *err)
 
 int launch_tangent_gather_f32(Context *c, double *vals)
 {
-  tangent_gather_f32_kernel<<<(unsigned)(c->ndof / 3), TG_THREADS, 0, c->stream>>>(gather_map(c), c->d_fbuf, vals);
+  tangent_gather_f32_kernel<<<(unsigned)(c->ndof / 3), TGF_THREADS, 0, c->stream>>>(gather_map(c), c->d_fbuf, vals);
   count_launch();
   IGAP_CHECK_LAUNCH();
   return IGAPGPU_OK;
