@@ -84,6 +84,7 @@ def lib():
         L.igapgpu_density.argtypes = [vp, vp, vp]
         L.igapgpu_sample_field.argtypes = [vp, ctypes.c_int, vp, vp, vp, vp, vp]
         L.igapgpu_debug_slot_counts.argtypes = [vp, vp]
+        L.igapgpu_debug_set_error.argtypes = [vp, ctypes.c_int]
         L.igapgpu_save_solution.argtypes = [vp, ctypes.c_char_p]
         L.igapgpu_load_solution.argtypes = [vp, ctypes.c_char_p]
         L.igapgpu_impose_dirichlet.argtypes = [vp, vp]
@@ -291,6 +292,10 @@ class Assembly:
         out = np.zeros(self.nnz)
         _check(lib().igapgpu_debug_slot_counts(self.h, _ptr(out)))
         return out
+
+    def debug_set_error(self, code):
+        """Set the error words as a kernel that gave up does (a debug aid)."""
+        _check(lib().igapgpu_debug_set_error(self.h, code))
 
     def save_solution(self, fname):
         """Write the reference's solution file (IGAPSolvSaveSolution layout)."""

@@ -166,7 +166,7 @@ static int check_err_word(Context *c)
     set_error("tensor-core tangent: a bounded mbarrier wait expired (code %d)", herr);
     return IGAPGPU_ERR_TIMEOUT;
   }
-  return IGAPGPU_OK;
+  return check_async_error(c);
 }
 
 // Instance of every element and control point, for kernels over the whole

@@ -179,7 +179,8 @@ struct Context {
   short *d_xexp = nullptr;     // their row exponents
   double *d_xrow = nullptr;    // row 80 of every element's operand
   int exact_state = -1;        // -1 not decided, 0 off, 1 on
-  bool exact_ran = false;      // a launch whose error word has not been read yet
+  int *d_xerr = nullptr;       // their kernel's error words: [0] its last launch, [1] any launch not reported yet
+  bool exact_ran = false;      // a launch whose word [1] has not been read yet
   double *d_dens = nullptr;    // per-element density sums + result (igapgpu_density, lazy)
   int *d_dsparse = nullptr;    // sparse constant tangent: dptr | dcol | sptr | sl
   double *d_dval = nullptr;

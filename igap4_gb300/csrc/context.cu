@@ -183,7 +183,7 @@ static int free_ctx(Context *c)
   void *bufs[] = {c->d_wq, c->d_xq, c->d_w, c->d_X, c->d_Uhist, c->d_RR, c->d_vals,
                   c->d_rowptr, c->d_cols, c->d_Dconst, c->d_Fneu, c->d_dir_rows, c->d_dir_g, c->d_dirmap,
                   c->d_stage_a, c->d_stage_b, c->d_stage_v, c->d_V, c->d_Z, c->d_work,
-                  c->d_diag, c->d_bdiag, c->d_cinv, c->d_asmz, c->d_red, c->d_partial, c->d_err, c->d_geo, c->d_geof, c->d_gop, c->d_oz, c->d_ozexp, c->d_rpc, c->d_rel, c->d_upair, c->d_lin, c->d_preR, c->d_preD, c->d_ebuf, c->d_fbuf, c->d_sft, c->d_rbuf, c->d_xops, c->d_xexp, c->d_xrow, c->d_dens, c->d_dsparse, c->d_dval, c->d_sval, c->d_bct, c->d_neu};
+                  c->d_diag, c->d_bdiag, c->d_cinv, c->d_asmz, c->d_red, c->d_partial, c->d_err, c->d_geo, c->d_geof, c->d_gop, c->d_oz, c->d_ozexp, c->d_rpc, c->d_rel, c->d_upair, c->d_lin, c->d_preR, c->d_preD, c->d_ebuf, c->d_fbuf, c->d_sft, c->d_rbuf, c->d_xops, c->d_xexp, c->d_xrow, c->d_xerr, c->d_dens, c->d_dsparse, c->d_dval, c->d_sval, c->d_bct, c->d_neu};
   for (void *b : bufs)
     if (b) cudaFree(b);
   for (int d = 0; d < 3; d++) {
@@ -529,11 +529,11 @@ int check_async_error(Context *c)
   if (!c->exact_ran) return IGAPGPU_OK;
   c->exact_ran = false;
   int herr = 0;
-  IGAP_CUDA(cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  IGAP_CUDA(cudaMemcpyAsync(&herr, c->d_xerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   IGAP_CUDA(cudaStreamSynchronize(c->stream));
   if (!herr) return IGAPGPU_OK;
-  IGAP_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-  set_error("tensor-core tangent: a bounded mbarrier wait expired (code %d)", herr);
+  IGAP_CUDA(cudaMemsetAsync(c->d_xerr + 1, 0, sizeof(int), c->stream));
+  set_error("tensor-core assembly: a bounded mbarrier wait expired (code %d)", herr);
   return IGAPGPU_ERR_TIMEOUT;
 }
 
@@ -636,6 +636,19 @@ static void solution_levels(const Context *c, int *l0, int *l1)
 {
   *l0 = c->torder == 0 ? 0 : 1;
   *l1 = c->torder == 0 ? 1 : c->torder + 1;
+}
+
+int igapgpu_debug_set_error(igapgpu_t c, int code)
+{
+  if (!c || code == 0) return IGAPGPU_ERR_ARG;
+  const int words[2] = {code, code};
+  IGAP_CUDA(cudaStreamSynchronize(c->stream));
+  IGAP_CUDA(cudaMemcpy(c->d_err, words, sizeof(int), cudaMemcpyHostToDevice));
+  if (c->exact_state == 1) {
+    IGAP_CUDA(cudaMemcpy(c->d_xerr, words, sizeof words, cudaMemcpyHostToDevice));
+    c->exact_ran = true;
+  }
+  return IGAPGPU_OK;
 }
 
 int igapgpu_save_solution(igapgpu_t c, const char *fname)

@@ -531,7 +531,7 @@ int assembly_graph(Context *c, bool do_res, bool do_tan)
       return IGAPGPU_ERR_TIMEOUT;
     }
   }
-  return IGAPGPU_OK;
+  return c->batch ? check_async_error(c) : IGAPGPU_OK;
 }
 
 }  // namespace igap

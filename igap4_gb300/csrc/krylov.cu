@@ -572,7 +572,7 @@ int igapgpu_solve(igapgpu_t c, double *U, const igapgpu_solver_opts *opts, igapg
     if (uh) IGAP_CUDA(cudaMemcpyAsync(U, Ud, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
     IGAP_CUDA(cudaStreamSynchronize(c->stream));
     if (st) *st = S;
-    return IGAPGPU_OK;
+    return check_async_error(c);  // a NaN norm may be a kernel that gave up
   }
   for (int it = 0; it < o.snes_max_it; it++) {
     if (!isfinite(fnorm)) { S.reason = -4; break; }

@@ -53,9 +53,12 @@
 //     the linear law is K_e u_e from the blocks in shared memory (6,561 FMA an
 //     element under the next element's MMAs; the quadrature loop takes 93,312
 //     on the FP64 pipe).
-// Every mbarrier wait is bounded; a CTA that gives up sets the error word
-// (the gather then writes NaN), waits (bounded) for its copies and MMAs in
-// flight and frees its tensor memory.
+// Every mbarrier wait is bounded; a CTA that gives up sets the error words
+// (the gathers of this launch then write NaN; the context reports the other
+// word at its next synchronisation), waits (bounded) for its copies and MMAs in
+// flight and frees its tensor memory.  The words are this kernel's own: what
+// another kernel left in the context's shared word is not taken for a failure
+// of this launch, and another launch does not clear one before it is reported.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
@@ -120,7 +123,7 @@ struct ExactArgs {
   const DevMesh *meshes;
   const int64_t *eoff;
   const int *einst;
-  int *err;
+  int *err;  // [0] this launch, [1] until reported
 };
 
 __device__ __forceinline__ void mbar_arrive1(uint64_t *mbar)
@@ -627,6 +630,7 @@ __global__ void __launch_bounds__(XS_THREADS, 1) exact_tangent_kernel(ExactArgs 
     }
     if (S.accf_n > 0) tc::mbar_wait(&S.accfull, (S.accf_n - 1) & 1, XS_WAIT_LIMIT);
     atomicCAS(a.err, 0, 2);
+    atomicCAS(a.err + 1, 0, 2);
   }
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(taddr, XS_TMEM_COLS);
@@ -634,7 +638,7 @@ __global__ void __launch_bounds__(XS_THREADS, 1) exact_tangent_kernel(ExactArgs 
 
 static void exact_free(Context *c)
 {
-  void **p[] = {&c->d_xops, (void **)&c->d_xexp, (void **)&c->d_xrow};
+  void **p[] = {&c->d_xops, (void **)&c->d_xexp, (void **)&c->d_xrow, (void **)&c->d_xerr};
   for (void **q : p) {
     if (*q) cudaFree(*q);
     *q = nullptr;
@@ -673,7 +677,9 @@ bool ensure_exact(Context *c)
   int *d_bad = nullptr;
   bool ok = ensure_ebuf(c) && ensure_rbuf(c) && cudaMalloc(&c->d_xops, bytes) == cudaSuccess &&
             cudaMalloc(&c->d_xexp, nel * XS_EXP * sizeof(short)) == cudaSuccess &&
-            cudaMalloc(&c->d_xrow, rbytes) == cudaSuccess && cudaMalloc(&d_bad, sizeof(int)) == cudaSuccess;
+            cudaMalloc(&c->d_xrow, rbytes) == cudaSuccess && cudaMalloc(&c->d_xerr, 2 * sizeof(int)) == cudaSuccess &&
+            cudaMalloc(&d_bad, sizeof(int)) == cudaSuccess &&
+            cudaMemsetAsync(c->d_xerr, 0, 2 * sizeof(int), c->stream) == cudaSuccess;
   const size_t smem = sizeof(double) * XS_ROWS * (nchunk * 32 + 1);
   int bad = 1, dev = 0, nsm = 0;
   ok = ok && cudaFuncSetAttribute(exact_operand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -726,7 +732,8 @@ int launch_exact(Context *c, double *RR, double *vals)
   a.meshes = nullptr;
   a.eoff = nullptr;
   a.einst = nullptr;
-  a.err = c->d_err;
+  a.err = c->d_xerr;
+  IGAP_CUDA(cudaMemsetAsync(c->d_xerr, 0, sizeof(int), c->stream));
   if (c->batch) batch_element_map(c, &a.laws, &a.meshes, &a.eoff, &a.einst);
   const size_t smem = sizeof(XsSmem) + 1024;
   static bool attr_set = false;
@@ -751,8 +758,8 @@ int launch_exact(Context *c, double *RR, double *vals)
     c->prof_elements[0] += c->nelem_total;
   }
   c->exact_ran = true;
-  const int r = RR ? launch_residual_gather(c, RR, 1, c->d_err) : IGAPGPU_OK;
-  return r || !vals ? r : launch_tangent_gather(c, vals, c->d_err);
+  const int r = RR ? launch_residual_gather(c, RR, 1, c->d_xerr) : IGAPGPU_OK;
+  return r || !vals ? r : launch_tangent_gather(c, vals, c->d_xerr);
 }
 
 }  // namespace igap

@@ -180,6 +180,12 @@ int igapgpu_sample_field(igapgpu_t ctx, int nppe, double *field, double *xq, dou
  * whose support holds both control points of the slot.  Host or device. */
 int igapgpu_debug_slot_counts(igapgpu_t ctx, double *counts);
 
+/* Sets the context's error words as a kernel whose bounded wait ran out does
+ * (a debug aid; code != 0, nothing runs).  The next assembly starts from
+ * cleared words; the FP64 tensor-core kernel's failure is reported by the
+ * next igapgpu_synchronize, igapgpu_solve or call with host pointers. */
+int igapgpu_debug_set_error(igapgpu_t ctx, int code);
+
 /* IGAPSolvSaveSolution / IGAPSolvLoadSolution (src/interface.c:271-300): the
  * reference's solution file (write_solution / read_solution, src/ioutil.c:
  * 90-159), raw FP64 levels in DOF order; static laws level 0, the transient
