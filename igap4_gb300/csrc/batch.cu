@@ -175,7 +175,8 @@ static bool batch_tables(Context *c)
 {
   Batch *b = c->batch;
   if (b->tables >= 0) return b->tables == 1;
-  if (c->capturing) return false;
+  if (stream_capturing(c)) return false;
+  RelaxedCapture relaxed;
   b->tables = 0;
   const int64_t nel = b->elem_off[b->ninst], ncp = c->ndof / 3;
   std::vector<int> einst((size_t)nel), cpinst((size_t)ncp);

@@ -181,6 +181,7 @@ struct Context {
   int exact_state = -1;        // -1 not decided, 0 off, 1 on
   int *d_xerr = nullptr;       // their kernel's error words: [0] its last launch, [1] any launch not reported yet
   bool exact_ran = false;      // a launch whose word [1] has not been read yet
+  bool exact_captured = false; // the kernel is in a graph of the user's: any synchronisation reads word [1]
   double *d_dens = nullptr;    // per-element density sums + result (igapgpu_density, lazy)
   int *d_dsparse = nullptr;    // sparse constant tangent: dptr | dcol | sptr | sl
   double *d_dval = nullptr;
@@ -276,6 +277,16 @@ Context *new_context(const igapgpu_mesh_desc *mesh, const igapgpu_phys_desc *phy
                      const igapgpu_bc_desc *bc, int nquad);
 int context_init(Context *c, const igapgpu_mesh_desc *mesh);
 int context_free(Context *c);
+// Whether the context's stream is being captured, by the library or its user:
+// nothing is allocated, built or waited for then.
+bool stream_capturing(const Context *c);
+// One-time set-up (allocations) allowed while another thread captures a stream
+// of its own, as the libraries' allocators do.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 // after a synchronisation: the error word of asynchronous kernels with bounded waits
 int check_async_error(Context *c);
 

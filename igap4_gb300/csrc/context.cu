@@ -524,9 +524,20 @@ Context *new_context(const igapgpu_mesh_desc *mesh, const igapgpu_phys_desc *phy
   return c;
 }
 
+bool stream_capturing(const Context *c)
+{
+  if (c->capturing) return true;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) {  // the legacy stream beside a capture
+    cudaGetLastError();
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 int check_async_error(Context *c)
 {
-  if (!c->exact_ran) return IGAPGPU_OK;
+  if (!c->exact_ran && !c->exact_captured) return IGAPGPU_OK;
   c->exact_ran = false;
   int herr = 0;
   IGAP_CUDA(cudaMemcpyAsync(&herr, c->d_xerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));

@@ -319,7 +319,8 @@ template <typename T>
 static bool ensure_buffer(Context *c, T **p, int *state, size_t per_element)
 {
   if (*state >= 0) return *state == 1;
-  if (c->capturing) return false;
+  if (stream_capturing(c)) return false;
+  RelaxedCapture relaxed;
   *state = 0;
   const size_t bytes = sizeof(T) * per_element * (size_t)c->nelem_total;
   size_t freeb = 0, totb = 0;

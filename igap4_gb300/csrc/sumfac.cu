@@ -293,7 +293,8 @@ bool ensure_sumfac(Context *c, const DevLaw &L)
 {
   if (!L.preD || c->nquad != 4 || c->porder != P || c->batch) return false;
   if (c->sf_state >= 0) return c->sf_state == 1;
-  if (c->capturing) return false;
+  if (stream_capturing(c)) return false;
+  RelaxedCapture relaxed;
   c->sf_state = 0;
   const size_t bytes = sizeof(double) * SF_NT * SF_Q * (size_t)c->nelem_total;
   size_t freeb = 0, totb = 0;

@@ -653,7 +653,8 @@ static void exact_free(Context *c)
 bool ensure_exact(Context *c)
 {
   if (c->exact_state >= 0) return c->exact_state == 1;
-  if (c->capturing) return false;
+  if (stream_capturing(c)) return false;
+  RelaxedCapture relaxed;
   c->exact_state = 0;
   const char *env = getenv("IGAPGPU_TC_EXACT");
   const int npts = c->nquad * c->nquad * c->nquad, nchunk = (npts + PW - 1) / PW;
@@ -758,6 +759,7 @@ int launch_exact(Context *c, double *RR, double *vals)
     c->prof_elements[0] += c->nelem_total;
   }
   c->exact_ran = true;
+  if (!c->capturing && stream_capturing(c)) c->exact_captured = true;
   const int r = RR ? launch_residual_gather(c, RR, 1, c->d_xerr) : IGAPGPU_OK;
   return r || !vals ? r : launch_tangent_gather(c, vals, c->d_xerr);
 }
