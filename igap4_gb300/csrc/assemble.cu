@@ -1282,6 +1282,8 @@ int launch_neumann(Context *c, const double nfac[NFACE][2])
   neumann_kernel<<<(unsigned)((c->ndof + 127) / 128), 128, 0, c->stream>>>(T, c->d_wq, c->nquad, c->ndof, c->d_Fneu);
   count_launch();
   IGAP_CHECK_LAUNCH();
+  // the load is complete on return: the caller may assemble on another stream next
+  IGAP_CUDA(cudaStreamSynchronize(c->stream));
   return IGAPGPU_OK;
 }
 

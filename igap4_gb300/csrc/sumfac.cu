@@ -308,7 +308,8 @@ bool ensure_sumfac(Context *c, const DevLaw &L)
   m.geo = nullptr;
   sumfac_t_kernel<<<(unsigned)c->nelem_total, 256, 0, c->stream>>>(m, c->d_sft);
   count_launch();
-  if (cudaGetLastError() != cudaSuccess) return false;
+  // complete before a later call on another stream reads it
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(c->stream) != cudaSuccess) return false;
   c->sf_state = 1;
   return true;
 }

@@ -248,9 +248,9 @@ int igapgpu_solve(igapgpu_t ctx, double *U, const igapgpu_solver_opts *opts,
 void igapgpu_default_solver_opts(igapgpu_solver_opts *opts);
 
 /* Replace the constant traction table (index 6*face + 3*order + d) and
- * recompute the Neumann load on the device; bc_type is unchanged.  Used by
- * time-dependent loading (the reference's neumann callback may depend on
- * par_neumann, include/bcimpl.h:6). */
+ * recompute the Neumann load on the device (complete on return); bc_type is
+ * unchanged.  Used by time-dependent loading (the reference's neumann callback
+ * may depend on par_neumann, include/bcimpl.h:6). */
 int igapgpu_set_neumann(igapgpu_t ctx, const double *table);
 
 int igapgpu_set_precision(igapgpu_t ctx, int mode);
