@@ -270,12 +270,14 @@ static int batch_kernels(Context *c, bool do_res, bool do_tan, double *RR, doubl
   }
   // the linear law's FP64 assembly of the whole queue on the tensor cores
   bool fp64_queue = fp64_tan;
-  if ((do_res || fp64_tan) && nitems == b->nitems && ensure_exact(c)) {
+  const bool x_res = do_res && exact_residual(c, fp64_tan);
+  if ((x_res || fp64_tan) && nitems == b->nitems && ensure_exact(c)) {
     if (which & 1) {
-      int r = launch_exact(c, do_res ? RR : nullptr, fp64_tan ? vals : nullptr);
+      int r = launch_exact(c, x_res ? RR : nullptr, fp64_tan ? vals : nullptr);
       if (r) return r;
     }
-    do_res = fp64_queue = false;
+    do_res = do_res && !x_res;
+    fp64_queue = false;
   }
   if ((do_res || fp64_queue) && (which & 1)) {
     int grid = 0;
@@ -323,8 +325,8 @@ int launch_batch_assembly(Context *c, bool do_res, bool do_tan, double *RR, doub
 {
   Batch *b = c->batch;
   // the exact kernel's gathers write every row and slot
-  const bool x_res = do_res && !batch_res_df(c) && ensure_exact(c);
   const bool x_tan = do_tan && c->prec != IGAPGPU_PREC_SPLIT && ensure_exact(c);
+  const bool x_res = do_res && !batch_res_df(c) && exact_residual(c, do_tan && c->prec != IGAPGPU_PREC_SPLIT) && ensure_exact(c);
   if (do_res && !x_res)
     IGAP_CUDA(cudaMemcpyAsync(RR, c->d_Fneu, sizeof(double) * c->ndof, cudaMemcpyDeviceToDevice, c->stream));
   if (do_tan && !x_tan) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));
