@@ -1183,8 +1183,8 @@ int launch_assembly(Context *c, bool do_res, bool do_tan, double *RR, double *va
   }
   // the linear law's FP64 tangent and residual on the tensor cores where its
   // slices are built
-  const bool x_tan = fp64_tan && ensure_exact(c);
-  const bool x_res = do_res && !df_res && exact_residual(c, fp64_tan) && ensure_exact(c);
+  const bool x_tan = fp64_tan && ensure_exact(c) && ensure_ebuf(c);
+  const bool x_res = do_res && !df_res && exact_residual(c, x_tan) && ensure_exact(c);
   // the reference laws' residual from precomputed law outputs
   const bool p_res = do_res && !df_res && c->law != IGAPGPU_LAW_LINGRAD && L.preR && c->d_geo && ensure_rbuf(c);
   // and their FP64 tangent by sum factorisation

@@ -270,15 +270,14 @@ static int batch_kernels(Context *c, bool do_res, bool do_tan, double *RR, doubl
   }
   // the linear law's FP64 assembly of the whole queue on the tensor cores
   bool fp64_queue = fp64_tan;
-  const bool x_res = do_res && exact_residual(c, fp64_tan);
-  if ((x_res || fp64_tan) && nitems == b->nitems && ensure_exact(c)) {
-    if (which & 1) {
-      int r = launch_exact(c, x_res ? RR : nullptr, fp64_tan ? vals : nullptr);
-      if (r) return r;
-    }
-    do_res = do_res && !x_res;
-    fp64_queue = false;
+  const bool x_tan = fp64_tan && nitems == b->nitems && ensure_exact(c) && ensure_ebuf(c);
+  const bool x_res = do_res && nitems == b->nitems && exact_residual(c, x_tan) && ensure_exact(c);
+  if ((x_res || x_tan) && (which & 1)) {
+    int r = launch_exact(c, x_res ? RR : nullptr, x_tan ? vals : nullptr);
+    if (r) return r;
   }
+  do_res = do_res && !x_res;
+  fp64_queue = fp64_queue && !x_tan;
   if ((do_res || fp64_queue) && (which & 1)) {
     int grid = 0;
     int r = fp64_grid(c, do_res, fp64_queue, &grid);
@@ -325,8 +324,8 @@ int launch_batch_assembly(Context *c, bool do_res, bool do_tan, double *RR, doub
 {
   Batch *b = c->batch;
   // the exact kernel's gathers write every row and slot
-  const bool x_tan = do_tan && c->prec != IGAPGPU_PREC_SPLIT && ensure_exact(c);
-  const bool x_res = do_res && !batch_res_df(c) && exact_residual(c, do_tan && c->prec != IGAPGPU_PREC_SPLIT) && ensure_exact(c);
+  const bool x_tan = do_tan && c->prec != IGAPGPU_PREC_SPLIT && ensure_exact(c) && ensure_ebuf(c);
+  const bool x_res = do_res && !batch_res_df(c) && exact_residual(c, x_tan) && ensure_exact(c);
   if (do_res && !x_res)
     IGAP_CUDA(cudaMemcpyAsync(RR, c->d_Fneu, sizeof(double) * c->ndof, cudaMemcpyDeviceToDevice, c->stream));
   if (do_tan && !x_tan) IGAP_CUDA(cudaMemsetAsync(vals, 0, sizeof(double) * c->nnz, c->stream));

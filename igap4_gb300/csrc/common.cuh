@@ -175,7 +175,7 @@ struct Context {
   int ebuf_state = -1, rbuf_state = -1, fbuf_state = -1;  // -1 not decided, 0 off, 1 on
   double *d_sft = nullptr;     // parametric-to-physical derivative maps [element][73][64] (sumfac.cu)
   int sf_state = -1;           // -1 not decided, 0 off, 1 on
-  void *d_xops = nullptr;      // linear law: 9-bit slices of the Gram operands (FP64 tensor-core tangent)
+  void *d_xops = nullptr;      // linear law: 9-bit slices of the Gram operands (FP64 tensor-core tangent); behind them:
   short *d_xexp = nullptr;     // their row exponents
   double *d_xrow = nullptr;    // row 80 of every element's operand
   int exact_state = -1;        // -1 not decided, 0 off, 1 on

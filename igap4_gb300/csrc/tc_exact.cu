@@ -638,18 +638,21 @@ __global__ void __launch_bounds__(XS_THREADS, 1) exact_tangent_kernel(ExactArgs 
 
 static void exact_free(Context *c)
 {
-  void **p[] = {&c->d_xops, (void **)&c->d_xexp, (void **)&c->d_xrow, (void **)&c->d_xerr};
-  for (void **q : p) {
-    if (*q) cudaFree(*q);
-    *q = nullptr;
-  }
+  if (c->d_xops) cudaFree(c->d_xops);  // the others lie behind the slices
+  c->d_xops = nullptr;
+  c->d_xrow = nullptr;
+  c->d_xexp = nullptr;
+  c->d_xerr = nullptr;
 }
 
-// Builds the slices at the first FP64 tangent (outside a capture) and says
-// whether the tensor-core path is available: the linear law, at most 64 Gauss
-// points, the FP64 geometry cache of every instance, memory for the slices
-// (275 KB an element) and the element buffers with 4 GB to spare, and digits
-// within the exactness bound.  IGAPGPU_TC_EXACT=0 keeps the FP64 kernel.
+// Builds the slices at the first call that wants them (outside a capture) and
+// says whether the tensor-core path is available: the linear law, at most 64
+// Gauss points, the FP64 geometry cache of every instance, memory for the slices
+// (275 KB an element) with 4 GB to spare, and digits within the exactness
+// bound.  The tangent needs the element buffers as well (ensure_ebuf).  One
+// allocation, and the residual buffer's beside the operand kernel: an allocation
+// takes 70 us and 100 to 150 us a GB.
+// IGAPGPU_TC_EXACT=0 keeps the FP64 kernel.
 bool ensure_exact(Context *c)
 {
   if (c->exact_state >= 0) return c->exact_state == 1;
@@ -670,22 +673,29 @@ bool ensure_exact(Context *c)
   for (Context *s : subs)
     if (!s->d_geo) return false;
   const size_t nel = (size_t)c->nelem_total;
-  const size_t bytes = nel * nchunk * XS_CH_BYTES, rbytes = nel * nchunk * 32 * sizeof(double);
+  // slices, rows 80, exponents, error words and the exactness flag
+  const size_t bytes = nel * nchunk * XS_CH_BYTES, rbytes = nel * nchunk * 32 * sizeof(double),
+               ebytes = nel * XS_EXP * sizeof(short), total = bytes + rbytes + ebytes + 3 * sizeof(int);
   size_t freeb = 0, totb = 0;
   if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess ||
-      bytes + rbytes + nel * (XS_EXP * sizeof(short) + (EBUF + NE) * sizeof(double)) + ((size_t)4 << 30) > freeb)
+      total + nel * NE * sizeof(double) + ((size_t)4 << 30) > freeb)
     return false;
-  int *d_bad = nullptr;
-  bool ok = ensure_ebuf(c) && ensure_rbuf(c) && cudaMalloc(&c->d_xops, bytes) == cudaSuccess &&
-            cudaMalloc(&c->d_xexp, nel * XS_EXP * sizeof(short)) == cudaSuccess &&
-            cudaMalloc(&c->d_xrow, rbytes) == cudaSuccess && cudaMalloc(&c->d_xerr, 2 * sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&d_bad, sizeof(int)) == cudaSuccess &&
-            cudaMemsetAsync(c->d_xerr, 0, 2 * sizeof(int), c->stream) == cudaSuccess;
+  bool ok = cudaMalloc(&c->d_xops, total) == cudaSuccess;
+  if (ok) {
+    unsigned char *p = (unsigned char *)c->d_xops + bytes;
+    c->d_xrow = (double *)p;
+    c->d_xexp = (short *)(p + rbytes);
+    c->d_xerr = (int *)(p + rbytes + ebytes);
+    ok = cudaMemsetAsync(c->d_xerr, 0, 3 * sizeof(int), c->stream) == cudaSuccess;
+  } else {
+    c->d_xops = nullptr;
+  }
+  int *d_bad = ok ? c->d_xerr + 2 : nullptr;
   const size_t smem = sizeof(double) * XS_ROWS * (nchunk * 32 + 1);
   int bad = 1, dev = 0, nsm = 0;
   ok = ok && cudaFuncSetAttribute(exact_operand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(sizeof(double) * XS_ROWS * (XS_MAXCH * 32 + 1))) == cudaSuccess &&
-       cudaMemsetAsync(d_bad, 0, sizeof(int), c->stream) == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess &&
+       cudaGetDevice(&dev) == cudaSuccess &&
        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
   for (size_t i = 0; ok && i < subs.size(); i++) {
     const Context *s = subs[i];
@@ -697,9 +707,8 @@ bool ensure_exact(Context *c)
     count_launch();
     ok = cudaGetLastError() == cudaSuccess;
   }
-  ok = ok && cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream) == cudaSuccess &&
+  ok = ok && ensure_rbuf(c) && cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream) == cudaSuccess &&
        cudaStreamSynchronize(c->stream) == cudaSuccess && !bad;
-  if (d_bad) cudaFree(d_bad);
   if (!ok) {
     cudaGetLastError();
     exact_free(c);
