@@ -147,6 +147,13 @@ __global__ void __launch_bounds__(256) conv_bwd_weight(const float *__restrict__
 // outside the lattice left out, as the one-output kernel: the same bits (a
 // BF16 rounding that falls the other way would travel through the layers).
 constexpr int CS_THREADS = 256;
+// Points up to which the one-output kernels are the faster ones: a tile's block
+// loads the layer's weights and its threads work through more outputs, 38 to 44
+// us (9 -> 32), 24 to 33 us (32 -> 3) and 13 to 16 us (the data gradient)
+// whatever the lattice below 11,000 points.  One output a thread takes 11.3 us
+// at 27 points, 40.2 at 3,920 and 58.2 at 6,800 (9 -> 32); 20.8 at 64 and 28.3 at
+// 120 (32 -> 3); 9.1 at 27, 13.9 at 1,800 and 20.5 at 3,920 (the data gradient).
+constexpr int64_t CS_MIN_IN = 4096, CS_MIN_OUT = 96, CS_MIN_DATA = 2560;
 
 template <int CI, int CO, int PT, int CT>
 __global__ void __launch_bounds__(CS_THREADS) conv_fwd_tile(const __nv_bfloat16 *__restrict__ in,
@@ -933,13 +940,13 @@ int net_forward_t(igapgpu_net *n, int B)
       const __nv_bfloat16 *x = (const __nv_bfloat16 *)n->act[l], *w = (const __nv_bfloat16 *)n->Wt + n->woff[l];
       __nv_bfloat16 *y = (__nv_bfloat16 *)n->act[l + 1];
       const int64_t pts = (int64_t)B * L.P;
-      if (kCin[l] == 9 && kCout[l] == 32) {
+      if (kCin[l] == 9 && kCout[l] == 32 && pts > CS_MIN_IN) {
         conv_fwd_tile<9, 32, 8, 8><<<(unsigned)((pts + 511) / 512), CS_THREADS, 0, n->stream>>>(x, w, n->bias + n->boff[l], y,
                                                                                               L, B, l < NL - 1);
         count_launch();
         continue;
       }
-      if (kCin[l] == 32 && kCout[l] == 3) {
+      if (kCin[l] == 32 && kCout[l] == 3 && pts > CS_MIN_OUT) {
         conv_fwd_tile<32, 3, 2, 4><<<(unsigned)((pts + 511) / 512), CS_THREADS, 0, n->stream>>>(x, w, n->bias + n->boff[l], y,
                                                                                               L, B, l < NL - 1);
         count_launch();
@@ -1006,7 +1013,7 @@ int net_backward_t(igapgpu_net *n, int B)
       if (tcd) {
         const int r = launch_conv_tc<1>(n, n->dZh, (const __nv_bfloat16 *)n->Wt + n->woff[l], nullptr, dnext, B, 0);
         if (r) return r;
-      } else if (sizeof(T) == 2 && kCout[l] == 3 && kCin[l] == 32) {
+      } else if (sizeof(T) == 2 && kCout[l] == 3 && kCin[l] == 32 && (int64_t)B * L.P > CS_MIN_DATA) {
         conv_bwd_data_out<2, 16><<<(unsigned)(((int64_t)B * L.P + 255) / 256), CS_THREADS, 0, n->stream>>>(
             dcur, (const __nv_bfloat16 *)n->Wt + n->woff[l], dnext, L, B);
         count_launch();
