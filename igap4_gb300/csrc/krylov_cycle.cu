@@ -583,6 +583,7 @@ __global__ void __launch_bounds__(CY_THREADS, 1) gmres_cycle_kernel(CycleArgs a)
       st->rnorm = fabs(S.g[k]);
     }
   }
+  if (!isfinite(S.g[k])) return;  // breakdown: every block holds this value; x stays as the last cycle left it
   if (!grid_sync(a, S, target)) return;
   for (int i = tid; i < k; i += CY_THREADS) S.h[i] = __ldcg(a.y + i);
   __syncthreads();
