@@ -212,6 +212,7 @@ struct Context {
   // CUDA graphs (graph.cu)
   GraphWork *gmres_graph = nullptr;
   CycleWork *cycle = nullptr;  // GMRES cycle kernel (krylov_cycle.cu)
+  bool cycle_unfit = false;    // its grid cannot be resident at once here
   cudaGraphExec_t asm_graph[12] = {};  // key: residual + 2 tangent + 4 precision mode
   int64_t asm_graph_nodes[12] = {};
   bool capturing = false;
@@ -362,6 +363,7 @@ int dev_diff_norm2(Context *c, const double *b, double *w, double *out);
 int setup_pc(Context *c, int pc, const double **pcd);
 // krylov_cycle.cu: GMRES restart cycles as one cooperative kernel each
 bool cycle_applies(const Context *c, int m);
+constexpr int CYCLE_UNFIT = 1;  // ksp_cycles: the grid does not fit the device, nothing was done
 int ksp_cycles(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int m, int pc, const double *pcd,
                double *V, double *Z, double *w, double *wd, bool cap, int *its, double *rnorm);
 int launch_diag_reciprocal(Context *c, double *inv);

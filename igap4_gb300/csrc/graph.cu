@@ -408,8 +408,8 @@ int ksp_gmres_graph(Context *c, const double *b, double *x, const igapgpu_solver
     const double *pcd;
     int r = setup_pc(c, pc, &pcd);
     if (r) return r;
-    return ksp_cycles(c, b, x, o, m, pc, pcd, c->d_V, c->d_Z, c->d_work, c->d_work + 3 * c->ndof, false, its_out,
-                      rnorm_out);
+    r = ksp_cycles(c, b, x, o, m, pc, pcd, c->d_V, c->d_Z, c->d_work, c->d_work + 3 * c->ndof, false, its_out, rnorm_out);
+    if (r != CYCLE_UNFIT) return r;
   }
   if (!c->gmres_graph || c->gmres_graph->m != m || c->gmres_graph->pc != pc || c->gmres_graph->orth != orth ||
       c->gmres_graph->df != spmv_df(c)) {

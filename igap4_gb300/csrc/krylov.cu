@@ -322,7 +322,7 @@ int setup_pc(Context *c, int pc, const double **pcd)
 
 // Right-preconditioned GMRES(m) with MGS, x in/out (device), b device.  The
 // cycle kernel (krylov_cycle.cu) takes it unless the restart is too long for
-// its shared memory; then one launch per vector operation.
+// its shared memory or its grid does not fit; then one launch per vector operation.
 int ksp_gmres(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int *its_out,
               double *rnorm_out)
 {
@@ -341,7 +341,10 @@ int ksp_gmres(Context *c, const double *b, double *x, const igapgpu_solver_opts 
   const int pc = o->pc >= 1 && o->pc <= 4 ? o->pc : 0;
   const double *pcd;
   if ((r = setup_pc(c, pc, &pcd))) return r;
-  if (cycle_applies(c, m)) return ksp_cycles(c, b, x, o, m, pc, pcd, V, Z, w, c->d_work + 3 * n, true, its_out, rnorm_out);
+  if (cycle_applies(c, m)) {
+    r = ksp_cycles(c, b, x, o, m, pc, pcd, V, Z, w, c->d_work + 3 * n, true, its_out, rnorm_out);
+    if (r != CYCLE_UNFIT) return r;
+  }
   std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m);
   double rnorm0 = -1.0, rnorm = 0.0;
   int its = 0;

@@ -45,6 +45,7 @@
 // and returns, the others see the word and return.
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include "common.cuh"
@@ -639,10 +640,12 @@ static int ensure_cycle(Context *c, int m)
   cycle_release(c);
   CycleWork *cw = new CycleWork();
   c->cycle = cw;
-  int dev = 0, nsm = 0;
+  int dev = 0, grid = 0;
   IGAP_CUDA(cudaGetDevice(&dev));
-  IGAP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const size_t cnt = (size_t)(m + 1) * m + (size_t)(m + 1) + 2 * (size_t)(m + 1) * CY_RMAX + 3 * (size_t)nsm;
+  IGAP_CUDA(cudaDeviceGetAttribute(&grid, cudaDevAttrMultiProcessorCount, dev));
+  const char *env = getenv("IGAPGPU_GMRES_CYCLE");
+  if (env && atoi(env) > 0) grid = atoi(env);
+  const size_t cnt = (size_t)(m + 1) * m + (size_t)(m + 1) + 2 * (size_t)(m + 1) * CY_RMAX + 3 * (size_t)grid;
   if (cudaMalloc(&cw->buf, sizeof(double) * cnt) != cudaSuccess || cudaMalloc(&cw->ctl, CY_CTL_BYTES) != cudaSuccess ||
       cudaMallocHost(&cw->h_st, CY_CTL_BYTES) != cudaSuccess) {
     cudaGetLastError();
@@ -651,16 +654,25 @@ static int ensure_cycle(Context *c, int m)
     return IGAPGPU_ERR_NOMEM;
   }
   cw->m = m;
-  cw->grid = nsm;
+  cw->grid = grid;
   return IGAPGPU_OK;
 }
 
 static size_t cycle_smem(int m) { return sizeof(CycleSmem) + sizeof(double) * ((size_t)m * (m + 1) / 2); }
 
-// Whether the cycle kernel takes this solve (19 times faster than the separate
-// launches at 32x8x8, so up to the longest restart that fits): T fits in shared memory, the
-// multiply in FP64 arithmetic (IGAPGPU_SPMV_DF keeps the separate kernels).
-bool cycle_applies(const Context *c, int m) { return m <= CY_MAX_RESTART && !spmv_df(c); }
+// Whether the cycle kernel takes this solve: T fits in shared memory, the
+// multiply is in FP64 (IGAPGPU_SPMV_DF keeps the separate kernels), and the grid
+// can be resident at once (a process limited to part of the SMs falls back, or
+// names its blocks: IGAPGPU_GMRES_CYCLE=blocks; 0 keeps the separate kernels).
+// The size draws no line: against the separate launches it is 26 times faster
+// at 32x8x8 (restart 100), 8.3 at 64x16x16, and where the matrix is ten times L2
+// (128x32x32, 1.2 GB) 1.2 times with restart 10, 1.5 with 30, 2.5 with 100, 3.3
+// with 200 (Jacobi; 1.04 with the Schwarz preconditioner, whose own data bound it).
+bool cycle_applies(const Context *c, int m)
+{
+  const char *env = getenv("IGAPGPU_GMRES_CYCLE");
+  return m <= CY_MAX_RESTART && !spmv_df(c) && !c->cycle_unfit && !(env && env[0] == '0');
+}
 
 // GMRES cycles on the context matrix; b, x device vectors, pcd the
 // preconditioner's data, V and Z the basis buffers, w 2 n and wd n scratch.  `cap`: stop at ksp_max_it
@@ -712,8 +724,14 @@ int ksp_cycles(Context *c, const double *b, double *x, const igapgpu_solver_opts
     if (cap && o->ksp_max_it - its < m) a.steps = o->ksp_max_it - its > 0 ? o->ksp_max_it - its : 0;
     IGAP_CUDA(cudaMemsetAsync(cw->ctl, 0, 256, c->stream));
     void *params[] = {&a};
-    IGAP_CUDA(cudaLaunchCooperativeKernel((const void *)gmres_cycle_kernel, dim3(cw->grid), dim3(CY_THREADS), params,
-                                          smem, c->stream));
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)gmres_cycle_kernel, dim3(cw->grid), dim3(CY_THREADS),
+                                                      params, smem, c->stream);
+    if (its == 0 && (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
+      cudaGetLastError();
+      c->cycle_unfit = true;
+      return CYCLE_UNFIT;
+    }
+    IGAP_CUDA(e);
     count_launch();
     IGAP_CUDA(cudaMemcpyAsync(cw->h_st, cw->ctl, CY_CTL_BYTES, cudaMemcpyDeviceToHost, c->stream));
     IGAP_CUDA(cudaStreamSynchronize(c->stream));
