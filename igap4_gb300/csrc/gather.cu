@@ -314,7 +314,8 @@ int launch_residual_gather(Context *c, double *RR, int parts, const int *err)
 }
 
 // Allocated at the first use outside a capture; a buffer that would leave less
-// than 4 GB free is not, and the colour launches stay in use.
+// than 4 GB free is not, and the colour launches stay in use (also with
+// IGAPGPU_ELEMENT_BUFFERS=0).
 template <typename T>
 static bool ensure_buffer(Context *c, T **p, int *state, size_t per_element)
 {
@@ -322,6 +323,8 @@ static bool ensure_buffer(Context *c, T **p, int *state, size_t per_element)
   if (stream_capturing(c)) return false;
   RelaxedCapture relaxed;
   *state = 0;
+  const char *env = getenv("IGAPGPU_ELEMENT_BUFFERS");
+  if (env && env[0] == '0') return false;
   const size_t bytes = sizeof(T) * per_element * (size_t)c->nelem_total;
   size_t freeb = 0, totb = 0;
   if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess || bytes + ((size_t)4 << 30) > freeb) return false;
