@@ -1361,7 +1361,7 @@ extern "C" int igapgpu_debug_slot_counts(igapgpu_t c, double *counts)
   }
   const bool host = !is_device_ptr(counts);
   double *d = counts;
-  if (host && cudaMalloc(&d, sizeof(double) * (size_t)c->nnz) != cudaSuccess) {
+  if (host && room_malloc(c, &d, sizeof(double) * (size_t)c->nnz) != cudaSuccess) {
     cudaGetLastError();
     set_error("debug_slot_counts: allocation failed");
     return IGAPGPU_ERR_NOMEM;

@@ -236,7 +236,7 @@ static void batch_res_df_setup(Context *c)
   for (Context *s : b->subs) ok = ok && s->d_geo != nullptr;
   if (!ok) return;
   if (!batch_tables(c)) return;
-  if (cudaMalloc(&b->d_rel, sizeof(float2) * NE * (size_t)b->elem_off[b->ninst]) == cudaSuccess) {
+  if (room_malloc(c, &b->d_rel, sizeof(float2) * NE * (size_t)b->elem_off[b->ninst]) == cudaSuccess) {
     b->rdf_state = 1;
     return;
   }
@@ -515,6 +515,7 @@ int igapgpu_batch_init(igapgpu_t *out, int ninst, const igapgpu_mesh_desc *meshe
   for (int i = 0; i < ninst; i++) {
     Context *s = new_context(meshes + i, phys + i, bcs + i, nquad);
     s->sub = true;
+    s->owner = c;
     s->stream = c->stream;
     s->geo_mode = c->geo_mode;
     b->subs.push_back(s);

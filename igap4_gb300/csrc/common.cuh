@@ -181,7 +181,8 @@ struct Context {
   int exact_state = -1;        // -1 not decided, 0 off, 1 on
   int *d_xerr = nullptr;       // their kernel's error words: [0] its last launch, [1] any launch not reported yet
   bool exact_ran = false;      // a launch whose word [1] has not been read yet
-  bool exact_captured = false; // the kernel is in a graph of the user's: any synchronisation reads word [1]
+  int async_code = 0;          // word [1] of caches that were released before it was reported
+  bool user_captured = false;  // the caches are in a graph of the user's: never released, word [1] read at any synchronisation
   double *d_dens = nullptr;    // per-element density sums + result (igapgpu_density, lazy)
   int *d_dsparse = nullptr;    // sparse constant tangent: dptr | dcol | sptr | sl
   double *d_dval = nullptr;
@@ -219,6 +220,7 @@ struct Context {
   // batched instances (batch.cu): this context is then their block-diagonal union
   Batch *batch = nullptr;
   bool sub = false;  // an instance of a batch (no matrix or state of its own)
+  Context *owner = nullptr;    // the batch of an instance
   int geo_mode = -1;  // geometry cache: -1 by free memory, 0 none, 1 FP64, 2 FP64 + FP32
   std::vector<int64_t> h_rowptr;  // host CSR offsets (kept for instances of a batch)
   // element-kernel timing (igapgpu_profile)
@@ -288,6 +290,21 @@ struct RelaxedCapture {
   RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
   ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
+// gather.cu: caches that the assembly builds for itself at its first call (slices,
+// element buffers, derivative maps).  One is built when it takes at most a
+// quarter of the free memory and leaves 4 GB, and all of them go when another
+// allocation of the context needs the room; the next assembly decides again.
+bool cache_fits(size_t bytes);
+void note_user_capture(Context *c);
+bool release_caches(Context *c);
+// free device memory, after releasing the caches if that is less than `need`
+int free_memory(Context *c, size_t need, size_t *freeb);
+cudaError_t room_malloc_bytes(Context *c, void **p, size_t bytes);
+template <typename T>
+cudaError_t room_malloc(Context *c, T **p, size_t bytes)
+{
+  return room_malloc_bytes(c, (void **)p, bytes);
+}
 // after a synchronisation: the error word of asynchronous kernels with bounded waits
 int check_async_error(Context *c);
 
@@ -393,6 +410,7 @@ int ksp_gmres_graph(Context *c, const double *b, double *x, const igapgpu_solver
                     double *rnorm);
 int assembly_graph(Context *c, bool do_res, bool do_tan);
 void graph_release(Context *c);
+void assembly_graphs_release(Context *c);
 
 }  // namespace igap
 

@@ -537,13 +537,19 @@ bool stream_capturing(const Context *c)
 
 int check_async_error(Context *c)
 {
-  if (!c->exact_ran && !c->exact_captured) return IGAPGPU_OK;
-  c->exact_ran = false;
-  int herr = 0;
-  IGAP_CUDA(cudaMemcpyAsync(&herr, c->d_xerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  IGAP_CUDA(cudaStreamSynchronize(c->stream));
+  int herr = c->async_code;
+  c->async_code = 0;
+  if (c->exact_state == 1 && (c->exact_ran || c->user_captured)) {
+    c->exact_ran = false;
+    int word = 0;
+    IGAP_CUDA(cudaMemcpyAsync(&word, c->d_xerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    IGAP_CUDA(cudaStreamSynchronize(c->stream));
+    if (word) {
+      IGAP_CUDA(cudaMemsetAsync(c->d_xerr + 1, 0, sizeof(int), c->stream));
+      herr = word;
+    }
+  }
   if (!herr) return IGAPGPU_OK;
-  IGAP_CUDA(cudaMemsetAsync(c->d_xerr + 1, 0, sizeof(int), c->stream));
   set_error("tensor-core assembly: a bounded mbarrier wait expired (code %d)", herr);
   return IGAPGPU_ERR_TIMEOUT;
 }

@@ -412,7 +412,7 @@ extern "C" int igapgpu_density(igapgpu_t c, double *HH, int *ndensity)
   }
   const int nd = c->law == IGAPGPU_LAW_GRADELAST ? 13 : 2;
   if (!c->d_dens) {
-    cudaError_t e = cudaMalloc(&c->d_dens, sizeof(double) * ((size_t)c->nelem_total * nd + MAXD + 1));
+    cudaError_t e = room_malloc(c, &c->d_dens, sizeof(double) * ((size_t)c->nelem_total * nd + MAXD + 1));
     if (e != cudaSuccess) {
       cudaGetLastError();
       c->d_dens = nullptr;
@@ -485,7 +485,7 @@ extern "C" int igapgpu_sample_field(igapgpu_t c, int nppe, double *field, double
     if (host[i]) tot += len[i];
   }
   double *buf = nullptr;
-  cudaError_t e = cudaMalloc(&buf, sizeof(double) * tot);
+  cudaError_t e = room_malloc(c, &buf, sizeof(double) * tot);
   if (e != cudaSuccess) {
     cudaGetLastError();
     set_error("sample_field: cudaMalloc of %zu bytes failed: %s", sizeof(double) * tot, cudaGetErrorString(e));

@@ -313,21 +313,77 @@ int launch_residual_gather(Context *c, double *RR, int parts, const int *err)
   return IGAPGPU_OK;
 }
 
-// Allocated at the first use outside a capture; a buffer that would leave less
-// than 4 GB free is not, and the colour launches stay in use (also with
+bool cache_fits(size_t bytes)
+{
+  size_t freeb = 0, totb = 0;
+  return cudaMemGetInfo(&freeb, &totb) == cudaSuccess && bytes <= freeb / 4 && bytes + ((size_t)4 << 30) <= freeb;
+}
+
+void note_user_capture(Context *c)
+{
+  if (!c->user_captured && !c->capturing && stream_capturing(c)) c->user_captured = true;
+}
+
+bool release_caches(Context *c)
+{
+  if (c->user_captured || stream_capturing(c)) return false;
+  void **bufs[] = {(void **)&c->d_ebuf, (void **)&c->d_rbuf, (void **)&c->d_fbuf, (void **)&c->d_sft, &c->d_xops};
+  bool any = false;
+  for (void **p : bufs) any = any || *p;
+  if (!any) return false;
+  int word = 0;
+  if (cudaStreamSynchronize(c->stream) != cudaSuccess) return false;
+  if (c->exact_state == 1 && c->exact_ran &&
+      cudaMemcpy(&word, c->d_xerr + 1, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess && word)
+    c->async_code = word;
+  assembly_graphs_release(c);  // they hold the pointers
+  for (void **p : bufs) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+  c->d_xrow = nullptr;
+  c->d_xexp = nullptr;
+  c->d_xerr = nullptr;
+  c->exact_ran = false;
+  c->ebuf_state = c->rbuf_state = c->fbuf_state = c->sf_state = c->exact_state = -1;
+  return true;
+}
+
+int free_memory(Context *c, size_t need, size_t *freeb)
+{
+  size_t totb = 0;
+  IGAP_CUDA(cudaMemGetInfo(freeb, &totb));
+  if (*freeb < need && release_caches(c->owner ? c->owner : c)) IGAP_CUDA(cudaMemGetInfo(freeb, &totb));
+  return IGAPGPU_OK;
+}
+
+cudaError_t room_malloc_bytes(Context *c, void **p, size_t bytes)
+{
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (release_caches(c->owner ? c->owner : c)) e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
+// Allocated at the first use outside a capture, when it fits beside what else
+// the context may need; else the colour launches stay in use (also with
 // IGAPGPU_ELEMENT_BUFFERS=0).
 template <typename T>
 static bool ensure_buffer(Context *c, T **p, int *state, size_t per_element)
 {
-  if (*state >= 0) return *state == 1;
+  if (*state >= 0) {
+    if (*state == 1) note_user_capture(c);
+    return *state == 1;
+  }
   if (stream_capturing(c)) return false;
   RelaxedCapture relaxed;
   *state = 0;
   const char *env = getenv("IGAPGPU_ELEMENT_BUFFERS");
   if (env && env[0] == '0') return false;
   const size_t bytes = sizeof(T) * per_element * (size_t)c->nelem_total;
-  size_t freeb = 0, totb = 0;
-  if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess || bytes + ((size_t)4 << 30) > freeb) return false;
+  if (!cache_fits(bytes)) return false;
   if (cudaMalloc(p, bytes) != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;

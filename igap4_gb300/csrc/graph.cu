@@ -271,14 +271,19 @@ static void free_graph(GraphWork *gw)
   delete gw;
 }
 
-void graph_release(Context *c)
+void assembly_graphs_release(Context *c)
 {
-  free_graph(c->gmres_graph);
-  c->gmres_graph = nullptr;
   for (int i = 0; i < 12; i++) {
     if (c->asm_graph[i]) cudaGraphExecDestroy(c->asm_graph[i]);
     c->asm_graph[i] = nullptr;
   }
+}
+
+void graph_release(Context *c)
+{
+  free_graph(c->gmres_graph);
+  c->gmres_graph = nullptr;
+  assembly_graphs_release(c);
 }
 
 
@@ -296,7 +301,7 @@ static int build_gmres_graph(Context *c, int m, int pc, int orth)
   c->gmres_graph = nullptr;
   GraphWork *gw = new GraphWork();
   const int64_t n = c->ndof;
-  auto alloc = [&](double **p, size_t cnt) { return cudaMalloc((void **)p, sizeof(double) * cnt); };
+  auto alloc = [&](double **p, size_t cnt) { return room_malloc(c, p, sizeof(double) * cnt); };
   if (alloc(&gw->b, n) || alloc(&gw->x, n) || alloc(&gw->r, n) || alloc(&gw->w, n) ||
       alloc(&gw->V, (size_t)(m + 1) * n) || alloc(&gw->Z, (size_t)m * n) ||
       alloc(&gw->H, (size_t)(m + 1) * m) || alloc(&gw->cs, m) || alloc(&gw->sn, m) ||

@@ -175,9 +175,9 @@ static int dev_dot(Context *c, const double *a, const double *b, double *out, in
 static int ensure_krylov(Context *c, int restart)
 {
   if (c->d_work == nullptr) {
-    if (cudaMalloc(&c->d_work, sizeof(double) * 4 * c->ndof) != cudaSuccess ||
-        cudaMalloc(&c->d_diag, sizeof(double) * c->ndof) != cudaSuccess ||
-        cudaMalloc(&c->d_bdiag, sizeof(double) * 3 * c->ndof) != cudaSuccess) {
+    if (room_malloc(c, &c->d_work, sizeof(double) * 4 * c->ndof) != cudaSuccess ||
+        room_malloc(c, &c->d_diag, sizeof(double) * c->ndof) != cudaSuccess ||
+        room_malloc(c, &c->d_bdiag, sizeof(double) * 3 * c->ndof) != cudaSuccess) {
       cudaGetLastError();
       set_error("Krylov workspace allocation failed");
       return IGAPGPU_ERR_NOMEM;
@@ -189,7 +189,7 @@ static int ensure_krylov(Context *c, int restart)
     c->d_red = nullptr;
     c->h_red = nullptr;
     c->red_cap = 0;
-    if (cudaMalloc(&c->d_red, sizeof(double) * (restart + 8)) != cudaSuccess ||
+    if (room_malloc(c, &c->d_red, sizeof(double) * (restart + 8)) != cudaSuccess ||
         cudaMallocHost(&c->h_red, sizeof(double) * (restart + 8)) != cudaSuccess) {
       cudaGetLastError();
       set_error("reduction scratch allocation failed");
@@ -201,8 +201,8 @@ static int ensure_krylov(Context *c, int restart)
     if (c->d_V) cudaFree(c->d_V);
     if (c->d_Z) cudaFree(c->d_Z);
     c->d_V = c->d_Z = nullptr;
-    if (cudaMalloc(&c->d_V, sizeof(double) * (size_t)(restart + 1) * c->ndof) != cudaSuccess ||
-        cudaMalloc(&c->d_Z, sizeof(double) * (size_t)restart * c->ndof) != cudaSuccess) {
+    if (room_malloc(c, &c->d_V, sizeof(double) * (size_t)(restart + 1) * c->ndof) != cudaSuccess ||
+        room_malloc(c, &c->d_Z, sizeof(double) * (size_t)restart * c->ndof) != cudaSuccess) {
       cudaGetLastError();
       c->ksp_restart = 0;
       set_error("GMRES basis of restart %d does not fit", restart);
@@ -249,7 +249,7 @@ int ensure_cblock(Context *c, int64_t ncell)
     set_error("cell-block Jacobi (pc = 3) needs a single lattice; a batch takes pc 0, 1 or 2");
     return IGAPGPU_ERR_ARG;
   }
-  if (!c->d_cinv && cudaMalloc(&c->d_cinv, sizeof(double) * (size_t)ncell * CBS * CBS) != cudaSuccess) {
+  if (!c->d_cinv && room_malloc(c, &c->d_cinv, sizeof(double) * (size_t)ncell * CBS * CBS) != cudaSuccess) {
     cudaGetLastError();
     c->d_cinv = nullptr;
     set_error("cell-block Jacobi: allocation of %lld blocks failed", (long long)ncell);
@@ -307,7 +307,7 @@ int setup_pc(Context *c, int pc, const double **pcd)
     count_launch();
     *pcd = c->d_cinv;
   } else if (pc == 4) {  // restricted additive Schwarz
-    if (!c->d_asmz && cudaMalloc(&c->d_asmz, sizeof(float) * (size_t)ncell * AS_NC * AS_N) != cudaSuccess) {
+    if (!c->d_asmz && room_malloc(c, &c->d_asmz, sizeof(float) * (size_t)ncell * AS_NC * AS_N) != cudaSuccess) {
       cudaGetLastError();
       c->d_asmz = nullptr;
       set_error("additive Schwarz: allocation of %lld subdomains failed", (long long)ncell);

@@ -646,7 +646,7 @@ static int ensure_cycle(Context *c, int m)
   const char *env = getenv("IGAPGPU_GMRES_CYCLE");
   if (env && atoi(env) > 0) grid = atoi(env);
   const size_t cnt = (size_t)(m + 1) * m + (size_t)(m + 1) + 2 * (size_t)(m + 1) * CY_RMAX + 3 * (size_t)grid;
-  if (cudaMalloc(&cw->buf, sizeof(double) * cnt) != cudaSuccess || cudaMalloc(&cw->ctl, CY_CTL_BYTES) != cudaSuccess ||
+  if (room_malloc(c, &cw->buf, sizeof(double) * cnt) != cudaSuccess || room_malloc(c, &cw->ctl, CY_CTL_BYTES) != cudaSuccess ||
       cudaMallocHost(&cw->h_st, CY_CTL_BYTES) != cudaSuccess) {
     cudaGetLastError();
     cycle_release(c);

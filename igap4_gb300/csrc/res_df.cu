@@ -704,8 +704,9 @@ int ensure_res_pairs(Context *c)
     const size_t lbytes = (size_t)c->nelem_total * npts * 64 * sizeof(double);
     const size_t rbytes = (size_t)c->nelem_total * NE * sizeof(float2);
     const size_t ubytes = (size_t)ncomb * c->ndof * sizeof(float2);
-    size_t freeb = 0, totb = 0;
-    IGAP_CUDA(cudaMemGetInfo(&freeb, &totb));
+    size_t freeb = 0;
+    int r = free_memory(c, 2 * (lbytes + rbytes + ubytes + ((size_t)4 << 30)), &freeb);
+    if (r) return r;
     if (lbytes + rbytes + ubytes + ((size_t)4 << 30) > freeb / 2) return IGAPGPU_OK;
     if (cudaMalloc(&c->d_lin, lbytes) != cudaSuccess || cudaMalloc(&c->d_rel, rbytes) != cudaSuccess ||
         cudaMalloc(&c->d_upair, ubytes) != cudaSuccess) {
@@ -724,8 +725,9 @@ int ensure_res_pairs(Context *c)
   const size_t bytes = (size_t)c->nelem_total * npts * RP_V * sizeof(float2);
   const size_t rbytes = (size_t)c->nelem_total * NE * sizeof(float2);
   const size_t ubytes = (size_t)c->ndof * sizeof(float2);
-  size_t freeb = 0, totb = 0;
-  IGAP_CUDA(cudaMemGetInfo(&freeb, &totb));
+  size_t freeb = 0;
+  int r = free_memory(c, bytes + rbytes + ubytes + ((size_t)4 << 30), &freeb);
+  if (r) return r;
   if (bytes + rbytes + ubytes + ((size_t)4 << 30) > freeb) return IGAPGPU_OK;
   if (cudaMalloc(&c->d_rpc, bytes) != cudaSuccess || cudaMalloc(&c->d_rel, rbytes) != cudaSuccess ||
       cudaMalloc(&c->d_upair, ubytes) != cudaSuccess) {

@@ -292,13 +292,15 @@ __global__ void __launch_bounds__(SF_THREADS, 1)
 bool ensure_sumfac(Context *c, const DevLaw &L)
 {
   if (!L.preD || c->nquad != 4 || c->porder != P || c->batch) return false;
-  if (c->sf_state >= 0) return c->sf_state == 1;
+  if (c->sf_state >= 0) {
+    if (c->sf_state == 1) note_user_capture(c);
+    return c->sf_state == 1;
+  }
   if (stream_capturing(c)) return false;
   RelaxedCapture relaxed;
   c->sf_state = 0;
   const size_t bytes = sizeof(double) * SF_NT * SF_Q * (size_t)c->nelem_total;
-  size_t freeb = 0, totb = 0;
-  if (!ensure_ebuf(c) || cudaMemGetInfo(&freeb, &totb) != cudaSuccess || bytes + ((size_t)4 << 30) > freeb) return false;
+  if (!ensure_ebuf(c) || !cache_fits(bytes)) return false;
   if (cudaMalloc(&c->d_sft, bytes) != cudaSuccess) {
     cudaGetLastError();
     c->d_sft = nullptr;

@@ -648,14 +648,16 @@ static void exact_free(Context *c)
 // Builds the slices at the first call that wants them (outside a capture) and
 // says whether the tensor-core path is available: the linear law, at most 64
 // Gauss points, the FP64 geometry cache of every instance, memory for the slices
-// (275 KB an element) with 4 GB to spare, and digits within the exactness
-// bound.  The tangent needs the element buffers as well (ensure_ebuf).  One
+// (275 KB an element, cache_fits), and digits within the exactness bound.  The tangent needs the element buffers as well (ensure_ebuf).  One
 // allocation, and the residual buffer's beside the operand kernel: an allocation
 // takes 70 us and 100 to 150 us a GB.
 // IGAPGPU_TC_EXACT=0 keeps the FP64 kernel.
 bool ensure_exact(Context *c)
 {
-  if (c->exact_state >= 0) return c->exact_state == 1;
+  if (c->exact_state >= 0) {
+    if (c->exact_state == 1) note_user_capture(c);
+    return c->exact_state == 1;
+  }
   if (stream_capturing(c)) return false;
   RelaxedCapture relaxed;
   c->exact_state = 0;
@@ -676,10 +678,7 @@ bool ensure_exact(Context *c)
   // slices, rows 80, exponents, error words and the exactness flag
   const size_t bytes = nel * nchunk * XS_CH_BYTES, rbytes = nel * nchunk * 32 * sizeof(double),
                ebytes = nel * XS_EXP * sizeof(short), total = bytes + rbytes + ebytes + 3 * sizeof(int);
-  size_t freeb = 0, totb = 0;
-  if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess ||
-      total + nel * NE * sizeof(double) + ((size_t)4 << 30) > freeb)
-    return false;
+  if (!cache_fits(total + nel * NE * sizeof(double))) return false;
   bool ok = cudaMalloc(&c->d_xops, total) == cudaSuccess;
   if (ok) {
     unsigned char *p = (unsigned char *)c->d_xops + bytes;
@@ -768,7 +767,6 @@ int launch_exact(Context *c, double *RR, double *vals)
     c->prof_elements[0] += c->nelem_total;
   }
   c->exact_ran = true;
-  if (!c->capturing && stream_capturing(c)) c->exact_captured = true;
   const int r = RR ? launch_residual_gather(c, RR, 1, c->d_xerr) : IGAPGPU_OK;
   return r || !vals ? r : launch_tangent_gather(c, vals, c->d_xerr);
 }

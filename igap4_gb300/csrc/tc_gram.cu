@@ -996,8 +996,9 @@ int ensure_gram_operands(Context *c)
   if (env && env[0] == '0') return IGAPGPU_OK;
   const int npts = c->nquad * c->nquad * c->nquad, nchunk = (npts + PW - 1) / PW;
   const size_t bytes = (size_t)c->nelem_total * nchunk * S_CH_BYTES;
-  size_t freeb = 0, totb = 0;
-  IGAP_CUDA(cudaMemGetInfo(&freeb, &totb));
+  size_t freeb = 0;
+  int r = free_memory(c, bytes + ((size_t)4 << 30), &freeb);
+  if (r) return r;
   if (bytes + ((size_t)4 << 30) > freeb) return IGAPGPU_OK;  // the plain Gram kernel stays in use
   if (cudaMalloc(&c->d_gop, bytes) != cudaSuccess) {
     cudaGetLastError();

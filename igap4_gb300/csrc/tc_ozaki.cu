@@ -476,8 +476,9 @@ int ensure_ozaki_operands(Context *c)
   const int npts = c->nquad * c->nquad * c->nquad, nchunk = (npts + PW - 1) / PW;
   const size_t bytes = (size_t)c->nelem_total * nchunk * OZ_CH_BYTES;
   const size_t ebytes = (size_t)c->nelem_total * OZ_EXP;
-  size_t freeb = 0, totb = 0;
-  IGAP_CUDA(cudaMemGetInfo(&freeb, &totb));
+  size_t freeb = 0;
+  int r = free_memory(c, bytes + ebytes + ((size_t)4 << 30), &freeb);
+  if (r) return r;
   if (bytes + ebytes + ((size_t)4 << 30) > freeb) return IGAPGPU_OK;
   int *d_bad = nullptr;
   if (cudaMalloc(&c->d_oz, bytes) != cudaSuccess || cudaMalloc(&c->d_ozexp, ebytes) != cudaSuccess ||

@@ -207,7 +207,15 @@ int igapgpu_residual(igapgpu_t ctx, const double *U, double *RR);
 /* Tangent_iga (src/assmcore_iga.c:507-858): CSR values of dRR/dU in the
  * pattern order, Dirichlet rows and columns zeroed with unit diagonal
  * (MatZeroRowsColumns).  vals may be NULL: the context's own matrix (used by
- * igapgpu_matmult / the Newton solver) is assembled.  U may be NULL. */
+ * igapgpu_matmult / the Newton solver) is assembled.  U may be NULL.
+ *
+ * Device memory: the first FP64 residual (64 points) or tangent of the linear
+ * law builds slices of its Gram operands (up to 275 KB an element;
+ * IGAPGPU_TC_EXACT=0: none), a tangent through element buffers 27 KB an element
+ * more (IGAPGPU_ELEMENT_BUFFERS=0: none), the reference's laws' FP64 tangent
+ * 37 KB of derivative maps.  Each is built when it takes at most a quarter of the
+ * free memory and leaves 4 GB; they are given up when another allocation of the
+ * context needs the room, unless a graph of the caller's holds them. */
 int igapgpu_tangent(igapgpu_t ctx, const double *U, double *vals);
 /* Residual and tangent in one fused element pass (same results as the two
  * calls above).  RR / vals may be NULL as above. */
