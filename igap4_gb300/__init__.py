@@ -509,7 +509,8 @@ class BatchAssembly(Assembly):
     def autotune(self, reps=2, frac=0.1):
         """Time the candidate schedules, keep the fastest; returns
         (schedule dict, best FP64-kernel ms, best tensor-core-kernel ms) on
-        the timed queue prefix."""
+        the timed queue prefix (FP64 work of a kernel without a schedule: on
+        the whole queue)."""
         s = BatchSchedule()
         m64, mtc = ctypes.c_double(), ctypes.c_double()
         _check(lib().igapgpu_batch_autotune(self.h, int(reps), float(frac), ctypes.byref(s),

@@ -708,8 +708,13 @@ int igapgpu_batch_autotune(igapgpu_t c, int reps, double frac, igapgpu_batch_sch
   if (!(frac > 0.0) || frac > 1.0) frac = 1.0;
   Batch *b = c->batch;
   const bool split = c->prec == IGAPGPU_PREC_SPLIT;
-  // the FP64 kernel computes the residual (and, in FP64 mode, the tangent)
-  const bool tan64 = !split && !ensure_exact(c);
+  // The queue's FP64 kernel computes the residual (and, in FP64 mode, the
+  // tangent), but for what kernels without a schedule take from the whole queue:
+  // in FP64 mode the exact kernel the tangent and the residual beside it (alone
+  // as well with 64 points), in split mode the pair residual.
+  const bool exact = !split && ensure_exact(c) && ensure_ebuf(c);
+  const bool tan64 = !split && !exact;
+  const bool queue64 = split ? !batch_res_df(c) : !(exact && exact_residual(c, false));
   int occ = 1;
   int r = element_batch_occupancy(c->law, true, tan64, &occ);
   if (r) return r;
@@ -722,11 +727,12 @@ int igapgpu_batch_autotune(igapgpu_t c, int reps, double frac, igapgpu_batch_sch
   const bool prof = c->prof;
   c->prof = false;
   auto time_one = [&](int which, double *ms) -> int {
-    const int64_t n = std::max<int64_t>(1, (int64_t)(frac * (double)b->nitems));
+    const bool queue = which == 2 || queue64;
+    const int64_t n = queue ? std::max<int64_t>(1, (int64_t)(frac * (double)b->nitems)) : b->nitems;
     float tmin = 1e30f;
     for (int k = 0; k < reps; k++) {
       IGAP_CUDA(cudaEventRecord(e0, c->stream));
-      int rr = batch_kernels(c, which == 1, which == 1 ? tan64 : true, c->d_RR, c->d_vals, n, which);
+      int rr = batch_kernels(c, which == 1, which == 1 ? tan64 || !queue : true, c->d_RR, c->d_vals, n, which);
       if (rr) return rr;
       IGAP_CUDA(cudaEventRecord(e1, c->stream));
       IGAP_CUDA(cudaEventSynchronize(e1));
@@ -738,15 +744,17 @@ int igapgpu_batch_autotune(igapgpu_t c, int reps, double frac, igapgpu_batch_sch
     return IGAPGPU_OK;
   };
   igapgpu_batch_schedule keep = b->sched, bestS = b->sched;
-  double best_total = 1e300, best64 = 0.0, besttc = 0.0;
+  double best_total = 1e300, best64 = 0.0, besttc = 0.0, fixed64 = 0.0;
+  if (!queue64) r = time_one(1, &fixed64);
   for (int order = 0; order < 2 && r == 0; order++) {
+    if (!queue64 && !split && order != keep.order) continue;  // nothing to choose
     igapgpu_batch_schedule s = b->sched;
     s.order = order;
     if ((r = build_items(c, order))) break;
-    double t64 = 1e300, ttc = split ? 1e300 : 0.0;
-    int g64 = 1, c64 = 1, gtc = 1;
+    double t64 = queue64 ? 1e300 : fixed64, ttc = split ? 1e300 : 0.0;
+    int g64 = queue64 ? 1 : keep.grab_fp64, c64 = queue64 ? 1 : keep.ctas_per_sm_fp64, gtc = split ? 1 : keep.grab_tc;
     for (int g : grabs)
-      for (int k = 1; k <= occ && r == 0; k++) {
+      for (int k = 1; queue64 && k <= occ && r == 0; k++) {
         b->sched.grab_fp64 = g;
         b->sched.ctas_per_sm_fp64 = k;
         double ms = 0.0;

@@ -336,7 +336,10 @@ int igapgpu_batch_get_schedule(igapgpu_t ctx, igapgpu_batch_schedule *s);
 /* Times candidate schedules of both kernels on the current state (each
  * candidate runs `reps` times on a prefix of `frac` of the work queue), keeps
  * the fastest and returns it; ms_fp64 / ms_tc: best time of each kernel on the
- * prefix (may be NULL).  Leaves the context's residual and matrix invalid. */
+ * prefix (may be NULL).  Where a kernel without a schedule takes the FP64 work
+ * (the linear law's FP64 assembly with 64 points, the split mode's residual),
+ * ms_fp64 is that kernel's time on the whole queue and the FP64 entries of the
+ * schedule stay.  Leaves the context's residual and matrix invalid. */
 int igapgpu_batch_autotune(igapgpu_t ctx, int reps, double frac, igapgpu_batch_schedule *best,
                            double *ms_fp64, double *ms_tc);
 
