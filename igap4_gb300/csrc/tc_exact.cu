@@ -30,10 +30,14 @@
 //    the entry (80, 80) is a 256-term FP64 dot product of the row itself.
 // Residual: exact for constants as the quadrature loop is not (the state enters
 // as differences from the element's middle function: a translation of 5 beside
-// displacements of 1e-3 costs the quadrature loop 2e-13).
-// Measured: against 64-bit reference sums the error is the FP64 kernel's (7e-16
-// at 16x4x4, 3e-15 at 63x17x15 distorted, both from the geometry; the two
-// tangents differ by 2e-16).  Residual and tangent at 16x4x4 7.9 ms (FP64 kernel,
+// displacements of 1e-3 costs the quadrature loop 2e-13, this 1e-15).
+// Measured: against 64-bit reference sums the tangent's error is the FP64 kernel's
+// (7e-16 at 16x4x4, 3e-15 at 63x17x15 distorted, both from the geometry; the two
+// tangents differ by 2e-16).  The residual's error against long double is the
+// quadrature loop's within 10 % on random, sinusoidal and most affine states (1e-15 to
+// 4e-15 of |F|); on pure bending, whose Hessian terms cancel, the rounding of the
+// rows of S adds to the geometry's and it is 1.2 to 1.7 times as large (1.4e-15 to
+// 7e-15 there, 2e-15 to 1.2e-14 here; affine states at length scale 0.2 up to 1.3).  Residual and tangent at 16x4x4 7.9 ms (FP64 kernel,
 // colour by colour) -> 76 us, 63x17x15 36.7 -> 2.05 ms.  Per element and SM 31 k
 // clocks, 27 k of them MMAs (73 clocks each: shared-memory operand reads).
 //
