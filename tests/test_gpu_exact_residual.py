@@ -1,7 +1,8 @@
 """FP64 residual of the linear law from the element matrices (csrc/tc_exact.cu)
 against the quadrature kernel: smooth, affine, bending and translated states,
 alone and beside the tangent, rational weights, several elements per block and
-partial chunks."""
+partial chunks; and the context whose digits leave the exactness bound, which
+keeps the quadrature kernel and its bits."""
 import numpy as np
 import pytest
 
@@ -58,3 +59,32 @@ def test_translations_drop_out(monkeypatch):
     A, X = make(monkeypatch, "1", (9, 4, 5), perturb=True, clamp=False)
     U = np.round(state("random", X, np.random.default_rng(0)) * 0.1 * 2.0 ** 40) / 2.0 ** 40
     np.testing.assert_array_equal(A.residual(U + 5.0), A.residual(U))
+
+
+def both_routes(monkeypatch, nelem, ell):
+    out = []
+    for flag in ("1", "0"):
+        A, X = make(monkeypatch, flag, nelem, par=(1.0, 1.0, ell))
+        U = state("random", X, np.random.default_rng(0))
+        RR, K = np.zeros(A.ndof), np.zeros(A.nnz)
+        A.assemble(U, RR, K)
+        out.append((A.residual(U), A.tangent(U), RR, K))
+        A.close()
+    return zip(*out)
+
+
+# regular meshes whose largest digit norms, taken together over an element's rows,
+# exceed what sums exactly in FP32, and no pair of rows does: still the tensor-core
+# route, with its accuracy (4e-15: both sides round 64 x 36 products a pair in 53 bits)
+@pytest.mark.parametrize("nelem,ell", [((16, 4, 5), 0.1778), ((4, 4, 6), 0.1857), ((7, 6, 5), 0.1828),
+                                       ((30, 3, 4), 0.1044), ((24, 13, 24), 0.1755)])
+def test_bound_holds_entry_by_entry(monkeypatch, nelem, ell):
+    for a, b in both_routes(monkeypatch, nelem, ell):
+        assert not np.array_equal(a, b)
+        assert np.linalg.norm(a - b) <= 4e-15 * np.linalg.norm(b)
+
+
+def test_digits_beyond_the_bound_keep_the_quadrature_kernel(monkeypatch):
+    """A mesh where a pair of rows does exceed it: the FP64 kernel and its bits."""
+    for a, b in both_routes(monkeypatch, (20, 10, 3), 0.09793557511207801):
+        np.testing.assert_array_equal(a, b)
