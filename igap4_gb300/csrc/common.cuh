@@ -379,7 +379,7 @@ int dev_diff_norm2(Context *c, const double *b, double *w, double *out);
 // preconditioner data of the context matrix for the cycle kernel
 int setup_pc(Context *c, int pc, const double **pcd);
 // krylov_cycle.cu: GMRES restart cycles as one cooperative kernel each
-bool cycle_applies(const Context *c, int m);
+bool cycle_applies(const Context *c, int m, int orth);
 constexpr int CYCLE_UNFIT = 1;  // ksp_cycles: the grid does not fit the device, nothing was done
 int ksp_cycles(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int m, int pc, const double *pcd,
                double *V, double *Z, double *w, double *wd, bool cap, int *its, double *rnorm);

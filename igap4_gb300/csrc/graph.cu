@@ -409,7 +409,7 @@ int ksp_gmres_graph(Context *c, const double *b, double *x, const igapgpu_solver
     set_error("block preconditioners (pc = 3, 4) need a single lattice; a batch takes pc 0, 1 or 2");
     return IGAPGPU_ERR_ARG;
   }
-  if (cycle_applies(c, m)) {
+  if (cycle_applies(c, m, orth)) {
     const double *pcd;
     int r = setup_pc(c, pc, &pcd);
     if (r) return r;

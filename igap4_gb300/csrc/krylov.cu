@@ -322,7 +322,8 @@ int setup_pc(Context *c, int pc, const double **pcd)
 
 // Right-preconditioned GMRES(m) with MGS, x in/out (device), b device.  The
 // cycle kernel (krylov_cycle.cu) takes it unless the restart is too long for
-// its shared memory or its grid does not fit; then one launch per vector operation.
+// its shared memory or short for the size, or its grid does not fit; then one
+// launch per vector operation.
 int ksp_gmres(Context *c, const double *b, double *x, const igapgpu_solver_opts *o, int *its_out,
               double *rnorm_out)
 {
@@ -341,7 +342,7 @@ int ksp_gmres(Context *c, const double *b, double *x, const igapgpu_solver_opts 
   const int pc = o->pc >= 1 && o->pc <= 4 ? o->pc : 0;
   const double *pcd;
   if ((r = setup_pc(c, pc, &pcd))) return r;
-  if (cycle_applies(c, m)) {
+  if (cycle_applies(c, m, 0)) {  // always modified Gram-Schmidt here
     r = ksp_cycles(c, b, x, o, m, pc, pcd, V, Z, w, c->d_work + 3 * n, true, its_out, rnorm_out);
     if (r != CYCLE_UNFIT) return r;
   }

@@ -664,14 +664,32 @@ static size_t cycle_smem(int m) { return sizeof(CycleSmem) + sizeof(double) * ((
 // multiply is in FP64 (IGAPGPU_SPMV_DF keeps the separate kernels), and the grid
 // can be resident at once (a process limited to part of the SMs falls back, or
 // names its blocks: IGAPGPU_GMRES_CYCLE=blocks; 0 keeps the separate kernels).
-// The size draws no line: against the separate launches it is 26 times faster
-// at 32x8x8 (restart 100), 8.3 at 64x16x16, and where the matrix is ten times L2
-// (128x32x32, 1.2 GB) 1.2 times with restart 10, 1.5 with 30, 2.5 with 100, 3.3
-// with 200 (Jacobi; 1.04 with the Schwarz preconditioner, whose own data bound it).
-bool cycle_applies(const Context *c, int m)
+//
+// Size and restart: the cycle saves launches and passes over the basis, both
+// growing with the step number, and loses on the multiply once the matrix is far
+// beyond L2 (every stage waits for the slowest SM, where the separate multiply's
+// blocks are handed out as SMs come free).  Separate / cycle, ms:
+//   one lattice   64x16x16 (64 k rows)    restart 5   1.02 /  0.68, 30  10.6 /  2.9, 100   88 /  11
+//                 128x32x32 (451 k)                   3.27 /  3.01,     21.5 / 13.9,      132 /  51
+//                 192x48x48 (1.46 M)                  8.90 /  8.99,     48.1 / 42.6,      227 / 157
+//                 256x64x64 (3.37 M)      10  34.5 / 36.3, 20  66.3 / 67.6, 30  101 / 99, 100  431 / 364
+//   batches       88 k rows               faster at every restart
+//   (generic      366 k                   5   2.39 /  2.33, 30  16.6 / 10.9
+//    multiply)    821 k, graphs           10  saves -0.5 of 6, 30  1.6 of 23
+//                 4.56 M                  10  37.7 / 45.1, 60  249 / 256, 100  483 / 461
+//   batches with CGS2 (graphs, whose two block passes are cheap):
+//                 366 k                   10 -0.16 of 3.8, 30 -0.05 of 11, 60  0.7 of 24
+//                 821 k                   30 -1.5 of 21, 60 -1.4 of 48
+// so the shortest restart it takes grows with the rows.  IGAPGPU_GMRES_CYCLE=blocks
+// overrides the line.
+bool cycle_applies(const Context *c, int m, int orth)
 {
   const char *env = getenv("IGAPGPU_GMRES_CYCLE");
-  return m <= CY_MAX_RESTART && !spmv_df(c) && !c->cycle_unfit && !(env && env[0] == '0');
+  if (m > CY_MAX_RESTART || spmv_df(c) || c->cycle_unfit || (env && env[0] == '0')) return false;
+  if (c->ndof < 200000 || (env && atoi(env) > 0)) return true;
+  const double rows = 1e-6 * (double)c->ndof;
+  const double line = c->batch ? (orth == 1 ? 110.0 * rows : fmin(22.0 * rows, 75.0)) : fmin(3.0 * rows * rows, 75.0);
+  return m >= line;
 }
 
 // GMRES cycles on the context matrix; b, x device vectors, pcd the

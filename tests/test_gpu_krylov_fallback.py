@@ -39,3 +39,32 @@ def test_other_grids_and_separate_launches(monkeypatch, blocks):
         assert np.linalg.norm(U0 - U) <= 1e-8 * np.linalg.norm(U)
     assert n_ref < 20
     assert (n > 1000) == (blocks in ("0", "1000000"))
+
+
+def test_short_restarts_of_large_systems(monkeypatch):
+    """366 k rows in a batch: restarts below the line run as separate launches, the
+    others as cycles, with the same residual norms."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("IGAPGPU_GEOMETRY_CACHE", "0")
+    A = ig.BatchAssembly(ig.batch_instances(24))
+    assert A.ndof > 300_000
+    U = torch.zeros(A.ndof, dtype=torch.float64, device="cuda")
+    b = torch.zeros_like(U)
+    torch.cuda.synchronize()
+    A.residual(U, b)
+    A.tangent_internal(U)
+    A.synchronize()
+    for m, cycle in ((5, False), (20, True)):
+        got = []
+        for blocks in (None, "152"):  # the rule, then the cycle kernel whatever it says
+            monkeypatch.delenv("IGAPGPU_GMRES_CYCLE", raising=False)
+            if blocks:
+                monkeypatch.setenv("IGAPGPU_GMRES_CYCLE", blocks)
+            x = torch.zeros_like(b)
+            torch.cuda.synchronize()
+            n0 = ig.launch_count()
+            its, rn = A.ksp_solve(b, x, ksp_restart=m, ksp_max_it=m, ksp_rtol=1e-30, pc=1)
+            got.append((ig.launch_count() - n0 < 12, rn))
+            assert its == m
+        assert got[0][0] == cycle and got[1][0]
+        assert abs(got[0][1] - got[1][1]) <= 1e-9 * got[0][1]
