@@ -272,8 +272,8 @@ def bench_batched(ig, torch, dev, n, steps, warmup, flush, peaks):
     """Batched uneven instances: n seeded linear-law beams (nx in 8..64,
     ny = nz in 2..16, lambda, mu in [0.5, 2], length scale in [0.02, 0.2]),
     split-precision tangent (one persistent launch) + double-FP32 residual
-    (one launch over every element and a gather per DOF) per assembly; schedule from the autotuner; one Newton step (assembly and
-    GMRES cycles) replayed from CUDA graphs."""
+    (one launch over every element and a gather per DOF) per assembly; schedule from the autotuner; one Newton step (assembly
+    replayed from CUDA graphs, GMRES cycles of one kernel each)."""
     t0 = time.perf_counter()
     insts = ig.batch_instances(n, seed=SEED)
     B = ig.BatchAssembly(insts, law=ig.LAW_LINGRAD)
@@ -311,8 +311,8 @@ def bench_batched(ig, torch, dev, n, steps, warmup, flush, peaks):
     res_ms, res_l, res_e = kinds[0]
     tc_ach = TAN_FLOP_PER_ELEM * tc_e / (tc_ms * 1e-3) / 1e12 if tc_ms > 0 else None
     bf16_peak = peaks.get("bf16_tflops", 1900.0)
-    # one Newton step of the block-diagonal system from zero: assembly, then a
-    # a fixed number of GMRES(100) iterations (Jacobi), replayed from CUDA graphs
+    # one Newton step of the block-diagonal system from zero: assembly (a graph),
+    # then a fixed number of GMRES(100) iterations (Jacobi), a kernel a cycle
     B.set_stream(None)
     Z = torch.zeros(B.ndof, dtype=torch.float64, device=dev)
     kits = 200
@@ -339,7 +339,7 @@ def bench_batched(ig, torch, dev, n, steps, warmup, flush, peaks):
            "value": B.nelem_total / (ms_step * 1e-3), "unit": "elements/s", "ms_per_step": ms_step,
            "step_ms": ms, "steps": steps, "gpu_launches_per_step": launches / steps,
            "tc_kernel_ms_per_step": tc_ms / steps, "residual_kernel_ms_per_step": res_ms / steps,
-           "schedule": sched, "autotune_s": t_tune, "autotune_prefix_ms": {"fp64": t64, "tc": ttc},
+           "schedule": sched, "autotune_s": t_tune, "autotune_ms": {"residual": t64, "tc_prefix": ttc},
            "init_s": t_init,
            "roofline": {"bound": "tensor", "kernel": "tc_tangent_kernel<batch>", "achieved": tc_ach,
                         "peak": bf16_peak, "unit": "TFLOP/s",
@@ -350,7 +350,7 @@ def bench_batched(ig, torch, dev, n, steps, warmup, flush, peaks):
                            "instance_residual_reduction": {"median": float(np.median(red)),
                                                            "max": float(np.max(red))},
                            "options": f"one Newton step from U=0: assembly then {kits} GMRES(100) MGS "
-                                      "iterations with Jacobi, replayed from CUDA graphs"}}
+                                      "iterations with Jacobi, one kernel a cycle"}}
     B.close()
     return out
 
@@ -437,8 +437,8 @@ def bench_transient(ig, torch, nelem, steps, start_steps=200, seed=9001, dt=5e-4
     grows from 1e-6 to order 1); both arms then run the same `steps` steps
     from that state.  Newton: the FP64 law's residual (its inputs and
     projection in double-FP32 arithmetic), tangent on the tensor cores,
-    GMRES(100) with cell-block Jacobi and two-pass classical Gram-Schmidt,
-    replayed from CUDA graphs.  The step time is the wall time of the whole step
+    GMRES(100) with cell-block Jacobi and two-pass classical Gram-Schmidt, one
+    kernel a cycle; assembly from CUDA graphs.  The step time is the wall time of the whole step
     (predictor, acceptance test, Newton)."""
     from igap4_gb300.train_predictor import load_network, transient_problem
     from igap4_gb300.transient import TipLoad, run_transient
@@ -472,7 +472,7 @@ def bench_transient(ig, torch, nelem, steps, start_steps=200, seed=9001, dt=5e-4
                        f"(seed {seed})",
            "tolerance": "Newton |F| <= 1e-8 (residual within 1e-12 of FP64)",
            "solver": "Newton, GMRES(100) rtol 1e-5 with two-pass classical Gram-Schmidt and cell-block "
-                     "Jacobi (pc 3), cycles replayed from CUDA graphs",
+                     "Jacobi (pc 3), one kernel a cycle, assembly replayed from CUDA graphs",
            "plain": summary(plain),
            "warm_steps": {"steps": start_steps, "seconds": t_warm,
                           "all_converged": bool(all(r.converged for r in warm))}}

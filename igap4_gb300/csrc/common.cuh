@@ -353,10 +353,10 @@ bool ensure_exact(Context *c);
 int launch_exact(Context *c, double *RR, double *vals);
 // Whether that kernel gives the residual.  Beside the tangent it costs almost
 // nothing.  Alone, it pays the 23 products of K_e for 6,561 FMA, where the
-// quadrature takes 1,458 a point: with 64 points it is the faster one (1.79
-// against 4.04 ms at 64x16x16, and 4.82 against 5.28 ms with the first call's
-// set-up of the slices), with 8 the slower (1.33 against 0.61 ms), and with 27
-// the set-up of a first call costs more than the 0.56 ms saved (3.5 against 2.1 ms).
+// quadrature takes 1,458 a point.  At 64x16x16: with 64 points 1.79 against 4.04
+// ms (a first call, with its set-up of the slices, 4.61 against 4.23; 5.28 before
+// the element buffers), with 8 points 1.33 against 0.61 ms, and with 27 points
+// the set-up of a first call costs more than the 0.56 ms saved (3.5 against 2.1).
 inline bool exact_residual(const Context *c, bool with_tangent) { return with_tangent || c->nquad >= 4; }
 // res_df.cu (linear law residual in double-FP32 arithmetic)
 int ensure_res_pairs(Context *c);

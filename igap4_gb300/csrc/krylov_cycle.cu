@@ -34,9 +34,8 @@
 //    four basis vectors, and the partial sums of several rows or vectors are
 //    folded together (9 instead of 40 additions for 8 sums).
 //
-// Measured: 100 iterations at 32x8x8 (10,200 rows, Jacobi) 86.2 -> 3.3 ms; with
-// the assembly as it was before, the static solve of the 16x4x4 beam 79.3 ->
-// 13.9 ms and the transient step at 32x8x8 (cell blocks, CGS2) 18.3 -> 13.8 ms.
+// Measured: 100 iterations at 32x8x8 (10,200 rows, Jacobi) 86.2 ms as separate
+// launches, 3.3 ms here; figures over sizes and restarts at cycle_applies.
 //
 // One block of 1024 threads per SM (cooperative launch: all blocks resident).
 // Data that other blocks wrote are read with plain or L2 loads after the

@@ -39,7 +39,7 @@
 // 4e-15 of |F|); on pure bending, whose Hessian terms cancel, the rounding of the
 // rows of S adds to the geometry's and it is 1.2 to 1.7 times as large (1.4e-15 to
 // 7e-15 there, 2e-15 to 1.2e-14 here; affine states at length scale 0.2 up to 1.3).  Residual and tangent at 16x4x4 7.9 ms (FP64 kernel,
-// colour by colour) -> 76 us, 63x17x15 36.7 -> 2.05 ms.  Per element and SM 31 k
+// colour by colour) -> 78 us, 63x17x15 36.7 -> 1.98 ms.  Per element and SM 31 k
 // clocks, 27 k of them MMAs (73 clocks each: shared-memory operand reads).
 //
 // One persistent CTA per SM over all elements; results go to the element

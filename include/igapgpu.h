@@ -50,7 +50,8 @@ extern "C" {
  * In both tensor-core modes the residual's contractions run in double-FP32 arithmetic
  * (pairs of floats, compensated sums; the reference's laws keep their FP64 law between
  * them): relative error <= 1e-12 vs FP64 (measured ~1e-14); IGAPGPU_RES_DF=0 keeps FP64. */
-#define IGAPGPU_PREC_FP64 0  /* FP64 everywhere */
+#define IGAPGPU_PREC_FP64 0  /* FP64; the linear law's element matrices from exact sums of BF16 slices of 54-bit
+                                operands (errors of FP64 size; IGAPGPU_TC_EXACT=0: FP64 arithmetic) */
 #define IGAPGPU_PREC_SPLIT 1 /* tangent on the tensor cores: TF32x3 products (hi*hi + hi*lo + lo*hi),
                                 FP32 accumulate; relative error <= 1e-5 (measured ~2e-6) */
 #define IGAPGPU_PREC_OZAKI 2 /* FP64-quality tangent on the tensor cores (linear law): the sqrt(w)-weighted
@@ -105,12 +106,14 @@ typedef struct {
                           4 = restricted additive Schwarz: the cells of 3 extended by one control-point layer
                               (up to 192 DOFs), FP32 subdomain solves, each DOF from its own cell (the
                               reference's default PCASM / PC_ASM_RESTRICT, src/interface.c:240-241; single lattice) */
-  int use_graphs;      /* 1: assembly and GMRES cycles replayed as CUDA graphs */
+  int use_graphs;      /* 1: assembly replayed as CUDA graphs, and GMRES whole cycles at a time: one kernel a
+                          cycle, or a graph of separate kernels (restart above 200, or short for a large
+                          system) */
   int orth;            /* GMRES orthogonalisation: 0 = modified Gram-Schmidt (the reference's
                           KSPGMRESModifiedGramSchmidtOrthogonalization, src/interface.c:234);
                           1 = classical Gram-Schmidt applied twice (CGS2: two block passes per
                           Arnoldi step instead of one dot and one update per basis vector;
-                          graph GMRES only, the host-driven GMRES always uses MGS) */
+                          with use_graphs only, else always MGS) */
   double snes_f0_max;  /* > 0: an initial iterate whose |F| exceeds this is rejected before any Newton
                           step (reason IGAPGPU_REASON_REJECTED, U unchanged): a predicted guess is
                           tried against the residual of the plain guess without a second solve */
