@@ -40,7 +40,10 @@ def test_residual_alone_takes_no_element_matrices():
 def leave_free(nbytes):
     """a tensor that leaves about nbytes of device memory"""
     torch.cuda.empty_cache()
-    return torch.empty(free_bytes() - nbytes, dtype=torch.uint8, device="cuda")
+    try:
+        return torch.empty(free_bytes() - nbytes, dtype=torch.uint8, device="cuda")
+    except torch.OutOfMemoryError:
+        pytest.skip("the free memory is not available in one piece")
 
 
 def test_caches_take_at_most_a_quarter(monkeypatch):
